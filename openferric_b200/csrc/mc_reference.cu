@@ -17,6 +17,7 @@
 
 #include "of_device.cuh"
 #include "of_internal.h"
+#include "ref_stream.cuh"
 
 namespace {
 
@@ -33,6 +34,15 @@ struct RefParams {
   const double* inj;    // injected normals or nullptr
   const of_div_trigger* div;  // GBM discrete dividends by trigger step, or nullptr
   int32_t n_div;
+  // the log-space kernels
+  int32_t bar_hit0;           // barrier: path[0] is beyond the level
+  double bar_sign, bar_thr, bar_step;  // +1 up / -1 down; threshold of sign * sum(z) before step 1, its move per step
+  double w0, geo0;            // Asian: observations of path[0]; sum of w_j (ln s0 + j drift)
+  double y_floor;             // Heston: ln(1e-12 / s0)
+  const double2* obs;         // Asian: (w_j, w_j e^(j drift)) of steps 1..steps
+  double* partials;           // [blocks][5]
+  unsigned* ticket;
+  double* out;                // [5], pinned host memory
 };
 
 struct Leg {
@@ -175,59 +185,207 @@ __global__ void __launch_bounds__(128) mc_ref_kernel(RefParams P, double* __rest
     for (int k = 0; k < 5; ++k) partials[(int64_t)blockIdx.x * 5 + k] = acc[k];
 }
 
-// GBM European without dividends: the path matters only through S_T, a
-// product of per-step factors, so two adjacent lanes share a sample.  Both
-// step the sample's stream; lane p computes the normal and the factor
-// exp(fma(sigma sqrt(dt), z, drift)) of the steps j = p (mod 2), and the pair
-// multiplies its two partial products.  The draws and each step's factor are
-// mc_ref_kernel's; only the order of the product's roundings differs (S_T to
-// about 1e-15 relative).  Half the FP64 work per lane and twice the lanes
-// for the same samples: this workload has too few samples per SM to hide the
-// FP64 exp and divide latencies with one lane per sample.
+// ---------------------------------------------------------------------------
+// The kernels of the reference stream without injected normals and without
+// dividends: one lane per sample, the normals of ref_stream.cuh, log-space
+// paths.  A step's factor exp(drift + diff z) multiplies the spot in the
+// reference (simulation.rs:67-71); here its exponent is added, and the spot is
+// formed where a payoff reads it.  The draws are the same and the roundings
+// fewer: prices agree with mc_ref_kernel's to about 1e-15 relative.
+//
+// What bounds them: instruction issue, shared by the FP64 pipe (17 operations
+// a draw) and the integer pipe (the xoshiro update, 24), about 100 cycles a
+// draw and warp at five warps per scheduler.  mc_ref_kernel spent most of its
+// issue slots in the tails' branch and the per-step exp.  Device time before
+// and after on one B200 (launch included):
+//   European 100,000 x 252              387 -> 90 us
+//   Asian 50,000 pairs x 252, both averages  ~660 -> 95 us
+//   knock-out 25,001 pairs x 126        144 -> 38 us
+//   Heston European 131,072 x 256       940 -> 250 us
+// ---------------------------------------------------------------------------
+constexpr int kRefThreads = 64;  // small blocks: 100,000 samples fill 148 SMs to 96 %, blocks of 128 to 88 %
+
+__device__ __forceinline__ void ref_account(const RefParams& P, const Leg& a, const Leg& b, double (&acc)[5]) {
+  double x = leg_payoff(a, P);
+  double y = leg_cv(a, P);
+  if (P.antithetic) {  // simulation.rs:235-252
+    x = 0.5 * (x + leg_payoff(b, P));
+    y = 0.5 * (y + leg_cv(b, P));
+  }
+  acc[0] += x;
+  acc[1] += x * x;
+  acc[2] += y;
+  acc[3] += x * y;
+  acc[4] += y * y;
+}
+
+// GBM European (its control variate, if any, reads S_T only): the sum of the
+// path's normals, one exp per leg.
 template <typename RNG>
-__global__ void __launch_bounds__(128) mc_ref_gbm_terminal(RefParams P, double* __restrict__ partials) {
-  __shared__ double sh[5 * 4];
+__global__ void __launch_bounds__(kRefThreads) mc_ref_gbm_terminal(const __grid_constant__ RefParams P) {
+  __shared__ double list[kRefThreads * of::kTailCap];
+  __shared__ double sh[kRefThreads];
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  const int lane = (int)(threadIdx.x & 31u), par = lane & 1;
-  const int64_t pair0 = ((int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> 1;  // the warp's first sample
-  const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 1;
-  for (int64_t base = pair0; base < P.samples; base += stride) {  // warp-uniform trip count
-    const int64_t i = base + (lane >> 1);
-    const bool valid = i < P.samples;
+  const int64_t stride = (int64_t)gridDim.x * kRefThreads;
+  const double base = P.drift * (double)P.steps;
+  for (int64_t first = (int64_t)blockIdx.x * kRefThreads; first < P.samples; first += stride) {
+    const int64_t i = first + threadIdx.x;
     RNG rng;
     rng.seed(P.seed + (uint64_t)i * 7919ULL);  // stream_seed, fast_rng.rs:203-205
-    double fa = 1.0, fb = 1.0;
-    // both lanes draw steps j and j+1 of the stream; each takes its own (no
-    // divergence: every lane runs the inverse normal and exp each iteration)
-    for (int64_t j = 0; j < P.steps; j += 2) {
-      const double u0 = rng.next_f64();
-      const double u1 = j + 1 < P.steps ? rng.next_f64() : 0.5;
-      if (j + par < P.steps) {
-        const double z = of::acklam_inv_cdf(par ? u1 : u0);
-        fa *= exp(fma(P.diffusion, z, P.drift));  // simulation.rs:67-71
-        if (P.antithetic) fb *= exp(fma(P.diffusion, -z, P.drift));
-      }
-    }
-    const double oa = __shfl_xor_sync(of::kFullMask, fa, 1);
-    const double ob = __shfl_xor_sync(of::kFullMask, fb, 1);
-    if (par == 0 && valid) {
-      Leg a{P.s0 * fa * oa, 0.0, 0.0, 0.0, false}, b{P.s0 * fb * ob, 0.0, 0.0, 0.0, false};
-      double x = vanilla(P.option_type, a.s, P.strike);
-      double y = leg_cv(a, P);
-      if (P.antithetic) {  // simulation.rs:235-252
-        x = 0.5 * (x + vanilla(P.option_type, b.s, P.strike));
-        y = 0.5 * (y + leg_cv(b, P));
-      }
-      acc[0] += x;
-      acc[1] += x * x;
-      acc[2] += y;
-      acc[3] += x * y;
-      acc[4] += y * y;
+    const double w = of::stream_normal_sum(rng, P.steps, list + threadIdx.x, kRefThreads);
+    if (i < P.samples) {
+      Leg a{P.s0 * exp(fma(P.diffusion, w, base)), 0.0, 0.0, 0.0, false}, b = a;
+      if (P.antithetic) b.s = P.s0 * exp(fma(-P.diffusion, w, base));
+      ref_account(P, a, b, acc);
     }
   }
-  of::block_sum<5>(acc, sh);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 5; ++k) partials[(int64_t)blockIdx.x * 5 + k] = acc[k];
+  of::grid_sum<5, kRefThreads>(acc, sh, P.partials, P.ticket, P.out);
+}
+
+// GBM barrier or Asian.  With W the running sum of the normals, the log-spot
+// of a leg after step j is j drift +- diff W:
+//   barrier: the spot is beyond the level when +-W reaches a threshold that
+//     moves by -drift/diff a step (no exp, one comparison per leg);
+//   Asian: sum_j w_j e^(j drift) E^(+-1), E = exp(diff W), with the
+//     weights w_j e^(j drift) from the host: the antithetic leg costs a
+//     reciprocal instead of a second exp; the geometric sum is diff sum w_j W_j.
+enum : int { RK_BARRIER = 0, RK_ARITH = 1, RK_GEO = 2, RK_BOTH = 3 };
+
+template <typename RNG, int KIND, bool ANTI>
+__global__ void __launch_bounds__(kRefThreads) mc_ref_gbm_path(const __grid_constant__ RefParams P) {
+  __shared__ of::DrawBuf bufs[kRefThreads / 32];
+  __shared__ double tab[64];
+  __shared__ double sh[kRefThreads];
+  constexpr bool kArith = KIND == RK_ARITH || KIND == RK_BOTH, kGeo = KIND == RK_GEO || KIND == RK_BOTH;
+  if (kArith) of::exp_table_load(tab);
+  __syncthreads();
+  of::DrawBuf& buf = bufs[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  const int64_t stride = (int64_t)gridDim.x * kRefThreads;
+  const double base = P.drift * (double)P.steps;
+  const int32_t steps = (int32_t)P.steps;
+  for (int64_t first = (int64_t)blockIdx.x * kRefThreads; first < P.samples; first += stride) {
+    const int64_t i = first + threadIdx.x;
+    RNG rng;
+    rng.seed(P.seed + (uint64_t)i * 7919ULL);
+    double w = 0.0, aa = P.w0, ab = P.w0, g = 0.0, thr = P.bar_thr;
+    bool ha = P.bar_hit0 != 0, hb = ha;
+    for (int32_t j0 = 0; j0 < steps; j0 += of::kDrawBatch) {
+      of::stream_normals(rng, buf, lane);
+      const int n = steps - j0 < of::kDrawBatch ? steps - j0 : of::kDrawBatch;
+#pragma unroll 4
+      for (int k = 0; k < n; ++k) {
+        w += buf.z[k * 32 + lane];
+        if (KIND == RK_BARRIER) {
+          thr += P.bar_step;
+          const double sw = P.bar_sign * w;
+          ha |= sw >= thr;
+          if (ANTI) hb |= -sw >= thr;
+        } else {
+          const double2 c = __ldg(P.obs + j0 + k);  // (w_j, w_j e^(j drift)) of step j0 + k + 1
+          if (c.x != 0.0) {
+            if (kArith) {
+              const double e = of::exp64(P.diffusion * w, tab);
+              aa = fma(c.y, e, aa);
+              if (ANTI) ab = fma(c.y, of::rcp64(e), ab);
+            }
+            if (kGeo) g = fma(c.x, w, g);
+          }
+        }
+      }
+      __syncwarp();
+    }
+    if (i < P.samples) {
+      const double y = P.diffusion * w, gy = P.diffusion * g;
+      Leg a{P.s0 * exp(base + y), 0.0, P.s0 * aa, P.geo0 + gy, ha}, b = a;
+      if (ANTI) b = Leg{P.s0 * exp(base - y), 0.0, P.s0 * ab, P.geo0 - gy, hb};
+      ref_account(P, a, b, acc);
+    }
+  }
+  of::grid_sum<5, kRefThreads>(acc, sh, P.partials, P.ticket, P.out);
+}
+
+// Heston European: heston_step with the log-spot in place of the spot.
+template <typename RNG, bool ANTI>
+__global__ void __launch_bounds__(kRefThreads) mc_ref_heston(const __grid_constant__ RefParams P) {
+  __shared__ of::DrawBuf bufs[kRefThreads / 32];
+  __shared__ double sh[kRefThreads];
+  of::DrawBuf& buf = bufs[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  const int64_t stride = (int64_t)gridDim.x * kRefThreads;
+  const int32_t steps = (int32_t)P.steps;
+  // the variance is floored at a positive 1e-290 for the square root's sake:
+  // its terms are lost in every sum, as those of 0 are
+  constexpr double kVFloor = 1e-290;
+  const double mudt = P.mu * P.dt, hdt = 0.5 * P.dt, omk = 1.0 - P.kappa * P.dt, kth = P.kappa * P.theta * P.dt;
+  const double xsd = P.xi * P.sqrt_dt, r1 = P.rho * P.sqrt_dt, r2 = P.rho_c * P.sqrt_dt;
+  auto step = [&](double& y, double& v, double z1, double zs) {
+    const double sq = of::sqrt64(v);
+    y = fmax(fma(sq, zs, fma(-hdt, v, y + mudt)), P.y_floor);
+    v = fmax(fma(sq, xsd * z1, fma(omk, v, kth)), kVFloor);
+  };
+  for (int64_t first = (int64_t)blockIdx.x * kRefThreads; first < P.samples; first += stride) {
+    const int64_t i = first + threadIdx.x;
+    RNG rng;
+    rng.seed(P.seed + (uint64_t)i * 7919ULL);
+    double ya = 0.0, yb = 0.0, va = fmax(P.v0, kVFloor), vb = va;
+    for (int32_t j0 = 0; j0 < steps; j0 += of::kDrawBatch / 2) {
+      of::stream_normals(rng, buf, lane);
+      const int n = steps - j0 < of::kDrawBatch / 2 ? steps - j0 : of::kDrawBatch / 2;
+#pragma unroll 2
+      for (int k = 0; k < n; ++k) {
+        const double z1 = buf.z[2 * k * 32 + lane], z2 = buf.z[(2 * k + 1) * 32 + lane];
+        const double zs = fma(r1, z1, r2 * z2);
+        step(ya, va, z1, zs);
+        if (ANTI) step(yb, vb, -z1, -zs);
+      }
+      __syncwarp();
+    }
+    if (i < P.samples) {
+      Leg a{P.s0 * exp(ya), 0.0, 0.0, 0.0, false}, b = a;
+      if (ANTI) b.s = P.s0 * exp(yb);
+      ref_account(P, a, b, acc);
+    }
+  }
+  of::grid_sum<5, kRefThreads>(acc, sh, P.partials, P.ticket, P.out);
+}
+
+typedef void (*RefKernel)(RefParams);
+
+template <typename RNG, bool ANTI>
+RefKernel ref_path_kernel(int kind) {
+  return kind == RK_BARRIER ? mc_ref_gbm_path<RNG, RK_BARRIER, ANTI>
+         : kind == RK_ARITH ? mc_ref_gbm_path<RNG, RK_ARITH, ANTI>
+         : kind == RK_GEO   ? mc_ref_gbm_path<RNG, RK_GEO, ANTI>
+                            : mc_ref_gbm_path<RNG, RK_BOTH, ANTI>;
+}
+
+// The log-space kernel for a request, or null where the general one runs:
+// injected normals, dividends (they act on the spot), path-dependent payoffs
+// under Heston, barriers under a vanishing volatility, Asians with so many
+// steps that their weights should not be staged in pinned memory, and Asians
+// whose log-spot could leave the range of exp64 or reach the reference's
+// 1e-12 floor under the logarithm.  (A sum of normals beyond 40 standard
+// deviations has probability below 1e-300.)
+template <typename RNG>
+RefKernel ref_kernel_for(const RefParams& P) {
+  if (P.inj || P.n_div) return nullptr;
+  const bool obs = P.need_arith || P.need_geo;
+  if (P.model != OF_MODEL_GBM) {
+    if (P.payoff != OF_PAYOFF_VANILLA || obs) return nullptr;
+    return P.antithetic ? mc_ref_heston<RNG, true> : mc_ref_heston<RNG, false>;
+  }
+  if (P.payoff == OF_PAYOFF_VANILLA && !obs) return mc_ref_gbm_terminal<RNG>;
+  if (P.payoff == OF_PAYOFF_BARRIER && !obs && P.diffusion > 1e-100)
+    return P.antithetic ? ref_path_kernel<RNG, true>(RK_BARRIER) : ref_path_kernel<RNG, false>(RK_BARRIER);
+  if (P.payoff != OF_PAYOFF_ASIAN || !obs || P.steps > (1 << 16)) return nullptr;
+  const double n = (double)P.steps, spread = 40.0 * P.diffusion * std::sqrt(n), drift = P.drift * n;
+  if (!(spread + std::fabs(drift) < 600.0)) return nullptr;
+  if (P.need_geo && !(std::log(P.s0) + std::fmin(drift, 0.0) - spread > std::log(1e-12))) return nullptr;
+  const int kind = P.need_arith ? (P.need_geo ? RK_BOTH : RK_ARITH) : RK_GEO;
+  return P.antithetic ? ref_path_kernel<RNG, true>(kind) : ref_path_kernel<RNG, false>(kind);
 }
 
 }  // namespace
@@ -383,13 +541,6 @@ extern "C" of_status of_mc_run(of_ctx* ctx, const of_model* m, const of_payoff* 
   P.terminal_only = terminal_only;
   P.n_obs = (double)p->n_observations;
 
-  void* d_obs = nullptr;
-  if (P.need_arith || P.need_geo) {
-    OF_TRY(of_scratch(ctx, SLOT_OBS, w.size() * sizeof(double), &d_obs));
-    OF_CUDA_TRY(ctx, cudaMemcpyAsync(d_obs, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-  }
-  P.obs_w = (const double*)d_obs;
-
   std::vector<of_div_trigger> trig;
   OF_TRY(of_dividend_triggers(ctx, m, trig));
   if (!trig.empty()) {
@@ -414,38 +565,77 @@ extern "C" of_status of_mc_run(of_ctx* ctx, const of_model* m, const of_payoff* 
     P.inj = (const double*)d_inj;
   }
 
-  const int block = 128;
-  // a GBM European without dividends (its control variate, if any, reads S_T
-  // only): two lanes per sample
-  const bool terminal = P.model == OF_MODEL_GBM && P.payoff == OF_PAYOFF_VANILLA && P.n_div == 0 && !P.inj &&
-                        P.cv_kind != OF_CV_GEOMETRIC_ASIAN;
-  const bool pcg = c->rng_kind == OF_RNG_PCG64;
-  const void* kern = terminal ? (pcg ? (const void*)mc_ref_gbm_terminal<of::Pcg64>
-                                     : (const void*)mc_ref_gbm_terminal<of::Xoshiro256pp>)
-                              : (pcg ? (const void*)mc_ref_kernel<of::Pcg64> : (const void*)mc_ref_kernel<of::Xoshiro256pp>);
-  const int64_t lanes = terminal ? 2 * P.samples : P.samples;
-  const int64_t want = (lanes + block - 1) / block;
-  const int64_t cap = (int64_t)ctx->sm_count * of_blocks_per_sm(kern, block, 0);
-  const int grid = (int)(want < cap ? want : cap);
-  void *d_part = nullptr, *d_sums = nullptr, *h = nullptr;
-  OF_TRY(of_scratch(ctx, SLOT_PARTIALS, (size_t)grid * 5 * sizeof(double), &d_part));
-  OF_TRY(of_scratch(ctx, SLOT_SUMS, 5 * sizeof(double), &d_sums));
-  OF_TRY(of_pinned(ctx, 5 * sizeof(double), &h));
-
-  OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
-  if (terminal && pcg) mc_ref_gbm_terminal<of::Pcg64><<<grid, block, 0, ctx->stream>>>(P, (double*)d_part);
-  else if (terminal) mc_ref_gbm_terminal<of::Xoshiro256pp><<<grid, block, 0, ctx->stream>>>(P, (double*)d_part);
-  else if (pcg) mc_ref_kernel<of::Pcg64><<<grid, block, 0, ctx->stream>>>(P, (double*)d_part);
-  else mc_ref_kernel<of::Xoshiro256pp><<<grid, block, 0, ctx->stream>>>(P, (double*)d_part);
-  OF_CUDA_TRY(ctx, cudaGetLastError());
-  OF_TRY(of_reduce_rows(ctx, (const double*)d_part, grid, 5, (double*)d_sums));
-  OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream));
-  OF_CUDA_TRY(ctx, cudaMemcpyAsync(h, d_sums, 5 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  OF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  float ms = 0.0f;
-  OF_CUDA_TRY(ctx, cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
+  void *d_part = nullptr, *h = nullptr;
   double sums[5];
-  std::memcpy(sums, h, sizeof(sums));
+  float ms = 0.0f;
+  const bool pcg = c->rng_kind == OF_RNG_PCG64;
+  if (RefKernel fast = pcg ? ref_kernel_for<of::Pcg64>(P) : ref_kernel_for<of::Xoshiro256pp>(P)) {
+    const bool obs = P.need_arith || P.need_geo;
+    const size_t table = obs ? (size_t)P.steps * sizeof(double2) : 0;
+    OF_TRY(of_pinned(ctx, table + 5 * sizeof(double), &h));
+    if (obs) {
+      void* d_obs = nullptr;
+      OF_TRY(of_scratch(ctx, SLOT_OBS, table, &d_obs));
+      double2* t = (double2*)h;
+      double geo = 0.0;
+      for (int64_t j = 1; j <= P.steps; ++j) {
+        const double wj = w[(size_t)j], yj = P.drift * (double)j;
+        t[j - 1] = make_double2(wj, wj != 0.0 ? wj * std::exp(yj) : 0.0);
+        geo += wj * yj;
+      }
+      P.w0 = w[0];
+      P.geo0 = P.n_obs * std::log(P.s0) + geo;  // every observation maps to a step, so the weights sum to n_obs
+      OF_CUDA_TRY(ctx, cudaMemcpyAsync(d_obs, t, table, cudaMemcpyHostToDevice, ctx->stream));
+      P.obs = (const double2*)d_obs;
+    }
+    if (P.payoff == OF_PAYOFF_BARRIER) {
+      P.bar_sign = P.barrier_up ? 1.0 : -1.0;
+      P.bar_hit0 = P.barrier_up ? P.s0 >= P.barrier : P.s0 <= P.barrier;
+      // a level <= 0 is below every spot
+      const double by = P.barrier <= 0.0 ? -INFINITY : std::log(P.barrier / P.s0);
+      P.bar_thr = P.bar_sign * by / P.diffusion;
+      P.bar_step = -P.bar_sign * P.drift / P.diffusion;
+    }
+    P.y_floor = std::log(1e-12 / P.s0);
+    const int64_t want = (P.samples + kRefThreads - 1) / kRefThreads, cap = (int64_t)ctx->sm_count * 16;
+    const int grid = (int)(want < cap ? want : cap);
+    OF_TRY(of_scratch(ctx, SLOT_PARTIALS, (size_t)grid * 5 * sizeof(double), &d_part));
+    OF_TRY(of_ticket(ctx, &P.ticket));
+    P.partials = (double*)d_part;
+    P.out = (double*)((char*)h + table);
+    OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
+    fast<<<grid, kRefThreads, 0, ctx->stream>>>(P);
+    OF_CUDA_TRY(ctx, cudaGetLastError());
+    OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream));
+    OF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    OF_CUDA_TRY(ctx, cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
+    std::memcpy(sums, P.out, sizeof(sums));
+  } else {
+    void *d_obs = nullptr, *d_sums = nullptr;
+    if (P.need_arith || P.need_geo) {
+      OF_TRY(of_scratch(ctx, SLOT_OBS, w.size() * sizeof(double), &d_obs));
+      OF_CUDA_TRY(ctx, cudaMemcpyAsync(d_obs, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    }
+    P.obs_w = (const double*)d_obs;
+    const int block = 128;
+    const void* kern = pcg ? (const void*)mc_ref_kernel<of::Pcg64> : (const void*)mc_ref_kernel<of::Xoshiro256pp>;
+    const int64_t want = (P.samples + block - 1) / block;
+    const int64_t cap = (int64_t)ctx->sm_count * of_blocks_per_sm(kern, block, 0);
+    const int grid = (int)(want < cap ? want : cap);
+    OF_TRY(of_scratch(ctx, SLOT_PARTIALS, (size_t)grid * 5 * sizeof(double), &d_part));
+    OF_TRY(of_scratch(ctx, SLOT_SUMS, 5 * sizeof(double), &d_sums));
+    OF_TRY(of_pinned(ctx, 5 * sizeof(double), &h));
+    OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
+    if (pcg) mc_ref_kernel<of::Pcg64><<<grid, block, 0, ctx->stream>>>(P, (double*)d_part);
+    else mc_ref_kernel<of::Xoshiro256pp><<<grid, block, 0, ctx->stream>>>(P, (double*)d_part);
+    OF_CUDA_TRY(ctx, cudaGetLastError());
+    OF_TRY(of_reduce_rows(ctx, (const double*)d_part, grid, 5, (double*)d_sums));
+    OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream));
+    OF_CUDA_TRY(ctx, cudaMemcpyAsync(h, d_sums, 5 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    OF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    OF_CUDA_TRY(ctx, cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
+    std::memcpy(sums, h, sizeof(sums));
+  }
   of_mc_finish(sums, P.samples, c->control_variate, c->cv_expected, c->discount_factor, out);
   out->kernel_ms = ms;
   return OF_OK;

@@ -71,6 +71,15 @@ of_status of_pinned(of_ctx* ctx, size_t bytes, void** out) {
   return OF_OK;
 }
 
+of_status of_ticket(of_ctx* ctx, unsigned** out) {
+  const bool fresh = ctx->slot_ptr[SLOT_TICKET] == nullptr;
+  void* p = nullptr;
+  OF_TRY(of_scratch(ctx, SLOT_TICKET, sizeof(unsigned), &p));
+  if (fresh) OF_CUDA_TRY(ctx, cudaMemsetAsync(p, 0, sizeof(unsigned), ctx->stream));
+  *out = (unsigned*)p;
+  return OF_OK;
+}
+
 int of_blocks_per_sm(const void* kernel, int block, size_t smem) {
   int n = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, smem) != cudaSuccess || n < 1) n = 1;
@@ -107,6 +116,9 @@ of_status of_reduce_rows(of_ctx* ctx, const double* in, int64_t rows, int64_t co
 
 void of_mc_finish(const double s[5], int64_t count, int32_t cv_kind, double e, double df, of_mc_result* out) {
   const double n = (double)count;
+  // a variance that only rounding made negative (a control variate equal to
+  // the payoff, a constant payoff) is 0
+  auto stderr_of = [&](double var) { return df * std::sqrt((var < 0.0 ? 0.0 : var) / n); };
   out->samples = count;
   out->sum_x = s[0];
   out->sum_x2 = s[1];
@@ -124,12 +136,12 @@ void of_mc_finish(const double s[5], int64_t count, int32_t cv_kind, double e, d
     const double mean = sum_adj / n;
     const double var = n > 1.0 ? (sum_adj_sq - sum_adj * sum_adj / n) / (n - 1.0) : 0.0;
     out->price = df * mean;
-    out->stderr_ = df * std::sqrt(var / n);
+    out->stderr_ = stderr_of(var);
   } else {
     const double mean = s[0] / n;
     const double var = n > 1.0 ? (s[1] - s[0] * s[0] / n) / (n - 1.0) : 0.0;
     out->price = df * mean;
-    out->stderr_ = df * std::sqrt(var / n);
+    out->stderr_ = stderr_of(var);
   }
 }
 

@@ -39,14 +39,14 @@ struct Xoshiro256pp {
   }
 
   __device__ __forceinline__ uint64_t next_u64() {
+    // the update written so that each new word is one three-input XOR
     const uint64_t result = rotl(s0 + s3, 23) + s0;
-    const uint64_t t = s1 << 17;
-    s2 ^= s0;
-    s3 ^= s1;
-    s1 ^= s2;
-    s0 ^= s3;
-    s2 ^= t;
-    s3 = rotl(s3, 45);
+    const uint64_t x = s3 ^ s1;
+    const uint64_t n2 = s2 ^ s0 ^ (s1 << 17);
+    s1 = s1 ^ s2 ^ s0;
+    s2 = n2;
+    s0 = s0 ^ x;
+    s3 = rotl(x, 45);
     return result;
   }
 

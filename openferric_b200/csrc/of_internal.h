@@ -28,7 +28,7 @@ enum OfSlot {
   SLOT_LSM_AUX = 10,   // LSM betas / counters
   SLOT_ADJ_CKPT = 11,  // adjoint checkpoints
   SLOT_ADJ_AUX = 12,
-  SLOT_STATUS = 13,    // device error word + counters
+  SLOT_TICKET = 13,    // last-block-done counter of grid_sum, zero between launches
   SLOT_MISC = 14,
   SLOT_JUMP = 15,      // xoshiro256++ GF(2) jump tables
   SLOT_LSM_PATHS_B = 16,   // second LSM buffer set: the next batch generates into it
@@ -73,6 +73,9 @@ of_status of_ctx_check(of_ctx* ctx);
 of_status of_scratch(of_ctx* ctx, int slot, size_t bytes, void** out);
 // Returns pinned host memory of at least `bytes`.
 of_status of_pinned(of_ctx* ctx, size_t bytes, void** out);
+// The context's last-block-done counter (zeroed when created; every kernel
+// that uses it leaves it zero).
+of_status of_ticket(of_ctx* ctx, unsigned** out);
 
 #define OF_CUDA_TRY(ctx, call)                                                                  \
   do {                                                                                          \
