@@ -8,7 +8,8 @@
 // and sweeps it backwards.  For the GBM log-Euler path the adjoint of every
 // step's exponent is the same number, dpv/dS_T * S_T, so the reverse sweep
 // collapses to closed forms of the forward quantities S_T, prod(growth) and
-// sum(z): the device keeps three registers per leg instead of a tape.
+// sum(z), and the first two are exp(steps drift + diffusion sum(z)): the
+// device keeps the sum of the stream's normals instead of a tape.
 // Compiled with --fmad=false (only explicit fma() contract, as in the
 // reference's mul_add).
 #include <cmath>
@@ -16,8 +17,11 @@
 
 #include "of_device.cuh"
 #include "of_internal.h"
+#include "ref_stream.cuh"
 
 namespace {
+
+constexpr int kGreekThreads = 64;  // as kRefThreads of mc_reference.cu
 
 struct GreekP {
   int32_t call, antithetic;
@@ -30,6 +34,10 @@ struct GreekP {
   double mu, kappa, theta, xi, rho, rho2, v0;
   // MonteCarloGreeksEngine (mc_greeks.rs:157-170)
   double g_drift, sig_sqrt_t, spot_up, spot_dn, spot_span, sqrt_t;
+  // grid_sum
+  double* partials;
+  unsigned* ticket;
+  double* out;
 };
 
 // One GBM leg through the tape semantics of gbm_single_path_reverse
@@ -70,32 +78,25 @@ __device__ __forceinline__ void aad_leg_finish(const AadLeg& L, const GreekP& P,
   g[3] = t_bar;
 }
 
-__global__ void __launch_bounds__(128) aad_kernel(GreekP P, double* __restrict__ partials) {
-  __shared__ double sh[6 * 4];
+__global__ void __launch_bounds__(kGreekThreads) aad_kernel(const __grid_constant__ GreekP P) {
+  __shared__ double list[kGreekThreads * of::kTailCap];
+  __shared__ double sh[kGreekThreads];
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P.samples; i += stride) {
+  const int64_t stride = (int64_t)gridDim.x * kGreekThreads;
+  const double base = P.drift * (double)P.steps;
+  for (int64_t first = (int64_t)blockIdx.x * kGreekThreads; first < P.samples; first += stride) {
+    const int64_t i = first + threadIdx.x;
     of::Xoshiro256pp rng;
     rng.seed(P.seed + (uint64_t)i * 7919ULL);
-    AadLeg a{P.spot, 1.0, 0.0}, b{P.spot, 1.0, 0.0};
-    for (int64_t j = 0; j < P.steps; ++j) {
-      const double z = of::acklam_inv_cdf(rng.next_f64());
-      const double ga = exp(P.drift + P.diffusion * z);
-      a.s = a.s * ga;
-      a.prod = a.prod * ga;
-      a.sumz += z;
-      if (P.antithetic) {
-        const double gb = exp(P.drift + P.diffusion * -z);
-        b.s = b.s * gb;
-        b.prod = b.prod * gb;
-        b.sumz += -z;
-      }
-    }
+    const double w = of::stream_normal_sum(rng, P.steps, list + threadIdx.x, kGreekThreads);
+    if (i >= P.samples) continue;  // no warp-wide operation below
+    const double ga = exp(fma(P.diffusion, w, base));
     double pv, g[4];
-    aad_leg_finish(a, P, pv, g);
+    aad_leg_finish(AadLeg{P.spot * ga, ga, w}, P, pv, g);
     if (P.antithetic) {  // mc_aad.rs:169-194
+      const double gb = exp(fma(-P.diffusion, w, base));
       double pv1, g1[4];
-      aad_leg_finish(b, P, pv1, g1);
+      aad_leg_finish(AadLeg{P.spot * gb, gb, -w}, P, pv1, g1);
       for (int k = 0; k < 4; ++k) g[k] = 0.5 * (g[k] + g1[k]);
       pv = 0.5 * (pv + pv1);
     }
@@ -103,43 +104,45 @@ __global__ void __launch_bounds__(128) aad_kernel(GreekP P, double* __restrict__
     acc[1] += pv * pv;
     for (int k = 0; k < 4; ++k) acc[2 + k] += g[k];
   }
-  of::block_sum<6>(acc, sh);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 6; ++k) partials[(int64_t)blockIdx.x * 6 + k] = acc[k];
+  of::grid_sum<6, kGreekThreads>(acc, sh, P.partials, P.ticket, P.out);
 }
 
-// heston_single_path_price_delta (mc_aad.rs:239-276): Dual forward mode in s.
-__global__ void __launch_bounds__(128) heston_delta_kernel(GreekP P, double* __restrict__ partials) {
-  __shared__ double sh[2 * 4];
+// heston_single_path_price_delta (mc_aad.rs:239-276): Dual forward mode in s,
+// whose derivative is the path's growth factor; log-space as mc_ref_heston.
+__global__ void __launch_bounds__(kGreekThreads) heston_delta_kernel(const __grid_constant__ GreekP P) {
+  __shared__ of::DrawBuf bufs[kGreekThreads / 32];
+  __shared__ double sh[kGreekThreads];
+  of::DrawBuf& buf = bufs[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
   double acc[2] = {0, 0};
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P.samples; i += stride) {
+  const int64_t stride = (int64_t)gridDim.x * kGreekThreads;
+  constexpr double kVFloor = 1e-290;  // in place of 0, for the square root
+  const double mudt = P.mu * P.dt, hdt = 0.5 * P.dt, omk = 1.0 - P.kappa * P.dt, kth = P.kappa * P.theta * P.dt;
+  const double xsd = P.xi * P.sqrt_dt, r1 = P.rho * P.sqrt_dt, r2 = P.rho2 * P.sqrt_dt;
+  for (int64_t first = (int64_t)blockIdx.x * kGreekThreads; first < P.samples; first += stride) {
+    const int64_t i = first + threadIdx.x;
     of::Xoshiro256pp rng;
     rng.seed(P.seed + (uint64_t)i * 7919ULL);
-    double s = P.spot, ds = 1.0, v = P.v0;
-    for (int64_t j = 0; j < P.steps; ++j) {
-      const double z1 = of::acklam_inv_cdf(rng.next_f64());
-      const double z2 = of::acklam_inv_cdf(rng.next_f64());
-      const double v_pos = v > 0.0 ? v : 0.0;
-      const double sqrt_v = sqrt(v_pos);
-      const double zs = P.rho * z1 + P.rho2 * z2;
-      double v_next = v + P.kappa * (P.theta - v_pos) * P.dt + P.xi * sqrt_v * P.sqrt_dt * z1;
-      v_next = v_next > 0.0 ? v_next : 0.0;
-      const double growth = exp((P.mu - 0.5 * v_pos) * P.dt + sqrt_v * P.sqrt_dt * zs);
-      s = s * growth;
-      ds = ds * growth;
-      v = v_next;
+    double y = 0.0, v = fmax(P.v0, kVFloor);
+    for (int64_t left = P.steps; left > 0; left -= of::kDrawBatch / 2) {
+      of::stream_normals(rng, buf, lane);
+      const int n = left < of::kDrawBatch / 2 ? (int)left : of::kDrawBatch / 2;
+#pragma unroll 2
+      for (int k = 0; k < n; ++k) {
+        const double z1 = buf.z[2 * k * 32 + lane], z2 = buf.z[(2 * k + 1) * 32 + lane];
+        const double sq = of::sqrt64(v);
+        y = fma(sq, fma(r1, z1, r2 * z2), fma(-hdt, v, y + mudt));
+        v = fmax(fma(sq, xsd * z1, fma(omk, v, kth)), kVFloor);
+      }
+      __syncwarp();
     }
-    double pv, dpv;
+    if (i >= P.samples) continue;  // no warp-wide operation below
+    const double ds = exp(y), s = P.spot * ds;
     const double val = P.call ? s - P.strike : P.strike - s;
-    pv = val > 0.0 ? val : 0.0;
-    dpv = val > 0.0 ? (P.call ? ds : -ds) : 0.0;
-    acc[0] += pv * P.disc;
-    acc[1] += dpv * P.disc;
+    acc[0] += val > 0.0 ? val * P.disc : 0.0;
+    acc[1] += val > 0.0 ? (P.call ? ds : -ds) * P.disc : 0.0;
   }
-  of::block_sum<2>(acc, sh);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 2; ++k) partials[(int64_t)blockIdx.x * 2 + k] = acc[k];
+  of::grid_sum<2, kGreekThreads>(acc, sh, P.partials, P.ticket, P.out);
 }
 
 // single_path_contribution (mc_greeks.rs:266-314).
@@ -166,8 +169,8 @@ __device__ __forceinline__ void greek_contrib(const GreekP& P, double z, double 
   o[4] = payoff * w_vega;
 }
 
-__global__ void __launch_bounds__(128) estimators_kernel(GreekP P, double* __restrict__ partials) {
-  __shared__ double sh[5 * 4];
+__global__ void __launch_bounds__(kGreekThreads) estimators_kernel(const __grid_constant__ GreekP P) {
+  __shared__ double sh[kGreekThreads];
   double acc[5] = {0, 0, 0, 0, 0};
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P.samples; i += stride) {
@@ -183,28 +186,23 @@ __global__ void __launch_bounds__(128) estimators_kernel(GreekP P, double* __res
     }
     for (int k = 0; k < 5; ++k) acc[k] += b[k];
   }
-  of::block_sum<5>(acc, sh);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 5; ++k) partials[(int64_t)blockIdx.x * 5 + k] = acc[k];
+  of::grid_sum<5, kGreekThreads>(acc, sh, P.partials, P.ticket, P.out);
 }
 
 template <int NS>
-of_status launch_and_sum(of_ctx* ctx, void (*kern)(GreekP, double*), const GreekP& P, double sums[NS],
-                         double* ms) {
-  const int block = 128;
-  const int64_t want = (P.samples + block - 1) / block;
-  const int64_t cap = (int64_t)ctx->sm_count * of_blocks_per_sm((const void*)kern, block, 0);
+of_status launch_and_sum(of_ctx* ctx, void (*kern)(GreekP), GreekP& P, double sums[NS], double* ms) {
+  const int64_t want = (P.samples + kGreekThreads - 1) / kGreekThreads, cap = (int64_t)ctx->sm_count * 16;
   const int grid = (int)(want < cap ? want : cap);
-  void *d_part = nullptr, *d_sums = nullptr, *h = nullptr;
+  void *d_part = nullptr, *h = nullptr;
   OF_TRY(of_scratch(ctx, SLOT_PARTIALS, (size_t)grid * NS * sizeof(double), &d_part));
-  OF_TRY(of_scratch(ctx, SLOT_SUMS, NS * sizeof(double), &d_sums));
+  OF_TRY(of_ticket(ctx, &P.ticket));
   OF_TRY(of_pinned(ctx, NS * sizeof(double), &h));
+  P.partials = (double*)d_part;
+  P.out = (double*)h;
   OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
-  kern<<<grid, block, 0, ctx->stream>>>(P, (double*)d_part);
+  kern<<<grid, kGreekThreads, 0, ctx->stream>>>(P);
   OF_CUDA_TRY(ctx, cudaGetLastError());
-  OF_TRY(of_reduce_rows(ctx, (const double*)d_part, grid, NS, (double*)d_sums));
   OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream));
-  OF_CUDA_TRY(ctx, cudaMemcpyAsync(h, d_sums, NS * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   OF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   float t = 0.0f;
   OF_CUDA_TRY(ctx, cudaEventElapsedTime(&t, ctx->ev_start, ctx->ev_stop));
