@@ -21,9 +21,11 @@
 //
 // FP64 reference mode reproduces the reference's draws: ONE xoshiro256++
 // stream seeded with `seed` feeds all paths in path-major order
-// (longstaff_schwartz.rs:467-509).  A thread owns a chunk of consecutive paths
-// and jumps its copy of the stream to the chunk's first draw with GF(2)
-// matrix powers of the (linear) xoshiro state transition.
+// (longstaff_schwartz.rs:467-509).  A lane owns a few consecutive paths and
+// starts at their first draw, found with GF(2) matrix powers of the (linear)
+// xoshiro state transition.  Where the blocks of all contracts fit the device
+// at once, the whole backward induction is one cooperative launch
+// (lsm_backward_ref); else one kernel per date, as above.
 // FP32 Philox mode: counter-based normals, FP32 path store.
 //
 // Compiled with --fmad=false (FP32 code uses explicit fmaf) and with the
@@ -40,6 +42,7 @@
 #include "of_internal.h"
 #include "bulk_copy.cuh"
 #include "path_fp32.cuh"
+#include "ref_stream.cuh"
 #include "f32x2.cuh"
 
 namespace {
@@ -153,6 +156,7 @@ struct LsmC {
   double spot, strike, inv_strike, drift, step_vol, disc, inv_spot;  // strike = terminal strike
   // local-vol and Heston Euler (longstaff_schwartz.rs:218-281), FP64
   double mu, dt, sqrt_dt, kappa, theta, xi, rho, v0;
+  double y_floor;            // ln(1e-12 / spot), the log-space generator's spot floor
   const double* lv_k;        // [lv_nk] strikes of the sampled surface
   const double* lv_v;        // [n_expiries][lv_nk] vols
   const float* lv_kf;        // FP32 copies for the Philox mode
@@ -197,14 +201,18 @@ struct LsmBatch {
   unsigned long long* ex_bits;   // [nc][steps+1] bits of the max (put) / min (call) exercised spot
   double* itm_count;             // [nc][steps+1] in-the-money paths at each regression date
   const double* disc_pow;        // [nc][steps+1] disc^k by repeated multiplication, as V is discounted
-  uint32_t* status;              // bit 0: a pass gave up waiting for its bulk copies; bit 1: its drain gave up too
+  uint32_t* status;              // bit 0: a pass gave up waiting for its bulk copies; bit 1: its drain gave up too;
+                                 // bit 2: lsm_backward_ref gave up waiting for its other blocks
   unsigned long long* term_itm;  // [nc] paths in the money at expiry
   uint64_t seed;
   of::PhiloxKeys keys;
   uint32_t contract_base;
   const double* inj;         // [nc][n][steps][draws] or null
   const uint64_t* jump;      // jump tables
-  int32_t chunk;             // paths per thread in the reference generator
+  int32_t chunk;             // paths per thread in lsm_gen_ref
+  int32_t lane_paths;        // paths per lane in lsm_gen_stream
+  const uint64_t* states;    // lsm_stream_setup's output
+  void* rows;                // [2][nc][gridDim.x][kRowWords] 16-byte words of lsm_backward_ref
 };
 
 template <typename T>
@@ -246,17 +254,11 @@ __device__ __forceinline__ T lsm_local_vol(const T* __restrict__ g, const T* __r
   return a + (b - a) * ew;
 }
 
-// Terminal cash flow of a path and, when boundary statistics are wanted,
-// the count of in-the-money paths at expiry (one atomic per thread that has any).
-__device__ __forceinline__ int terminal_value(const LsmC& C, double k_T, double s, double& v, double& dv) {
-  v = intrinsic_v<double>(C.put, s, k_T);
-  dv = v > 0.0 ? (C.put ? -s * C.inv_spot : s * C.inv_spot) : 0.0;
-  return v > 0.0 ? 1 : 0;
-}
-
-// FP64 reference generator: chunk of consecutive paths per thread.  The
-// single xoshiro256++ stream feeds path after path; 1 draw per step (GBM,
-// local vol) or 2 (Heston: z1 then z2), longstaff_schwartz.rs:190-283.
+// FP64 reference generator, the general form (injected normals; volatilities
+// beyond the range of lsm_gen_stream's exponential): a chunk of consecutive
+// paths per thread.  The single xoshiro256++ stream feeds path after path; 1
+// draw per step (GBM, local vol) or 2 (Heston: z1 then z2),
+// longstaff_schwartz.rs:190-283.
 __global__ void __launch_bounds__(128) lsm_gen_ref(LsmBatch B) {
   const int c = blockIdx.y;
   const LsmC C = B.c[c];
@@ -265,16 +267,12 @@ __global__ void __launch_bounds__(128) lsm_gen_ref(LsmBatch B) {
   const int draws = C.dynamics == DYN_HESTON ? 2 : 1;
   const LsmStep* st = B.st + (size_t)c * (B.steps + 1);
   double* S = (double*)B.S + (size_t)c * B.steps * B.npad;
-  double* V = (double*)B.V + (size_t)c * B.npad;
-  int32_t* tau = B.tau + (size_t)c * B.npad;
   of::Xoshiro256pp rng;
   if (!B.inj) {
     rng.seed(B.seed);
     xoshiro_jump(rng, (uint64_t)chunk0 * (uint64_t)B.steps * (uint64_t)draws, B.jump);
   }
-  const double k_T = st[B.steps].strike;
   const double rho_c = sqrt(1.0 - C.rho * C.rho);
-  int itm = 0;
   const int64_t end = chunk0 + B.chunk < B.n ? chunk0 + B.chunk : B.n;
   for (int64_t p = chunk0; p < end; ++p) {
     double s = C.spot, var = C.v0;
@@ -303,12 +301,206 @@ __global__ void __launch_bounds__(128) lsm_gen_ref(LsmBatch B) {
       }
       S[(size_t)(t - 1) * B.npad + p] = s;
     }
-    double v, dv;
-    itm += terminal_value(C, k_T, s, v, dv);
-    V[p] = v;
-    if (B.want_delta) tau[p] = B.steps;
   }
-  if (B.track && itm) atomicAdd(B.term_itm + c, (unsigned long long)itm);
+}
+
+// Cash flows at expiry for the launch-per-date passes of the FP64 mode and,
+// when boundary statistics are wanted, the paths in the money there.
+__global__ void __launch_bounds__(256) lsm_terminal_ref(const __grid_constant__ LsmBatch B) {
+  const int c = blockIdx.y;
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  double v = 0.0;
+  if (p < B.n) {
+    const double s = ((const double*)B.S)[((size_t)c * B.steps + B.steps - 1) * B.npad + p];
+    v = intrinsic_v<double>(B.c[c].put, s, B.st[(size_t)c * (B.steps + 1) + B.steps].strike);
+    ((double*)B.V)[(size_t)c * B.npad + p] = v;
+    if (B.want_delta) B.tau[(size_t)c * B.npad + p] = B.steps;
+  }
+  const unsigned m = __ballot_sync(of::kFullMask, v > 0.0);
+  if (B.track && (threadIdx.x & 31) == 0 && m) atomicAdd(B.term_itm + c, (unsigned long long)__popc(m));
+}
+
+// ---------------------------------------------------------------------------
+// FP64 reference generator, one warp per 32 m consecutive paths: lane l owns
+// the m paths from 32 m W + m l on and walks their draws in the stream's
+// order; m is 1, 2 or 4 (lsm_lane_paths).
+//
+// The lanes' start states are powers of the linear state transition T applied
+// to the seeded state.  A matrix-vector product over GF(2) is a warp's work:
+// lane j holds the columns of bits j, 32+j, ... (64 words), masks them with
+// the vector's bits and the warp adds (XORs) its lanes' sums with eight
+// reductions: about 100 instructions, where a lane by itself takes 3,300.
+// lsm_stream_setup forms the first state of every 32nd warp, T^(1024 m c G)
+// seed (c draws a path; one product per set bit of the exponent), and the ten
+// matrices T^(m c 2^k).  A generator's warp moves its group's state to its own
+// with up to five of them and doubles its known lane states with the other
+// five, 31 products.
+// ---------------------------------------------------------------------------
+constexpr int kLaneLevels = 5, kWarpLevels = 5;
+
+struct Gf2Cols {
+  uint32_t c[8][8];  // c[w]: the column of bit 32 w + lane
+};
+
+__device__ __forceinline__ void gf2_cols_load(Gf2Cols& M, const uint64_t* __restrict__ tab, int lane) {
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    const uint4* p = reinterpret_cast<const uint4*>(tab + (size_t)(w * 32 + lane) * 4);
+    const uint4 a = __ldg(p), b = __ldg(p + 1);
+    M.c[w][0] = a.x;
+    M.c[w][1] = a.y;
+    M.c[w][2] = a.z;
+    M.c[w][3] = a.w;
+    M.c[w][4] = b.x;
+    M.c[w][5] = b.y;
+    M.c[w][6] = b.z;
+    M.c[w][7] = b.w;
+  }
+}
+
+// s <- M s for a vector that all lanes hold
+__device__ __forceinline__ void gf2_warp_apply(const Gf2Cols& M, uint32_t (&s)[8], int lane) {
+  uint32_t r[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    const uint32_t m = 0u - ((s[w] >> lane) & 1u);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) r[k] ^= M.c[w][k] & m;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s[k] = __reduce_xor_sync(of::kFullMask, r[k]);
+}
+
+// Warps 0 .. 2559: column (g % 256) of T^(lane_draws 2^(g / 256)); the others:
+// the state after G 1024 lane_draws draws, G = g - 2560.  `out`: the ten
+// matrices (column-major, as the jump tables), then [G][4].
+constexpr int kSetupThreads = 128;
+constexpr int kSetupColumns = (kLaneLevels + kWarpLevels) * 256;
+
+__global__ void __launch_bounds__(kSetupThreads) lsm_stream_setup(uint64_t seed, uint64_t lane_draws, int groups,
+                                                                  const uint64_t* __restrict__ jump,
+                                                                  uint32_t* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int g = (int)((blockIdx.x * kSetupThreads + threadIdx.x) >> 5);
+  if (g >= kSetupColumns + groups) return;
+  uint32_t s[8];
+  uint64_t n;
+  if (g < kSetupColumns) {
+    const int col = g & 255;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s[w] = col >> 5 == w ? 1u << (col & 31) : 0u;
+    n = lane_draws << (g >> 8);
+  } else {
+    of::Xoshiro256pp x;
+    x.seed(seed);
+    const uint64_t u[4] = {x.s0, x.s1, x.s2, x.s3};
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s[w] = (uint32_t)(u[w >> 1] >> (32 * (w & 1)));
+    n = lane_draws * 1024 * (uint64_t)(g - kSetupColumns);
+  }
+  for (int k = 0; n; ++k, n >>= 1)
+    if (n & 1ULL) {
+      Gf2Cols M;
+      gf2_cols_load(M, jump + (size_t)k * 1024, lane);
+      gf2_warp_apply(M, s, lane);
+    }
+#pragma unroll
+  for (int w = 0; w < 8; ++w)
+    if (lane == w) out[(size_t)g * 8 + w] = s[w];
+}
+
+constexpr int kGenThreads = 64;
+
+template <int DYN>
+__global__ void __launch_bounds__(kGenThreads) lsm_gen_stream(const __grid_constant__ LsmBatch B) {
+  __shared__ of::DrawBuf bufs[kGenThreads / 32];
+  __shared__ double tab[64];
+  of::exp_table_load(tab);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = blockIdx.x * (kGenThreads / 32) + (threadIdx.x >> 5), c = blockIdx.y;
+  const int m = B.lane_paths;
+  const int64_t p0 = ((int64_t)warp * 32 + lane) * m;
+  if ((int64_t)warp * 32 * m >= B.n) return;  // whole warps: no block-wide operation below
+  of::DrawBuf& buf = bufs[threadIdx.x >> 5];
+  of::Xoshiro256pp rng;
+  {
+    uint32_t s[8];
+    const uint32_t* base = reinterpret_cast<const uint32_t*>(B.states) + (size_t)(kSetupColumns + (warp >> 5)) * 8;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s[w] = __ldg(base + w);
+#pragma unroll 1
+    for (int k = 0; k < kWarpLevels; ++k)
+      if ((warp >> k) & 1) {
+        Gf2Cols M;
+        gf2_cols_load(M, B.states + (size_t)(kLaneLevels + k) * 1024, lane);
+        gf2_warp_apply(M, s, lane);
+      }
+    // lane 0 holds the warp's state; level k gives lanes 2^k .. 2^(k+1)-1 theirs
+#pragma unroll 1
+    for (int k = 0; k < kLaneLevels; ++k) {
+      Gf2Cols M;
+      gf2_cols_load(M, B.states + (size_t)k * 1024, lane);
+#pragma unroll 1
+      for (int src = 0; src < (1 << k); ++src) {
+        uint32_t v[8];
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v[w] = __shfl_sync(of::kFullMask, s[w], src);
+        gf2_warp_apply(M, v, lane);
+#pragma unroll
+        for (int w = 0; w < 8; ++w)
+          if (lane == src + (1 << k)) s[w] = v[w];
+      }
+    }
+    rng.s0 = (uint64_t)s[1] << 32 | s[0];
+    rng.s1 = (uint64_t)s[3] << 32 | s[2];
+    rng.s2 = (uint64_t)s[5] << 32 | s[4];
+    rng.s3 = (uint64_t)s[7] << 32 | s[6];
+  }
+  const LsmC& C = B.c[c];
+  const LsmStep* st = B.st + (size_t)c * (B.steps + 1);
+  double* S = (double*)B.S + (size_t)c * B.steps * B.npad;
+  constexpr int kDraws = DYN == DYN_HESTON ? 2 : 1;
+  constexpr double kVFloor = 1e-290;  // in place of 0, for the square root (its terms vanish in every sum)
+  const double drift = C.drift, vol = C.step_vol, spot = C.spot, y_floor = C.y_floor;
+  const double mudt = C.mu * C.dt, hdt = 0.5 * C.dt, omk = 1.0 - C.kappa * C.dt, kth = C.kappa * C.theta * C.dt;
+  const double xsd = C.xi * C.sqrt_dt, r1 = C.rho * C.sqrt_dt, r2 = sqrt(1.0 - C.rho * C.rho) * C.sqrt_dt;
+  int at = of::kDrawBatch;  // draws of the batch that are used
+  for (int q = 0; q < m; ++q) {
+    const bool in = p0 + q < B.n;
+    double* out = S + p0 + q;
+    double y = 0.0, var = fmax(C.v0, kVFloor), s = spot;
+    for (int t = 0; t < B.steps;) {
+      if (at == of::kDrawBatch) {
+        __syncwarp();
+        of::stream_normals(rng, buf, lane);
+        at = 0;
+      }
+      const int have = (of::kDrawBatch - at) / kDraws, n = B.steps - t < have ? B.steps - t : have;
+      const double* zb = buf.z + at * 32 + lane;
+#pragma unroll 2
+      for (int k = 0; k < n; ++k, zb += 32 * kDraws, out += B.npad) {
+        const double z = zb[0];
+        if (DYN == DYN_GBM) {
+          y += fma(vol, z, drift);  // longstaff_schwartz.rs:213-214, in log space
+        } else if (DYN == DYN_LOCAL_VOL) {
+          // :223-235: sigma at the step's end time and the previous spot
+          const LsmStep& e = st[t + k + 1];
+          const double sigma = lsm_local_vol<double>(C.lv_k, C.lv_v, C.lv_nk, e.e0, e.e1, e.ew,
+                                                     s > 1.0e-8 ? s : 1.0e-8);
+          y = fmax(y + fma(sigma * C.sqrt_dt, z, fma(-hdt * sigma, sigma, mudt)), y_floor);
+        } else {
+          // Heston::step_euler (src/models/stochastic.rs:56-71), :259-275
+          const double zs = fma(r1, z, r2 * zb[32]), sq = of::sqrt64(var);
+          y = fmin(fmax(fma(sq, zs, fma(-hdt, var, y + mudt)), y_floor), 680.0);
+          var = fmax(fma(sq, xsd * z, fma(omk, var, kth)), kVFloor);
+        }
+        s = spot * of::exp64(y, tab);
+        if (in) *out = s;
+      }
+      t += n;
+      at += n * kDraws;
+    }
+  }
 }
 
 // FP32 Philox generator: 4 consecutive paths per thread, float4 stores.  The
@@ -458,7 +650,8 @@ __device__ void solve_beta(int degree, const double* m, double* beta, int32_t* o
   if (degree == 2) {
     // m = {s1, S, S^2, S^3, S^4, y, Sy, S^2y}; nalgebra LU with partial pivoting
     double a[3][3] = {{m[0], m[1], m[2]}, {m[1], m[2], m[3]}, {m[2], m[3], m[4]}};
-    double b[3] = {m[5], m[6], m[7]};
+    double b[3] = {m[5], m[6], m[7]}, inv[3] = {0.0, 0.0, 0.0};
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
       int piv = i;
       double best = fabs(a[i][i]);
@@ -468,30 +661,40 @@ __device__ void solve_beta(int degree, const double* m, double* beta, int32_t* o
           piv = k;
         }
       if (best == 0.0) continue;
-      if (piv != i) {
-        for (int j = 0; j < 3; ++j) {
-          const double t = a[i][j];
-          a[i][j] = a[piv][j];
-          a[piv][j] = t;
+#pragma unroll
+      for (int k = i + 1; k < 3; ++k)  // the row swap with compile-time indices: the matrix stays in registers
+        if (k == piv) {
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            const double t = a[i][j];
+            a[i][j] = a[k][j];
+            a[k][j] = t;
+          }
+          const double tb = b[i];
+          b[i] = b[k];
+          b[k] = tb;
         }
-        const double tb = b[i];
-        b[i] = b[piv];
-        b[piv] = tb;
-      }
+      // one reciprocal per pivot, taken as soon as the pivot is known: the
+      // chain of dependent divisions was most of the solve's latency
+      inv[i] = of::rcp64(a[i][i]);
+#pragma unroll
       for (int k = i + 1; k < 3; ++k) {
-        const double f = a[k][i] / a[i][i];
-        a[k][i] = f;
+        const double f = a[k][i] * inv[i];
+#pragma unroll
         for (int j = i + 1; j < 3; ++j) a[k][j] -= f * a[i][j];
         b[k] -= f * b[i];
       }
     }
+#pragma unroll
     for (int i = 0; i < 3; ++i)
       if (a[i][i] == 0.0) return;  // singular: beta = 0 (:592)
     double x[3];
+#pragma unroll
     for (int i = 2; i >= 0; --i) {
       double s = b[i];
+#pragma unroll
       for (int j = i + 1; j < 3; ++j) s -= a[i][j] * x[j];
-      x[i] = s / a[i][i];
+      x[i] = s * inv[i];
     }
     beta[0] = x[0];
     beta[1] = x[1];
@@ -1215,6 +1418,330 @@ __global__ void __launch_bounds__(kPassThreads) lsm_final(LsmBatch B) {
 
 }  // namespace
 
+
+namespace {
+
+// ---------------------------------------------------------------------------
+// The whole backward induction of the FP64 mode in one cooperative launch
+// (blocks wait for one another, so all are resident): a thread keeps the cash
+// flows and payment steps of its PPT paths in registers and reads each date's
+// spots once.  Per regression date a block reduces its moments, writes a row
+// and reads the rows of every block of its contract as they appear; then every
+// block adds them in the same order and solves for the betas itself, so
+// nothing is published a second time.  A row's moments are 16-byte words of
+// value and date number, stored and loaded whole: a reader that sees the
+// number has the value, without a counter or a fence.  Rows alternate between
+// two buffers: a block writes row k+2 only after it has read every row k+1,
+// and their writers had read every row k by then.
+//
+// What bounds it: the latency of a date (block reduction, one trip through
+// the L2, row sums, a solve): 3.1 us at 100,000 paths, 1.9 at 1,000; a launch
+// per date took 11 (100,000 paths x 50 dates, whole call 1,135 us before this
+// kernel and the stream generator, 260 after).  Every wait is bounded by the global timer; a block that gives up sets
+// B.status and leaves, and so do the others at their next wait.
+// ---------------------------------------------------------------------------
+constexpr int kBackThreads = 256;
+constexpr uint64_t kBackWaitNs = 1000000000ull;
+
+__device__ __forceinline__ uint64_t lsm_timer_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// The warp's sums of v[0..8): lane 4 m holds that of moment m.  Each of the
+// first three exchanges halves the values a lane carries.
+__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
+#pragma unroll
+  for (int half = 4; half >= 1; half >>= 1) {
+    const bool up = lane & (half * 4);
+#pragma unroll
+    for (int k = 0; k < half; ++k) {
+      const double send = up ? v[k] : v[k + half], keep = up ? v[k + half] : v[k];
+      v[k] = keep + __shfl_xor_sync(of::kFullMask, send, half * 4);
+    }
+  }
+  double a = v[0];
+  a += __shfl_xor_sync(of::kFullMask, a, 2);
+  a += __shfl_xor_sync(of::kFullMask, a, 1);
+  return a;
+}
+
+constexpr int kBackWarps = kBackThreads / 32;
+constexpr int kMaxRows = 1024;  // blocks of one launch, all contracts (one per SM)
+constexpr int kRowWords = 16;  // 16-byte words of a row: moments 0..10, padded
+
+struct BackShared {
+  double warp[kBackWarps][kRowWords];
+  double mom[kRowWords];
+  double beta[4];
+  int32_t ok;
+};
+
+__device__ __forceinline__ void row_store(ulonglong2* p, double v, uint64_t tag) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}"
+               :
+               : "l"(p), "l"(__double_as_longlong(v)), "l"(tag)
+               : "memory");
+}
+
+__device__ __forceinline__ bool row_load(const ulonglong2* p, uint64_t tag, double& v) {
+  uint64_t a, b;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(a), "=l"(b)
+               : "l"(p)
+               : "memory");
+  v = __longlong_as_double((long long)a);
+  return b == tag;
+}
+
+// The block's sums of per-warp values sh.warp[w][0..16): warp 0's lanes m and
+// m + 16 add half of the warps' each.  Valid in lanes m and m + 16 of warp 0.
+__device__ __forceinline__ double back_cross_warp(const BackShared& sh, int lane) {
+  double t = sh.warp[(lane >> 4) * (kBackWarps / 2)][lane & 15];
+#pragma unroll
+  for (int w = 1; w < kBackWarps / 2; ++w) t += sh.warp[(lane >> 4) * (kBackWarps / 2) + w][lane & 15];
+  return t + __shfl_xor_sync(of::kFullMask, t, 16);
+}
+
+// Sums mom over all blocks of the contract into sh.mom (of warp 0's threads;
+// the caller synchronises).  `k` counts the calls in this launch.  Returns
+// false, in every thread of the block, after a wait that gave up.
+template <int NM>
+__device__ __forceinline__ bool back_moments(const LsmBatch& B, int c, int k, const double (&mom)[NM],
+                                             BackShared& sh) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double lo[8], hi[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    lo[i] = mom[i];
+    hi[i] = i + 8 < NM ? mom[i + 8] : 0.0;
+  }
+  const double a = warp_sum8(lo, lane);
+  if ((lane & 3) == 0) sh.warp[warp][lane >> 2] = a;
+  if (NM > 8) {
+    const double b = warp_sum8(hi, lane);
+    if ((lane & 3) == 0) sh.warp[warp][8 + (lane >> 2)] = b;
+  }
+  __syncthreads();
+  const uint64_t tag = (uint64_t)k + 1;  // the buffers start zeroed
+  ulonglong2* rows = (ulonglong2*)B.rows + ((size_t)(k & 1) * B.nc + c) * gridDim.x * kRowWords;
+  if (warp == 0) {
+    const double t = back_cross_warp(sh, lane);
+    if (lane < NM) row_store(rows + (size_t)blockIdx.x * kRowWords + lane, t, tag);
+  }
+  // thread t adds rows t / 16, t / 16 + 16, ... of moment t % 16
+  const int m = threadIdx.x & 15;
+  double t = 0.0;
+  bool ok = true;
+  if (m < NM) {
+    constexpr int kAhead = 10;  // rows in flight per thread: 160 rows, more than a block per SM, in one trip
+    for (unsigned r0 = threadIdx.x >> 4; ok && r0 < gridDim.x; r0 += kAhead * (kBackThreads / 16)) {
+      double v[kAhead];
+      bool got = false;
+      const uint64_t start = lsm_timer_ns();
+      while (!got) {
+        got = true;
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+          const unsigned r = r0 + i * (kBackThreads / 16);
+          v[i] = 0.0;
+          if (r < gridDim.x) got &= row_load(rows + (size_t)r * kRowWords + m, tag, v[i]);
+        }
+        if (!got && lsm_timer_ns() - start > kBackWaitNs) {
+          ok = false;
+          break;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kAhead; i += 2) t += v[i] + v[i + 1];
+    }
+  }
+  t += __shfl_xor_sync(of::kFullMask, t, 16);
+  // sh.warp is free: warp 0 read it before it stored the row that the block waited for
+  if (!__syncthreads_and(ok)) {
+    if (threadIdx.x == 0) atomicOr(B.status, 4u);
+    return false;
+  }
+  if (lane < 16) sh.warp[warp][lane] = t;
+  __syncthreads();
+  if (warp == 0) {
+    const double u = back_cross_warp(sh, lane);
+    if (lane < NM) sh.mom[lane] = u;
+    __syncwarp();
+  }
+  return true;
+}
+
+template <int DEG, int PPT>
+__global__ void __launch_bounds__(kBackThreads, 1) lsm_backward_ref(const __grid_constant__ LsmBatch B) {
+  constexpr int NM = DEG == 2 ? 8 : 11;
+  __shared__ BackShared sh;
+  const int c = blockIdx.y;
+  const LsmC& C = B.c[c];
+  const bool put = C.put;
+  const double disc = C.disc;
+  const uint8_t* can = B.can_ex + (size_t)c * (B.steps + 1);
+  const LsmStep* st = B.st + (size_t)c * (B.steps + 1);
+  const double* S = (const double*)B.S + (size_t)c * B.steps * B.npad;
+  const int64_t p0 = (int64_t)blockIdx.x * kBackThreads * PPT + threadIdx.x;
+  double v[PPT], s1[PPT], s0[PPT];
+  int tau[PPT];
+  bool in[PPT];
+  int itm = 0;
+#pragma unroll
+  for (int q = 0; q < PPT; ++q) {
+    const int64_t p = p0 + q * kBackThreads;
+    in[q] = p < B.n;
+    s1[q] = in[q] ? S[(size_t)(B.steps - 1) * B.npad + p] : 0.0;
+    s0[q] = in[q] ? S[(size_t)(B.steps - 2) * B.npad + p] : 0.0;
+    v[q] = in[q] ? intrinsic_v<double>(put, s1[q], st[B.steps].strike) : 0.0;
+    itm += v[q] > 0.0 ? 1 : 0;
+    tau[q] = B.steps;
+  }
+  if (B.track) {
+    itm = __reduce_add_sync(of::kFullMask, itm);
+    if ((threadIdx.x & 31) == 0 && itm) atomicAdd(B.term_itm + c, (unsigned long long)itm);
+  }
+  const double none = put ? 0.0 : __longlong_as_double(0x7FF0000000000000LL);
+  bool have_beta = false;
+  double beta[4] = {0, 0, 0, 0};
+  int waits = 0, regressions = 0;
+  for (int t = B.steps - 1; t >= 1; --t) {
+    const bool ex_now = can[t];
+    const double k1 = st[t + 1].strike, ik1 = st[t + 1].inv_strike, k0 = st[t].strike, ik0 = st[t].inv_strike;
+    double mom[NM];
+#pragma unroll
+    for (int i = 0; i < NM; ++i) mom[i] = 0.0;
+    unsigned n_ex = 0, n_itm = 0;
+    double ext = none;
+    // lsm_path_update without branches, so that a thread's paths overlap: a
+    // path out of the money (or past the end) enters the sums as x = y = 0
+#pragma unroll
+    for (int q = 0; q < PPT; ++q) {
+      const double ex = put ? k1 - s1[q] : s1[q] - k1;
+      const double x1 = DEG == 2 ? s1[q] : s1[q] * ik1;
+      const double cont = DEG == 2 ? fma(fma(beta[2], x1, beta[1]), x1, beta[0])
+                                   : fma(fma(fma(beta[3], x1, beta[2]), x1, beta[1]), x1, beta[0]);
+      const bool now = have_beta && in[q] && ex > 0.0 && ex > cont;
+      v[q] = (now ? ex : v[q]) * disc;
+      tau[q] = now ? t + 1 : tau[q];
+      n_ex += now ? 1u : 0u;
+      ext = now ? (put ? fmax(ext, s1[q]) : fmin(ext, s1[q])) : ext;
+      const bool itm = ex_now && in[q] && (put ? k0 - s0[q] : s0[q] - k0) > 0.0;
+      n_itm += itm ? 1u : 0u;
+      const double x = itm ? (DEG == 2 ? s0[q] : s0[q] * ik0) : 0.0, y = itm ? v[q] : 0.0;
+      const double x2 = x * x, x3 = x2 * x;
+      mom[1] += x;
+      mom[2] += x2;
+      mom[3] += x3;
+      mom[4] = fma(x2, x2, mom[4]);
+      if (DEG == 2) {
+        mom[5] += y;
+        mom[6] = fma(x, y, mom[6]);
+        mom[7] = fma(x2, y, mom[7]);
+      } else {
+        mom[5] = fma(x2, x3, mom[5]);
+        mom[6] = fma(x3, x3, mom[6]);
+        mom[7] += y;
+        mom[8 % NM] = fma(x, y, mom[8 % NM]);
+        mom[9 % NM] = fma(x2, y, mom[9 % NM]);
+        mom[10 % NM] = fma(x3, y, mom[10 % NM]);
+      }
+    }
+    mom[0] = (double)n_itm;
+    if (B.track && have_beta) record_exercise(B, c, t + 1, put, n_ex, ext);
+#pragma unroll
+    for (int q = 0; q < PPT; ++q) {
+      s1[q] = s0[q];
+      // the next date's spots arrive while the blocks wait
+      if (t >= 2) s0[q] = in[q] ? S[(size_t)(t - 2) * B.npad + p0 + q * kBackThreads] : 0.0;
+    }
+    have_beta = false;
+    if (!ex_now) continue;
+    if (!back_moments<NM>(B, c, waits++, mom, sh)) return;  // block-uniform
+    if (threadIdx.x == 0) {
+      solve_beta(DEG, sh.mom, sh.beta, &sh.ok);
+      if (blockIdx.x == 0) {
+        regressions += sh.ok ? 1 : 0;
+        if (B.track) B.itm_count[(size_t)c * (B.steps + 1) + t] = sh.mom[0];
+      }
+    }
+    __syncthreads();
+    have_beta = sh.ok;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) beta[i] = have_beta ? sh.beta[i] : 0.0;
+  }
+  // exercise at date 1, the last discount and the sums, as lsm_final
+  unsigned n_ex = 0;
+  double ext = none;
+  double acc[NM];
+#pragma unroll
+  for (int i = 0; i < NM; ++i) acc[i] = 0.0;
+#pragma unroll
+  for (int q = 0; q < PPT; ++q) {
+    if (!in[q]) continue;
+    if (have_beta) {
+      const double ex = intrinsic_v<double>(put, s1[q], st[1].strike);
+      if (ex > 0.0 && ex > continuation(DEG, beta, s1[q], st[1].inv_strike)) {
+        v[q] = ex;
+        tau[q] = 1;
+        ++n_ex;
+        ext = put ? fmax(ext, s1[q]) : fmin(ext, s1[q]);
+      }
+    }
+    v[q] *= C.disc;
+    double dv = 0.0;
+    if (B.want_delta && v[q] > 0.0) {
+      const double D = B.disc_pow[(size_t)c * (B.steps + 1) + tau[q]];
+      const double K = st[tau[q]].strike;
+      dv = put ? -(K * D - v[q]) * C.inv_spot : (K * D + v[q]) * C.inv_spot;
+    }
+    acc[0] += v[q];
+    acc[1] += v[q] * v[q];
+    acc[2] += dv;
+  }
+  if (B.track && have_beta) record_exercise(B, c, 1, put, n_ex, ext);
+  if (!back_moments<NM>(B, c, waits, acc, sh)) return;
+  if (threadIdx.x == 0 && blockIdx.x == 0) {
+    const double n = (double)B.n;
+    const double var = B.n > 1 ? (sh.mom[1] - sh.mom[0] * sh.mom[0] / n) / (n - 1.0) : 0.0;
+    B.results[c * 3 + 0] = sh.mom[0] / n;
+    B.results[c * 3 + 1] = sqrt(var / n);
+    B.results[c * 3 + 2] = sh.mom[2] / n;
+    B.regress_count[c] = regressions;
+  }
+}
+
+typedef void (*LsmBackKernel)(LsmBatch);
+
+LsmBackKernel lsm_back_kernel(int degree, int ppt) {
+  if (degree == 2)
+    return ppt == 1 ? lsm_backward_ref<2, 1> : ppt == 2 ? lsm_backward_ref<2, 2>
+           : ppt == 4 ? lsm_backward_ref<2, 4> : ppt == 8 ? lsm_backward_ref<2, 8> : lsm_backward_ref<2, 16>;
+  return ppt == 1 ? lsm_backward_ref<3, 1> : ppt == 2 ? lsm_backward_ref<3, 2>
+         : ppt == 4 ? lsm_backward_ref<3, 4> : ppt == 8 ? lsm_backward_ref<3, 8> : lsm_backward_ref<3, 16>;
+}
+
+// Paths per thread of the one-launch backward induction: the fewest whose
+// blocks are all resident, one per SM (0: too many paths or contracts for it,
+// a launch per date).
+int lsm_back_ppt(const of_ctx* ctx, int64_t n, int nc) {
+  const int64_t most = std::min(ctx->sm_count, kMaxRows);
+  for (int ppt = 1; ppt <= 16; ppt *= 2)
+    if ((n + (int64_t)kBackThreads * ppt - 1) / ((int64_t)kBackThreads * ppt) * nc <= most) return ppt;
+  return 0;
+}
+
+// Paths per lane of lsm_gen_stream: more paths share the lane's start state
+// (31 products a warp, as long as 40 draws of a path), fewer fill the
+// schedulers.  Device time of a European on 50 steps with 1, 2 and 4 paths a
+// lane: 109, 109, 120 us at 50,000 paths; 157, 136, 147 at 100,000; 244, 211,
+// 195 at 200,000.
+int lsm_lane_paths(int64_t n) { return n < 60000 ? 1 : n < 150000 ? 2 : 4; }
+
+}  // namespace
+
 static of_status lsm_validate(of_ctx* ctx, const of_lsm_contract* k, int64_t paths) {
   if (k->option_type != OF_CALL && k->option_type != OF_PUT)
     return of_fail(ctx, OF_ERR_INVALID_INPUT, "unknown option type %d", k->option_type);
@@ -1326,16 +1853,20 @@ void fill_steps(LsmHost& h, int64_t steps, double expiry, const double* strike_o
   }
 }
 
-// Offsets of a run's tables in its auxiliary device block.
+// Offsets of a run's tables in its auxiliary device block.  The block begins
+// with an image of the pinned staging, uploaded in one copy: the tables, then
+// the counters and statistics at their initial values; its end, from `back`
+// on, holds the results and is read back in one copy.
 struct DevOffsets {
-  size_t part = 0, beta = 0, res = 0, c = 0, ok = 0, reg = 0, cnt = 0, can = 0, st = 0, exc = 0, exb = 0, itm = 0,
-         term = 0, dpow = 0, status = 0;
+  size_t c = 0, can = 0, st = 0, dpow = 0, ok = 0, cnt = 0;
+  size_t back = 0, reg = 0, status = 0, res = 0, exc = 0, exb = 0, itm = 0, term = 0, image = 0;
+  size_t part = 0, beta = 0, states = 0, rows = 0;  // beyond the image
 };
 
 // One batch of contracts sharing a step count, staged for an asynchronous
-// run on one of two device buffer sets: pinned host images of its tables
-// (uploaded when enqueued) and of its results (read back when enqueued, used
-// once the streams have drained).
+// run on one of two device buffer sets.  The pinned image carries its tables
+// up (uploaded when enqueued) and its results back (used once the streams
+// have drained).
 struct LsmRun {
   std::vector<LsmHost> hs;
   int64_t steps = 0;
@@ -1347,18 +1878,14 @@ struct LsmRun {
   LsmBatch B{};
   DevOffsets dev;
   void* d_inj = nullptr;
-  char* pin = nullptr;  // pinned staging, laid out by the o_* offsets
-  size_t o_hc = 0, o_can = 0, o_st = 0, o_dpow = 0, o_bits0 = 0, o_res = 0, o_reg = 0, o_status = 0, o_cnt = 0,
-         o_bits = 0, o_itm = 0, o_term = 0;
-  std::vector<size_t> o_lvh;  // [nc][4] staging offsets of the local-vol arrays
-  std::vector<size_t> o_lvd;  // [nc][4] their offsets in the auxiliary device block
+  char* pin = nullptr;        // the image in the context's staging memory
+  std::vector<size_t> o_lv;  // [nc][4] offsets of the local-vol arrays in the image
   size_t aux_bytes = 0, path_bytes = 0, value_bytes = 0;
   cudaEvent_t gen_done = nullptr, done = nullptr;
   LsmRun() = default;
   LsmRun(const LsmRun&) = delete;
   LsmRun& operator=(const LsmRun&) = delete;
   ~LsmRun() {
-    if (pin) cudaFreeHost(pin);
     if (gen_done) cudaEventDestroy(gen_done);
     if (done) cudaEventDestroy(done);
   }
@@ -1389,29 +1916,37 @@ void lsm_layout(LsmRun& r, const of_lsm_config* cfg) {
     return o;
   };
   DevOffsets& d = r.dev;
-  d.part = take((size_t)nc * blocks * kMaxMoments * sizeof(double));
-  d.beta = take((size_t)nc * 8 * sizeof(double));
-  d.res = take((size_t)nc * 3 * sizeof(double));
   d.c = take((size_t)nc * sizeof(LsmC));
-  d.ok = take((size_t)nc * 2 * sizeof(int32_t));
-  d.reg = take((size_t)nc * sizeof(int32_t));
-  d.cnt = take((size_t)nc * sizeof(uint32_t));
   d.can = take(ns);
   d.st = take(ns * sizeof(LsmStep));
-  d.exc = take(ns * sizeof(unsigned long long));
-  d.exb = take(ns * sizeof(unsigned long long));
-  d.itm = take(ns * sizeof(double));
-  d.term = take((size_t)nc * sizeof(unsigned long long));
   d.dpow = take(ns * sizeof(double));
-  d.status = take(sizeof(uint32_t));
-  r.o_lvd.assign((size_t)nc * 4, 0);
+  r.o_lv.assign((size_t)nc * 4, 0);
   for (int c = 0; c < nc; ++c) {
     const size_t nk = r.hs[(size_t)c].lv_k.size(), nv = r.hs[(size_t)c].lv_v.size();
     if (!nk) continue;
-    r.o_lvd[(size_t)c * 4 + 0] = take(nk * sizeof(double));
-    r.o_lvd[(size_t)c * 4 + 1] = take(nv * sizeof(double));
-    r.o_lvd[(size_t)c * 4 + 2] = take(nk * sizeof(float));
-    r.o_lvd[(size_t)c * 4 + 3] = take(nv * sizeof(float));
+    r.o_lv[(size_t)c * 4 + 0] = take(nk * sizeof(double));
+    r.o_lv[(size_t)c * 4 + 1] = take(nv * sizeof(double));
+    r.o_lv[(size_t)c * 4 + 2] = take(nk * sizeof(float));
+    r.o_lv[(size_t)c * 4 + 3] = take(nv * sizeof(float));
+  }
+  d.ok = take((size_t)nc * 2 * sizeof(int32_t));
+  d.cnt = take((size_t)nc * sizeof(uint32_t));
+  d.back = off;
+  d.reg = take((size_t)nc * sizeof(int32_t));
+  d.status = take(sizeof(uint32_t));
+  d.res = take((size_t)nc * 3 * sizeof(double));
+  const size_t nt = r.track ? ns : 0;
+  d.exc = take(nt * sizeof(unsigned long long));
+  d.exb = take(nt * sizeof(unsigned long long));
+  d.itm = take(nt * sizeof(double));
+  d.term = take(r.track ? (size_t)nc * sizeof(unsigned long long) : 0);
+  d.image = off;
+  d.part = take((size_t)nc * blocks * kMaxMoments * sizeof(double));
+  d.beta = take((size_t)nc * 8 * sizeof(double));
+  if (fp64) {
+    const int64_t groups = (N + 1023) / 1024;  // at least one path a lane
+    d.states = take((size_t)(kSetupColumns + groups) * 4 * sizeof(uint64_t));
+    d.rows = take((size_t)2 * kMaxRows * kRowWords * 16);
   }
   r.aux_bytes = off;
   LsmBatch& B = r.B;
@@ -1429,15 +1964,17 @@ void lsm_layout(LsmRun& r, const of_lsm_config* cfg) {
   B.chunk = 8;
 }
 
-// Points a laid-out run at its device buffers, fills its pinned staging and
-// creates its events.
+// Points a laid-out run at its device buffers and its part of the staging
+// memory (r.dev.image bytes), fills that, and creates its events where it
+// shares the device with another batch.
 of_status lsm_bind(of_ctx* ctx, LsmRun& r, const of_lsm_config* cfg, void* dS, void* dVal, void* dAux,
-                   const uint64_t* jump) {
+                   const uint64_t* jump, void* staging, bool events) {
   const bool fp64 = cfg->precision == OF_PREC_FP64_REFERENCE;
   const size_t esz = fp64 ? sizeof(double) : sizeof(float);
   const int nc = r.nc();
   const size_t ns = r.ns();
   const int dyn = r.hs[0].C.dynamics;
+  r.pin = (char*)staging;
   for (const LsmHost& h : r.hs)
     if (h.C.dynamics != dyn) return of_fail(ctx, OF_ERR_INVALID_INPUT, "an LSM batch mixes path dynamics");
   LsmBatch& B = r.B;
@@ -1458,46 +1995,18 @@ of_status lsm_bind(of_ctx* ctx, LsmRun& r, const of_lsm_config* cfg, void* dS, v
   B.term_itm = (unsigned long long*)(a + d.term);
   B.disc_pow = (const double*)(a + d.dpow);
   B.status = (uint32_t*)(a + d.status);
+  B.states = (const uint64_t*)(a + d.states);
+  B.rows = a + d.rows;
   B.S = dS;
   B.V = dVal;
   B.tau = fp64 ? (int32_t*)((char*)dVal + (size_t)nc * B.npad * esz) : nullptr;
   B.exflags = fp64 ? nullptr : (uint32_t*)((char*)dVal + (size_t)nc * B.npad * esz);
   B.jump = jump;
-  size_t off = 0;
-  auto take = [&off](size_t bytes) {
-    const size_t o = off;
-    off = (off + bytes + 15) & ~(size_t)15;
-    return o;
-  };
-  r.o_hc = take((size_t)nc * sizeof(LsmC));
-  r.o_can = take(ns);
-  r.o_st = take(ns * sizeof(LsmStep));
-  r.o_dpow = take(ns * sizeof(double));
-  r.o_bits0 = take(r.track ? ns * sizeof(unsigned long long) : 0);
-  r.o_lvh.assign((size_t)nc * 4, 0);
-  for (int c = 0; c < nc; ++c) {
-    const size_t nk = r.hs[(size_t)c].lv_k.size(), nv = r.hs[(size_t)c].lv_v.size();
-    if (!nk) continue;
-    r.o_lvh[(size_t)c * 4 + 0] = take(nk * sizeof(double));
-    r.o_lvh[(size_t)c * 4 + 1] = take(nv * sizeof(double));
-    r.o_lvh[(size_t)c * 4 + 2] = take(nk * sizeof(float));
-    r.o_lvh[(size_t)c * 4 + 3] = take(nv * sizeof(float));
-  }
-  r.o_res = take((size_t)nc * 3 * sizeof(double));
-  r.o_reg = take((size_t)nc * sizeof(int32_t));
-  r.o_status = take(sizeof(uint32_t));
-  r.o_cnt = take(r.track ? ns * sizeof(unsigned long long) : 0);
-  r.o_bits = take(r.track ? ns * sizeof(unsigned long long) : 0);
-  r.o_itm = take(r.track ? ns * sizeof(double) : 0);
-  r.o_term = take(r.track ? (size_t)nc * sizeof(unsigned long long) : 0);
-  if (cudaMallocHost(&r.pin, off) != cudaSuccess) {
-    r.pin = nullptr;
-    return of_fail(ctx, OF_ERR_ALLOC, "LSM staging allocation failed");
-  }
-  LsmC* hc = (LsmC*)(r.pin + r.o_hc);
-  uint8_t* can = (uint8_t*)(r.pin + r.o_can);
-  LsmStep* st = (LsmStep*)(r.pin + r.o_st);
-  double* dpow = (double*)(r.pin + r.o_dpow);
+  std::memset(r.pin, 0, d.image);
+  LsmC* hc = (LsmC*)(r.pin + r.dev.c);
+  uint8_t* can = (uint8_t*)(r.pin + r.dev.can);
+  LsmStep* st = (LsmStep*)(r.pin + r.dev.st);
+  double* dpow = (double*)(r.pin + r.dev.dpow);
   for (int c = 0; c < nc; ++c) {
     const LsmHost& h = r.hs[(size_t)c];
     LsmC C = h.C;
@@ -1510,74 +2019,79 @@ of_status lsm_bind(of_ctx* ctx, LsmRun& r, const of_lsm_config* cfg, void* dS, v
     dp[0] = 1.0;
     for (int64_t k = 1; k <= r.steps; ++k) dp[k] = dp[k - 1] * h.C.disc;
     if (!h.lv_k.empty()) {
-      C.lv_k = (const double*)(a + r.o_lvd[(size_t)c * 4 + 0]);
-      C.lv_v = (const double*)(a + r.o_lvd[(size_t)c * 4 + 1]);
-      C.lv_kf = (const float*)(a + r.o_lvd[(size_t)c * 4 + 2]);
-      C.lv_vf = (const float*)(a + r.o_lvd[(size_t)c * 4 + 3]);
+      C.lv_k = (const double*)(a + r.o_lv[(size_t)c * 4 + 0]);
+      C.lv_v = (const double*)(a + r.o_lv[(size_t)c * 4 + 1]);
+      C.lv_kf = (const float*)(a + r.o_lv[(size_t)c * 4 + 2]);
+      C.lv_vf = (const float*)(a + r.o_lv[(size_t)c * 4 + 3]);
       C.lv_nk = (int32_t)h.lv_k.size();
-      std::copy(h.lv_k.begin(), h.lv_k.end(), (double*)(r.pin + r.o_lvh[(size_t)c * 4 + 0]));
-      std::copy(h.lv_v.begin(), h.lv_v.end(), (double*)(r.pin + r.o_lvh[(size_t)c * 4 + 1]));
-      std::copy(h.lv_k.begin(), h.lv_k.end(), (float*)(r.pin + r.o_lvh[(size_t)c * 4 + 2]));
-      std::copy(h.lv_v.begin(), h.lv_v.end(), (float*)(r.pin + r.o_lvh[(size_t)c * 4 + 3]));
+      std::copy(h.lv_k.begin(), h.lv_k.end(), (double*)(r.pin + r.o_lv[(size_t)c * 4 + 0]));
+      std::copy(h.lv_v.begin(), h.lv_v.end(), (double*)(r.pin + r.o_lv[(size_t)c * 4 + 1]));
+      std::copy(h.lv_k.begin(), h.lv_k.end(), (float*)(r.pin + r.o_lv[(size_t)c * 4 + 2]));
+      std::copy(h.lv_v.begin(), h.lv_v.end(), (float*)(r.pin + r.o_lv[(size_t)c * 4 + 3]));
     }
     hc[c] = C;
   }
   if (r.track) {
-    unsigned long long* bits0 = (unsigned long long*)(r.pin + r.o_bits0);
+    unsigned long long* bits0 = (unsigned long long*)(r.pin + r.dev.exb);
     for (int c = 0; c < nc; ++c)  // identity of max (put) / min (call) over positive doubles
       std::fill(bits0 + (size_t)c * (r.steps + 1), bits0 + (size_t)(c + 1) * (r.steps + 1),
                 r.hs[(size_t)c].C.put ? 0ULL : 0x7FF0000000000000ULL);
   }
+  if (!events) return OF_OK;
   if (cudaEventCreateWithFlags(&r.gen_done, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&r.done, cudaEventDisableTiming) != cudaSuccess)
     return of_fail(ctx, OF_ERR_CUDA, "LSM event creation failed");
   return OF_OK;
 }
 
-// Enqueues a bound run: its tables, the path generation and the `gen_done`
-// event on `gs`; on `ms`, after `gen_done`, the passes, the final kernel, the
-// readback of the results into the pinned staging and the `done` event.
+// Whether a run's FP64 paths stay in the range of lsm_gen_stream's exponential
+// (|log-spot| < 690; a sum of normals beyond 40 standard deviations has
+// probability below 1e-300).  Heston's log-spot is clamped in the kernel.
+bool lsm_log_space(const LsmRun& r) {
+  if (r.inj_host) return false;
+  const double n = (double)r.steps;
+  for (const LsmHost& h : r.hs) {
+    const LsmC& C = h.C;
+    double spread = 0.0, drift = 0.0;
+    if (C.dynamics == DYN_GBM) {
+      spread = C.step_vol;
+      drift = std::fabs(C.drift);
+    } else if (C.dynamics == DYN_LOCAL_VOL) {
+      const double vol = *std::max_element(h.lv_v.begin(), h.lv_v.end());
+      spread = vol * C.sqrt_dt;
+      drift = (std::fabs(C.mu) + 0.5 * vol * vol) * C.dt;
+    }
+    if (!(40.0 * spread * std::sqrt(n) + drift * n < 600.0)) return false;
+  }
+  return true;
+}
+
+// Enqueues a bound run: its image and the path generation on `gs`; on `ms`,
+// after them, the passes, the final kernel and the readback of the results
+// into the image (then the `done` event, for a batch with events).
 of_status lsm_enqueue(of_ctx* ctx, LsmRun& r, const of_lsm_config* cfg, cudaStream_t gs, cudaStream_t ms) {
   const bool fp64 = cfg->precision == OF_PREC_FP64_REFERENCE;
   const int nc = r.nc();
-  const size_t ns = r.ns();
   LsmBatch& B = r.B;
-  OF_CUDA_TRY(ctx, cudaMemcpyAsync((void*)B.c, r.pin + r.o_hc, (size_t)nc * sizeof(LsmC), cudaMemcpyHostToDevice, gs));
-  OF_CUDA_TRY(ctx, cudaMemcpyAsync((void*)B.can_ex, r.pin + r.o_can, ns, cudaMemcpyHostToDevice, gs));
-  OF_CUDA_TRY(ctx, cudaMemcpyAsync((void*)B.st, r.pin + r.o_st, ns * sizeof(LsmStep), cudaMemcpyHostToDevice, gs));
-  OF_CUDA_TRY(ctx, cudaMemcpyAsync((void*)B.disc_pow, r.pin + r.o_dpow, ns * sizeof(double), cudaMemcpyHostToDevice,
-                                   gs));
-  const LsmC* hc = (const LsmC*)(r.pin + r.o_hc);
-  for (int c = 0; c < nc; ++c) {
-    const LsmHost& h = r.hs[(size_t)c];
-    if (h.lv_k.empty()) continue;
-    const size_t nk = h.lv_k.size(), nv = h.lv_v.size();
-    OF_CUDA_TRY(ctx, cudaMemcpyAsync((void*)hc[c].lv_k, r.pin + r.o_lvh[(size_t)c * 4 + 0], nk * sizeof(double),
-                                     cudaMemcpyHostToDevice, gs));
-    OF_CUDA_TRY(ctx, cudaMemcpyAsync((void*)hc[c].lv_v, r.pin + r.o_lvh[(size_t)c * 4 + 1], nv * sizeof(double),
-                                     cudaMemcpyHostToDevice, gs));
-    OF_CUDA_TRY(ctx, cudaMemcpyAsync((void*)hc[c].lv_kf, r.pin + r.o_lvh[(size_t)c * 4 + 2], nk * sizeof(float),
-                                     cudaMemcpyHostToDevice, gs));
-    OF_CUDA_TRY(ctx, cudaMemcpyAsync((void*)hc[c].lv_vf, r.pin + r.o_lvh[(size_t)c * 4 + 3], nv * sizeof(float),
-                                     cudaMemcpyHostToDevice, gs));
-  }
-  OF_CUDA_TRY(ctx, cudaMemsetAsync(B.beta_ok, 0, (size_t)nc * 2 * sizeof(int32_t), gs));
-  OF_CUDA_TRY(ctx, cudaMemsetAsync(B.regress_count, 0, (size_t)nc * sizeof(int32_t), gs));
-  OF_CUDA_TRY(ctx, cudaMemsetAsync(B.counters, 0, (size_t)nc * sizeof(uint32_t), gs));
-  OF_CUDA_TRY(ctx, cudaMemsetAsync(B.status, 0, sizeof(uint32_t), gs));
-  if (r.track) {
-    OF_CUDA_TRY(ctx, cudaMemsetAsync(B.ex_count, 0, ns * sizeof(unsigned long long), gs));
-    OF_CUDA_TRY(ctx, cudaMemcpyAsync(B.ex_bits, r.pin + r.o_bits0, ns * sizeof(unsigned long long),
-                                     cudaMemcpyHostToDevice, gs));
-    OF_CUDA_TRY(ctx, cudaMemsetAsync(B.itm_count, 0, ns * sizeof(double), gs));
-    OF_CUDA_TRY(ctx, cudaMemsetAsync(B.term_itm, 0, (size_t)nc * sizeof(unsigned long long), gs));
-  }
+  OF_CUDA_TRY(ctx, cudaMemcpyAsync((void*)B.c, r.pin, r.dev.image, cudaMemcpyHostToDevice, gs));
   if (r.inj_host) {
     const size_t cnt = (size_t)B.n * r.steps * r.draws;
     OF_CUDA_TRY(ctx, cudaMemcpyAsync(r.d_inj, r.inj_host, cnt * sizeof(double), cudaMemcpyHostToDevice, gs));
     B.inj = (const double*)r.d_inj;
   }
-  if (fp64) {
+  const int back_ppt = fp64 ? lsm_back_ppt(ctx, B.n, nc) : 0;
+  if (fp64 && lsm_log_space(r)) {
+    B.lane_paths = lsm_lane_paths(B.n);
+    const int64_t warps = (B.n + 32 * B.lane_paths - 1) / (32 * B.lane_paths);
+    const uint64_t lane_draws = (uint64_t)B.lane_paths * (uint64_t)r.steps * (uint64_t)r.draws;
+    const int64_t groups = (warps + 31) / 32, setup = (kSetupColumns + groups) * 32;
+    lsm_stream_setup<<<(unsigned)((setup + kSetupThreads - 1) / kSetupThreads), kSetupThreads, 0, gs>>>(
+        B.seed, lane_draws, (int)groups, B.jump, (uint32_t*)B.states);
+    const int dyn = r.hs[0].C.dynamics;
+    void (*gen)(LsmBatch) = dyn == DYN_HESTON ? lsm_gen_stream<DYN_HESTON>
+                            : dyn == DYN_LOCAL_VOL ? lsm_gen_stream<DYN_LOCAL_VOL> : lsm_gen_stream<DYN_GBM>;
+    gen<<<dim3((unsigned)((warps * 32 + kGenThreads - 1) / kGenThreads), nc), kGenThreads, 0, gs>>>(B);
+  } else if (fp64) {
     const int64_t chunks = (B.n + B.chunk - 1) / B.chunk;
     lsm_gen_ref<<<dim3((unsigned)((chunks + 127) / 128), nc), 128, 0, gs>>>(B);
   } else {
@@ -1587,9 +2101,12 @@ of_status lsm_enqueue(of_ctx* ctx, LsmRun& r, const of_lsm_config* cfg, cudaStre
                             : dyn == DYN_LOCAL_VOL ? lsm_gen_philox<DYN_LOCAL_VOL> : lsm_gen_philox<DYN_GBM>;
     gen<<<dim3((unsigned)((quads + 255) / 256), nc), 256, 0, gs>>>(B);
   }
+  if (fp64 && !back_ppt) lsm_terminal_ref<<<dim3((unsigned)((B.n + 255) / 256), nc), 256, 0, gs>>>(B);
   OF_CUDA_TRY(ctx, cudaGetLastError());
-  OF_CUDA_TRY(ctx, cudaEventRecord(r.gen_done, gs));
-  OF_CUDA_TRY(ctx, cudaStreamWaitEvent(ms, r.gen_done, 0));
+  if (gs != ms) {
+    OF_CUDA_TRY(ctx, cudaEventRecord(r.gen_done, gs));
+    OF_CUDA_TRY(ctx, cudaStreamWaitEvent(ms, r.gen_done, 0));
+  }
   // The passes: one wave of resident blocks over the whole batch, each block
   // striding over its contract's chunks.
   void (*pass)(LsmBatch, int) = fp64 ? (B.degree == 2 ? lsm_pass<double, 2> : lsm_pass<double, 3>)
@@ -1612,7 +2129,15 @@ of_status lsm_enqueue(of_ctx* ctx, LsmRun& r, const of_lsm_config* cfg, cudaStre
     if (fill >= 0.95 || bpc == B.blocks) break;
   }
   const dim3 pgrid((unsigned)pass_blocks, nc);
-  if (fp64) {
+  if (back_ppt) {
+    const int64_t per = (int64_t)kBackThreads * back_ppt;
+    const unsigned bpc = (unsigned)((B.n + per - 1) / per);
+    // no date number may be left from another launch
+    OF_CUDA_TRY(ctx, cudaMemsetAsync(B.rows, 0, (size_t)2 * nc * bpc * kRowWords * 16, ms));
+    void* args[] = {(void*)&B};
+    OF_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void*)lsm_back_kernel(B.degree, back_ppt),
+                                                 dim3(bpc, nc), dim3(kBackThreads), args, 0, ms));
+  } else if (fp64) {
     for (int t = (int)r.steps - 1; t >= 1; --t) pass<<<pgrid, kPassThreads, 0, ms>>>(B, t);
   } else {
     // FP32 passes: programmatic dependent launches (lsm_pass_f32 waits on its
@@ -1630,21 +2155,12 @@ of_status lsm_enqueue(of_ctx* ctx, LsmRun& r, const of_lsm_config* cfg, cudaStre
     for (int t = (int)r.steps - 1; t >= 1; --t) OF_CUDA_TRY(ctx, cudaLaunchKernelEx(&lc, pass, B, t));
   }
   const dim3 grid((unsigned)B.blocks, nc);
-  if (fp64) lsm_final<double><<<grid, kPassThreads, 0, ms>>>(B);
-  else lsm_final<float><<<grid, kPassThreads, 0, ms>>>(B);
+  if (fp64 && !back_ppt) lsm_final<double><<<grid, kPassThreads, 0, ms>>>(B);
+  else if (!fp64) lsm_final<float><<<grid, kPassThreads, 0, ms>>>(B);
   OF_CUDA_TRY(ctx, cudaGetLastError());
-  OF_CUDA_TRY(ctx, cudaMemcpyAsync(r.pin + r.o_res, B.results, (size_t)nc * 3 * sizeof(double), cudaMemcpyDeviceToHost,
-                                   ms));
-  OF_CUDA_TRY(ctx, cudaMemcpyAsync(r.pin + r.o_reg, B.regress_count, (size_t)nc * sizeof(int32_t),
+  OF_CUDA_TRY(ctx, cudaMemcpyAsync(r.pin + r.dev.back, (char*)B.c + r.dev.back, r.dev.image - r.dev.back,
                                    cudaMemcpyDeviceToHost, ms));
-  OF_CUDA_TRY(ctx, cudaMemcpyAsync(r.pin + r.o_status, B.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ms));
-  if (r.track) {
-    OF_CUDA_TRY(ctx, cudaMemcpyAsync(r.pin + r.o_cnt, B.ex_count, ns * 8, cudaMemcpyDeviceToHost, ms));
-    OF_CUDA_TRY(ctx, cudaMemcpyAsync(r.pin + r.o_bits, B.ex_bits, ns * 8, cudaMemcpyDeviceToHost, ms));
-    OF_CUDA_TRY(ctx, cudaMemcpyAsync(r.pin + r.o_itm, B.itm_count, ns * 8, cudaMemcpyDeviceToHost, ms));
-    OF_CUDA_TRY(ctx, cudaMemcpyAsync(r.pin + r.o_term, B.term_itm, (size_t)nc * 8, cudaMemcpyDeviceToHost, ms));
-  }
-  OF_CUDA_TRY(ctx, cudaEventRecord(r.done, ms));
+  if (r.done) OF_CUDA_TRY(ctx, cudaEventRecord(r.done, ms));
   return OF_OK;
 }
 
@@ -1653,24 +2169,26 @@ of_status lsm_enqueue(of_ctx* ctx, LsmRun& r, const of_lsm_config* cfg, cudaStre
 of_status lsm_collect(of_ctx* ctx, const LsmRun& r, std::vector<double>& results, std::vector<int32_t>& regs,
                       std::vector<LsmTrack>* track) {
   const int nc = r.nc();
-  const uint32_t status = *(const uint32_t*)(r.pin + r.o_status);
+  const uint32_t status = *(const uint32_t*)(r.pin + r.dev.status);
   if (status & 2u) {
     ctx->unusable = true;
     return of_fail(ctx, OF_ERR_TIMEOUT,
                    "LSM pass: a bulk copy into shared memory did not complete in time and could not be drained; "
                    "the context is unusable: destroy it and create a new one");
   }
+  if (status & 4u)
+    return of_fail(ctx, OF_ERR_TIMEOUT, "LSM backward induction: a wait for the other blocks did not complete in time");
   if (status)
     return of_fail(ctx, OF_ERR_TIMEOUT, "LSM pass: a bulk copy into shared memory did not complete in time");
-  const double* hres = (const double*)(r.pin + r.o_res);
-  const int32_t* hreg = (const int32_t*)(r.pin + r.o_reg);
+  const double* hres = (const double*)(r.pin + r.dev.res);
+  const int32_t* hreg = (const int32_t*)(r.pin + r.dev.reg);
   results.assign(hres, hres + (size_t)nc * 3);
   regs.assign(hreg, hreg + nc);
   if (track && r.track) {
-    const unsigned long long* hcnt = (const unsigned long long*)(r.pin + r.o_cnt);
-    const unsigned long long* hbits = (const unsigned long long*)(r.pin + r.o_bits);
-    const double* hitm = (const double*)(r.pin + r.o_itm);
-    const unsigned long long* hterm = (const unsigned long long*)(r.pin + r.o_term);
+    const unsigned long long* hcnt = (const unsigned long long*)(r.pin + r.dev.exc);
+    const unsigned long long* hbits = (const unsigned long long*)(r.pin + r.dev.exb);
+    const double* hitm = (const double*)(r.pin + r.dev.itm);
+    const unsigned long long* hterm = (const unsigned long long*)(r.pin + r.dev.term);
     track->assign((size_t)nc, LsmTrack{});
     for (int c = 0; c < nc; ++c) {
       LsmTrack& tr = (*track)[(size_t)c];
@@ -1716,7 +2234,9 @@ of_status lsm_run_batch(of_ctx* ctx, std::vector<LsmHost>& hs, int64_t steps, co
   OF_TRY(of_scratch(ctx, SLOT_LSM_AUX, r.aux_bytes, &dAux));
   if (inj_host)
     OF_TRY(of_scratch(ctx, SLOT_INJECT, (size_t)cfg->num_paths * steps * draws * sizeof(double), &r.d_inj));
-  OF_TRY(lsm_bind(ctx, r, cfg, dS, dVal, dAux, jump));
+  void* pin = nullptr;
+  OF_TRY(of_pinned(ctx, r.dev.image, &pin));
+  OF_TRY(lsm_bind(ctx, r, cfg, dS, dVal, dAux, jump, pin, false));
   OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
   const of_status st = lsm_enqueue(ctx, r, cfg, ctx->stream, ctx->stream);
   if (st == OF_OK) OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream));
@@ -1821,6 +2341,7 @@ extern "C" of_status of_lsm_price(of_ctx* ctx, const of_lsm_contract* ks, int64_
       C.drift = (k.rate - k.dividend_yield - 0.5 * k.vol * k.vol) * dt;  // :452
       C.step_vol = k.vol * std::sqrt(dt);
       C.disc = std::exp(-k.rate * dt);
+      C.y_floor = std::log(1e-12 / k.spot);
       C.fdrift = (float)C.drift;
       C.fstep_vol = (float)C.step_vol;
       C.fspot = (float)k.spot;
@@ -1870,10 +2391,15 @@ extern "C" of_status of_lsm_price(of_ctx* ctx, const of_lsm_contract* ks, int64_
     for (int k = 0; k < 3; ++k) OF_TRY(of_scratch(ctx, slots[s][k], need[s][k], &dbuf[s][k]));
   void* d_inj = nullptr;
   if (inj_need) OF_TRY(of_scratch(ctx, SLOT_INJECT, inj_need, &d_inj));  // fed by the side stream, in order
+  size_t staging = 0;
+  for (const std::unique_ptr<LsmRun>& run : runs) staging += run->dev.image;
+  void* pin = nullptr;
+  OF_TRY(of_pinned(ctx, staging, &pin));
   for (size_t i = 0; i < runs.size(); ++i) {
     runs[i]->d_inj = d_inj;
     const int s = (int)(i % 2);
-    OF_TRY(lsm_bind(ctx, *runs[i], cfg, dbuf[s][0], dbuf[s][1], dbuf[s][2], jump));
+    OF_TRY(lsm_bind(ctx, *runs[i], cfg, dbuf[s][0], dbuf[s][1], dbuf[s][2], jump, pin, sets == 2));
+    pin = (char*)pin + runs[i]->dev.image;
   }
   const cudaStream_t ms = ctx->stream;
   cudaStream_t gs = ms;
@@ -2021,6 +2547,7 @@ extern "C" of_status of_lsm_bermudan(of_ctx* ctx, const of_bermudan_contract* k,
   C.drift = (mu - 0.5 * k->vol * k->vol) * dt;  // longstaff_schwartz.rs:205
   C.step_vol = k->vol * sqdt;
   C.disc = std::exp(-k->rate * dt);
+  C.y_floor = std::log(1e-12 / k->spot);
   C.mu = mu;
   C.dt = dt;
   C.sqrt_dt = sqdt;
