@@ -123,8 +123,8 @@ typedef struct of_mc_config {
   int32_t antithetic; /* 0/1 */
   int32_t precision; /* OF_PREC_* */
   int32_t control_variate; /* OF_CV_* */
-  int32_t tile_ilp; /* FP32 strip tile shape: 0 = default (1), 1 or 2 samples in flight per thread,
-                       3 = warp-specialised (half the warps generate the Philox draws into a
+  int32_t tile_ilp; /* FP32 strip tile shape: 1 or 2 samples in flight per thread, 0 = chosen by the
+                       sample count, 3 = warp-specialised (half the warps generate the Philox draws into a
                        shared-memory ring, half simulate and price) */
   double cv_expected; /* E[Y] of the control variate, undiscounted */
   double discount_factor;

@@ -588,8 +588,8 @@ __global__ void __launch_bounds__(256, DYN == DYN_GBM ? 4 : 2) lsm_gen_philox(co
         for (int q = 0; q < 4; ++q) {
           const uint32_t* w = &r[q].x;
           if (DYN == DYN_HESTON) {
-            const float2 z = of::normal_pair_scaled_from_u32(w[2 * k], w[2 * k + 1], C.hc.bm_k2);
-            of::heston_euler_step(L[q], C.hc, z.x, z.y);
+            const of::Polar z = of::polar_from_u32(w[2 * k], w[2 * k + 1], C.hc.bm_k2);
+            of::heston_euler_step(L[q], C.hc, z.q, z.c, z.s);
           } else {
             if ((k & 1) == 0) zp[q] = of::normal_pair_from_u32(w[k], w[k + 1]);
             const float z = (k & 1) ? zp[q].y : zp[q].x;

@@ -66,147 +66,115 @@ StepConsts make_consts(const of_model* m) {
   return c;
 }
 
-// Simulates the terminal log-return of sample i (and of its antithetic twin).
-template <int MODEL, bool ANTI>
-__device__ __forceinline__ void simulate_terminal(const StepConsts& c, int32_t steps, uint64_t i, uint32_t stream,
-                                                  const of::PhiloxKeys& K, float& ya, float& yb) {
-  LegState a{0.0f, c.v0}, b{0.0f, c.v0};
-  const uint32_t lo = (uint32_t)i, hi = (uint32_t)(i >> 32);
-  if (MODEL == OF_MODEL_GBM) {
-    float wa = 0.0f;  // sum of normals; y_T = steps*drift + diff*sum
-    for (int32_t j = 0; j < steps; j += 4) {
-      const uint4 r = of::philox4x32_10(make_uint4((uint32_t)(j >> 2), lo, hi, stream), K);
-      const float2 p = of::normal_pair_from_u32(r.x, r.y), q = of::normal_pair_from_u32(r.z, r.w);
-      wa += p.x;
-      if (j + 1 < steps) wa += p.y;
-      if (j + 2 < steps) wa += q.x;
-      if (j + 3 < steps) wa += q.y;
-    }
-    const float base = (float)steps * c.drift;
-    ya = fmaf(c.diff, wa, base);
-    yb = fmaf(-c.diff, wa, base);
-  } else if (MODEL == OF_MODEL_HESTON_EULER) {
-    const int32_t pairs = steps >> 1;  // full Philox calls; an odd last step below
-    for (int32_t q = 0; q < pairs; ++q) {
-      const uint4 r = of::philox4x32_10(make_uint4((uint32_t)q, lo, hi, stream), K);
-      float2 z = of::normal_pair_scaled_from_u32(r.x, r.y, c.bm_k2);
-      of::heston_euler_step(a, c, z.x, z.y);
-      if (ANTI) of::heston_euler_step(b, c, -z.x, -z.y);
-      z = of::normal_pair_scaled_from_u32(r.z, r.w, c.bm_k2);
-      of::heston_euler_step(a, c, z.x, z.y);
-      if (ANTI) of::heston_euler_step(b, c, -z.x, -z.y);
-    }
-    if (steps & 1) {
-      const uint4 r = of::philox4x32_10(make_uint4((uint32_t)pairs, lo, hi, stream), K);
-      const float2 z = of::normal_pair_scaled_from_u32(r.x, r.y, c.bm_k2);
-      of::heston_euler_step(a, c, z.x, z.y);
-      if (ANTI) of::heston_euler_step(b, c, -z.x, -z.y);
-    }
-    ya = a.y;
-    yb = b.y;
-  } else {
-    for (int32_t j = 0; j < steps; j += 2) {
-      const uint4 r = of::philox4x32_10(make_uint4((uint32_t)(j >> 1), lo, hi, stream), K);
-      float u = of::uniform_from_u32(r.x), zx = of::normal_from_u32(r.y);
-      of::heston_qe_step(a, c, u, 1.0f, zx, r.x);
-      if (ANTI) of::heston_qe_step(b, c, 1.0f - u, -1.0f, -zx, r.x);
-      if (j + 1 < steps) {
-        u = of::uniform_from_u32(r.z);
-        zx = of::normal_from_u32(r.w);
-        of::heston_qe_step(a, c, u, 1.0f, zx, r.z);
-        if (ANTI) of::heston_qe_step(b, c, 1.0f - u, -1.0f, -zx, r.z);
+// Simulates the terminal log-returns of ILP samples (and of their antithetic
+// twins) in one loop: the Philox rounds of the samples are separate dependency
+// chains, so their instructions interleave and fill the gaps of one chain, and
+// they share each counter block's q terms.  Two samples run in packed pairs
+// (each half the one-sample loop's arithmetic, bit for bit) except Heston's
+// antithetic ones, whose four legs fit the register budget without the pair
+// alignment, and QE.
+// FULL: the q table covers every counter block.
+template <int MODEL, bool ANTI, int ILP, bool FULL>
+__device__ __forceinline__ void simulate_terminal(const StepConsts& c, int32_t steps, const of::PhiloxLane (&L)[ILP],
+                                                  const of::PhiloxTab& T, const of::PhiloxKeys& K, float (&ya)[ILP],
+                                                  float (&yb)[ILP]) {
+  if constexpr (MODEL == OF_MODEL_GBM) {
+    // y_T = steps drift + diff sum z; each Box-Muller pair enters as its sum
+    // (normal_pair_sum_from_u32), four steps a counter block
+    float2 w = make_float2(0.0f, 0.0f);  // ILP 1: the sums of the block's two pairs; ILP 2: of the two samples
+    const int32_t full = steps >> 2;
+    for (int32_t q = 0; q < full; ++q) {
+      const uint4 t = of::philox_terms<FULL>(T, (uint32_t)q, K);
+      const uint4 r = of::philox_block(t, L[0], K);
+      if constexpr (ILP == 1) {
+        w = of::add2(w, of::normal_pair_sums2_from_u32(r.x, r.y, r.z, r.w));
+      } else {
+        const uint4 r1 = of::philox_block(t, L[1], K);
+        w = of::add2(w, of::add2(of::normal_pair_sums2_from_u32(r.x, r.y, r1.x, r1.y),
+                                 of::normal_pair_sums2_from_u32(r.z, r.w, r1.z, r1.w)));
       }
     }
-    ya = a.y;
-    yb = b.y;
-  }
-}
-
-// ILP independent samples advanced in the same loop by one thread: the
-// Philox rounds of the samples are separate dependency chains, so their
-// instructions interleave and fill the fixed-latency gaps of one chain.
-template <int MODEL, bool ANTI, int ILP>
-__device__ __forceinline__ void simulate_terminal_n(const StepConsts& c, int32_t steps, const uint64_t (&idx)[ILP],
-                                                    uint32_t stream, const of::PhiloxKeys& K, float (&ya)[ILP],
-                                                    float (&yb)[ILP]) {
-  if (ILP == 1) {
-    simulate_terminal<MODEL, ANTI>(c, steps, idx[0], stream, K, ya[0], yb[0]);
-    return;
-  }
-  uint32_t lo[ILP], hi[ILP];
-#pragma unroll
-  for (int l = 0; l < ILP; ++l) {
-    lo[l] = (uint32_t)idx[l];
-    hi[l] = (uint32_t)(idx[l] >> 32);
-  }
-  if (MODEL == OF_MODEL_GBM) {
-    float w[ILP];
-#pragma unroll
-    for (int l = 0; l < ILP; ++l) w[l] = 0.0f;
-    for (int32_t j = 0; j < steps; j += 4) {
+    float sum[ILP];
+    if constexpr (ILP == 1) {
+      sum[0] = w.x + w.y;
+    } else {
+      sum[0] = w.x;
+      sum[1] = w.y;
+    }
+    if (const int32_t rem = steps & 3) {
+      const uint4 t = of::philox_terms<FULL>(T, (uint32_t)full, K);
 #pragma unroll
       for (int l = 0; l < ILP; ++l) {
-        const uint4 r = of::philox4x32_10(make_uint4((uint32_t)(j >> 2), lo[l], hi[l], stream), K);
-        const float2 p = of::normal_pair_from_u32(r.x, r.y), q = of::normal_pair_from_u32(r.z, r.w);
-        w[l] += p.x;
-        if (j + 1 < steps) w[l] += p.y;
-        if (j + 2 < steps) w[l] += q.x;
-        if (j + 3 < steps) w[l] += q.y;
+        const uint4 r = of::philox_block(t, L[l], K);
+        if (rem == 1) {
+          sum[l] += of::normal_pair_from_u32(r.x, r.y).x;
+        } else {
+          sum[l] += of::normal_pair_sum_from_u32(r.x, r.y);
+          if (rem == 3) sum[l] += of::normal_pair_from_u32(r.z, r.w).x;
+        }
       }
     }
     const float base = (float)steps * c.drift;
 #pragma unroll
     for (int l = 0; l < ILP; ++l) {
-      ya[l] = fmaf(c.diff, w[l], base);
-      yb[l] = fmaf(-c.diff, w[l], base);
+      ya[l] = fmaf(c.diff, sum[l], base);
+      yb[l] = fmaf(-c.diff, sum[l], base);
     }
-  } else if (MODEL == OF_MODEL_HESTON_EULER && ILP == 2 && !ANTI) {
-    // the two samples' legs in packed pairs: each half is the one-sample
-    // loop's arithmetic, bit for bit (antithetic pairs keep the scalar loop,
-    // whose four legs fit the register budget without the pair alignment)
+  } else if constexpr (MODEL == OF_MODEL_HESTON_EULER && ILP == 2 && !ANTI) {
     of::LegState2 a{make_float2(0.0f, 0.0f), make_float2(c.v0, c.v0)};
-    const int32_t pairs = steps >> 1;
-    float2 w1, w2;
+    const int32_t pairs = steps >> 1;  // full Philox calls; an odd last step below
     for (int32_t q = 0; q < pairs; ++q) {
-      const uint4 r0 = of::philox4x32_10(make_uint4((uint32_t)q, lo[0], hi[0], stream), K);
-      const uint4 r1 = of::philox4x32_10(make_uint4((uint32_t)q, lo[1], hi[1], stream), K);
-      of::normal_pairs_scaled2_from_u32(r0.x, r0.y, r1.x, r1.y, c.bm_k2, w1, w2);
-      of::heston_euler_step2(a, c, w1, w2);
-      of::normal_pairs_scaled2_from_u32(r0.z, r0.w, r1.z, r1.w, c.bm_k2, w1, w2);
-      of::heston_euler_step2(a, c, w1, w2);
+      const uint4 t = of::philox_terms<FULL>(T, (uint32_t)q, K);
+      const uint4 r0 = of::philox_block(t, L[0], K), r1 = of::philox_block(t, L[1], K);
+      of::heston_euler_step2(a, c, of::polars2_from_u32(r0.x, r0.y, r1.x, r1.y, c.bm_k2));
+      of::heston_euler_step2(a, c, of::polars2_from_u32(r0.z, r0.w, r1.z, r1.w, c.bm_k2));
     }
     if (steps & 1) {
-      const uint4 r0 = of::philox4x32_10(make_uint4((uint32_t)pairs, lo[0], hi[0], stream), K);
-      const uint4 r1 = of::philox4x32_10(make_uint4((uint32_t)pairs, lo[1], hi[1], stream), K);
-      of::normal_pairs_scaled2_from_u32(r0.x, r0.y, r1.x, r1.y, c.bm_k2, w1, w2);
-      of::heston_euler_step2(a, c, w1, w2);
+      const uint4 t = of::philox_terms<FULL>(T, (uint32_t)pairs, K);
+      const uint4 r0 = of::philox_block(t, L[0], K), r1 = of::philox_block(t, L[1], K);
+      of::heston_euler_step2(a, c, of::polars2_from_u32(r0.x, r0.y, r1.x, r1.y, c.bm_k2));
     }
     ya[0] = a.y.x;  // yb stays 0: there is no antithetic leg
     ya[1] = a.y.y;
-  } else if (MODEL == OF_MODEL_HESTON_EULER) {
+  } else if constexpr (MODEL == OF_MODEL_HESTON_QE && ILP > 1) {  // one after the other: two QE samples spill
+    for (int l = 0; l < ILP; ++l) {
+      const of::PhiloxLane L1[1] = {L[l]};
+      float a1[1], b1[1];
+      simulate_terminal<MODEL, ANTI, 1, FULL>(c, steps, L1, T, K, a1, b1);
+      ya[l] = a1[0];
+      yb[l] = b1[0];
+    }
+  } else {
     LegState a[ILP], b[ILP];
 #pragma unroll
     for (int l = 0; l < ILP; ++l) a[l] = b[l] = LegState{0.0f, c.v0};
+    auto step = [&](int l, uint32_t r0, uint32_t r1) {
+      if (MODEL == OF_MODEL_HESTON_EULER) {
+        const of::Polar z = of::polar_from_u32(r0, r1, c.bm_k2);
+        of::heston_euler_step(a[l], c, z.q, z.c, z.s);
+        if (ANTI) of::heston_euler_step(b[l], c, z.q, -z.c, -z.s);
+      } else {
+        const float u = of::uniform_from_u32(r0), zx = of::normal_from_u32(r1);
+        of::heston_qe_step(a[l], c, u, 1.0f, zx, r0);
+        if (ANTI) of::heston_qe_step(b[l], c, 1.0f - u, -1.0f, -zx, r0);
+      }
+    };
     const int32_t pairs = steps >> 1;
     for (int32_t q = 0; q < pairs; ++q) {
+      const uint4 t = of::philox_terms<FULL>(T, (uint32_t)q, K);
 #pragma unroll
       for (int l = 0; l < ILP; ++l) {
-        const uint4 r = of::philox4x32_10(make_uint4((uint32_t)q, lo[l], hi[l], stream), K);
-        float2 z = of::normal_pair_scaled_from_u32(r.x, r.y, c.bm_k2);
-        of::heston_euler_step(a[l], c, z.x, z.y);
-        if (ANTI) of::heston_euler_step(b[l], c, -z.x, -z.y);
-        z = of::normal_pair_scaled_from_u32(r.z, r.w, c.bm_k2);
-        of::heston_euler_step(a[l], c, z.x, z.y);
-        if (ANTI) of::heston_euler_step(b[l], c, -z.x, -z.y);
+        const uint4 r = of::philox_block(t, L[l], K);
+        step(l, r.x, r.y);
+        step(l, r.z, r.w);
       }
     }
     if (steps & 1) {
+      const uint4 t = of::philox_terms<FULL>(T, (uint32_t)pairs, K);
 #pragma unroll
       for (int l = 0; l < ILP; ++l) {
-        const uint4 r = of::philox4x32_10(make_uint4((uint32_t)pairs, lo[l], hi[l], stream), K);
-        const float2 z = of::normal_pair_scaled_from_u32(r.x, r.y, c.bm_k2);
-        of::heston_euler_step(a[l], c, z.x, z.y);
-        if (ANTI) of::heston_euler_step(b[l], c, -z.x, -z.y);
+        const uint4 r = of::philox_block(t, L[l], K);
+        step(l, r.x, r.y);
       }
     }
 #pragma unroll
@@ -214,9 +182,6 @@ __device__ __forceinline__ void simulate_terminal_n(const StepConsts& c, int32_t
       ya[l] = a[l].y;
       yb[l] = b[l].y;
     }
-  } else {
-#pragma unroll
-    for (int l = 0; l < ILP; ++l) simulate_terminal<MODEL, ANTI>(c, steps, idx[l], stream, K, ya[l], yb[l]);
   }
 }
 
@@ -229,36 +194,111 @@ struct StripParams {
   int32_t steps, n_strikes, option_type, antithetic;
   float s0;
   of::PhiloxKeys keys;
-  const float* strikes;
   uint32_t* status;  // warp-specialised kernel: nonzero when a ring wait gave up
+  unsigned* ticket;  // last block adds the rows of partials into `out` (strip_fused), or null
+  double* out;       // [2 n_strikes]
+  float strikes[128];
 };
 
+// Whether the block that finishes last adds the blocks' rows: each of its
+// threads then adds rows / strip_row_groups of them, about 0.4 us per 16 (one
+// trip to the L2); past 96 a reduction launch with a block per column is
+// quicker.
+constexpr int kStripThreads = 256;
+__host__ __device__ inline int strip_row_groups(int cols) { return kStripThreads / cols < 8 ? kStripThreads / cols : 8; }
+inline bool strip_fused(int64_t grid, int cols) { return grid <= 96 * (int64_t)strip_row_groups(cols); }
+
+// The last block's part (called by all threads of every block): `sh` holds
+// strip_row_groups(cols) x cols doubles.
+__device__ __forceinline__ void strip_finish(const StripParams& P, int cols, const double* __restrict__ partials,
+                                             double* sh) {
+  __shared__ bool last;
+  __threadfence();  // this thread's columns of the block's row
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(P.ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int groups = strip_row_groups(cols);
+  if ((int)threadIdx.x < groups * cols) {
+    const int col = threadIdx.x % cols;
+    double acc = 0.0;
+    for (unsigned r = threadIdx.x / cols; r < gridDim.x; r += 16 * groups) {
+      double v[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const unsigned row = r + k * groups;
+        v[k] = row < gridDim.x ? __ldcg(partials + (size_t)row * cols + col) : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < 16; ++k) acc += v[k];
+    }
+    sh[threadIdx.x] = acc;
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < cols) {
+    double acc = 0.0;
+    for (int g = 0; g < groups; ++g) acc += sh[g * cols + threadIdx.x];
+    P.out[threadIdx.x] = acc;
+    __threadfence_system();
+  }
+  if (threadIdx.x == 0) *P.ticket = 0;
+}
+
+constexpr uint32_t kStripTab = 256;  // counter blocks in the strip's q table (4 KB)
+
+// KPL 0: one strike, whose sums each lane keeps for its own samples (no
+// shuffles; for one strike these took longer than 16 steps).
+//
+// What bounds it: the FMA pipe's heavy half, 75-80 % busy, with Philox's 15
+// wide products of four cycles per counter block and half of the FP32
+// operations.  At 2^20 samples x 256 steps x 41 strikes, four blocks per SM and
+// two samples per thread: Heston Euler 475 us (548 before the q tables, the
+// shared square root, the funnel shifts and the even rounds; 529 and 573 with
+// one sample per thread), GBM 217 (288).
 template <int KPL, int MODEL, bool ANTI, int ILP = 1>
-__global__ void __launch_bounds__(256, 5) strip_kernel(const __grid_constant__ StripParams P,
+__global__ void __launch_bounds__(kStripThreads, 4) strip_kernel(const __grid_constant__ StripParams P,
                                                     double* __restrict__ partials) {
   extern __shared__ double sh_strip[];  // [warps][n_strikes][2]
+  __shared__ uint4 qtab[kStripTab];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  float K[KPL];
-  of::Kahan32 s1[KPL], s2[KPL];
+  constexpr int KA = KPL > 0 ? KPL : 1;
+  float K[KA];
+  of::KahanSq32 acc[KA];
 #pragma unroll
-  for (int q = 0; q < KPL; ++q) {
-    const int k = lane + 32 * q;
+  for (int q = 0; q < KA; ++q) {
+    const int k = KPL > 0 ? lane + 32 * q : 0;
     K[q] = k < P.n_strikes ? P.strikes[k] : 0.0f;
   }
   const bool call = P.option_type == OF_CALL;
-  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  // a warp round covers 32*ILP consecutive samples: lane + 32*l for l < ILP
-  for (int64_t base = ((int64_t)blockIdx.x * blockDim.x + warp * 32) * ILP; base < P.samples;
-       base += nthreads * ILP) {
-    uint64_t idx[ILP];
+  constexpr int kSpb = MODEL == OF_MODEL_GBM ? 4 : 2;  // steps per counter block
+  const uint32_t nq = ((uint32_t)P.steps + kSpb - 1) / kSpb;
+  of::PhiloxTab T{qtab, nq < kStripTab ? nq : kStripTab, 0u, kStripStreamTag};
+  of::philox_table_fill(qtab, T.n, T.hi, T.stream, P.keys);
+  __syncthreads();
+  // a warp round covers 32*ILP consecutive samples: lane + 32*l for l < ILP.
+  // They share the high word of their index: 2^32 is a multiple of a round.
+  // Rounds go to warp 0 of every block, then warp 1 of every block, ...: a
+  // last partial round then loads every SM alike, wherever its blocks run
+  // (block by block, the busiest SM had 16 % more rounds than the mean).
+  const int64_t nwarps = (int64_t)gridDim.x * nw;
+  for (int64_t base = ((int64_t)warp * gridDim.x + blockIdx.x) * 32 * ILP; base < P.samples;
+       base += nwarps * 32 * ILP) {
+    of::PhiloxLane L[ILP];
     float ya[ILP], yb[ILP], sa[ILP], sb[ILP];
+    if (const uint32_t hi = (uint32_t)(base >> 32)) {  // past 2^32 samples: the table's hi is 0
+      T.hi = hi;
+      T.n = 0;
+    }
 #pragma unroll
     for (int l = 0; l < ILP; ++l) {
-      idx[l] = (uint64_t)(base + lane + 32 * l);
+      L[l] = of::philox_lane((uint32_t)(base + lane + 32 * l), T.hi, P.keys);
       ya[l] = yb[l] = 0.0f;
     }
-    if (base + lane < P.samples)  // lanes past the end skip the paths; their shuffled values are unused
-      simulate_terminal_n<MODEL, ANTI, ILP>(P.c, P.steps, idx, kStripStreamTag, P.keys, ya, yb);
+    if (base + lane < P.samples) {  // lanes past the end skip the paths; their shuffled values are unused
+      if (T.n == nq) simulate_terminal<MODEL, ANTI, ILP, true>(P.c, P.steps, L, T, P.keys, ya, yb);
+      else simulate_terminal<MODEL, ANTI, ILP, false>(P.c, P.steps, L, T, P.keys, ya, yb);
+    }
 #pragma unroll
     for (int l = 0; l < ILP; ++l) {
       sa[l] = P.s0 * __expf(ya[l]);
@@ -268,6 +308,12 @@ __global__ void __launch_bounds__(256, 5) strip_kernel(const __grid_constant__ S
     for (int l = 0; l < ILP; ++l) {
       const int64_t rem = P.samples - (base + 32 * l);
       const int nvalid = rem < 0 ? 0 : (rem < 32 ? (int)rem : 32);
+      if constexpr (KPL == 0) {
+        float x = fmaxf(call ? sa[l] - K[0] : K[0] - sa[l], 0.0f);
+        if (ANTI) x = 0.5f * (x + fmaxf(call ? sb[l] - K[0] : K[0] - sb[l], 0.0f));
+        if (lane < nvalid) acc[0].add(x);
+        continue;
+      }
       for (int j = 0; j < nvalid; ++j) {
         const float st = __shfl_sync(of::kFullMask, sa[l], j);
         const float sta = ANTI ? __shfl_sync(of::kFullMask, sb[l], j) : 0.0f;
@@ -275,27 +321,36 @@ __global__ void __launch_bounds__(256, 5) strip_kernel(const __grid_constant__ S
         for (int q = 0; q < KPL; ++q) {
           float x = fmaxf(call ? st - K[q] : K[q] - st, 0.0f);
           if (ANTI) x = 0.5f * (x + fmaxf(call ? sta - K[q] : K[q] - sta, 0.0f));
-          s1[q].add(x);
-          s2[q].add(x * x);
+          acc[q].add(x);
         }
       }
     }
   }
   const int n = P.n_strikes;
+  if constexpr (KPL == 0) {
+    double v[2] = {acc[0].value(), acc[0].square()};
+    of::block_sum<2>(v, sh_strip);
+    if (threadIdx.x == 0) {
+      partials[(int64_t)blockIdx.x * 2] = v[0];
+      partials[(int64_t)blockIdx.x * 2 + 1] = v[1];
+    }
+  } else {
 #pragma unroll
-  for (int q = 0; q < KPL; ++q) {
-    const int k = lane + 32 * q;
-    if (k < n) {
-      sh_strip[(warp * n + k) * 2] = s1[q].value();
-      sh_strip[(warp * n + k) * 2 + 1] = s2[q].value();
+    for (int q = 0; q < KPL; ++q) {
+      const int k = lane + 32 * q;
+      if (k < n) {
+        sh_strip[(warp * n + k) * 2] = acc[q].value();
+        sh_strip[(warp * n + k) * 2 + 1] = acc[q].square();
+      }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < 2 * n; t += blockDim.x) {
+      double sum = 0.0;
+      for (int w = 0; w < nw; ++w) sum += sh_strip[w * 2 * n + t];
+      partials[(int64_t)blockIdx.x * 2 * n + t] = sum;
     }
   }
-  __syncthreads();
-  for (int t = threadIdx.x; t < 2 * n; t += blockDim.x) {
-    double acc = 0.0;
-    for (int w = 0; w < nw; ++w) acc += sh_strip[w * 2 * n + t];
-    partials[(int64_t)blockIdx.x * 2 * n + t] = acc;
-  }
+  if (P.ticket) strip_finish(P, 2 * n, partials, sh_strip);
 }
 
 // ---------------------------------------------------------------------------
@@ -342,13 +397,13 @@ __device__ __forceinline__ void ws_consume(const StepConsts& c, const uint4 r, i
     if (j + 2 < steps) w += pq.x;
     if (j + 3 < steps) w += pq.y;
   } else if (MODEL == OF_MODEL_HESTON_EULER) {
-    float2 z = of::normal_pair_scaled_from_u32(r.x, r.y, c.bm_k2);
-    of::heston_euler_step(a, c, z.x, z.y);
-    if (ANTI) of::heston_euler_step(b, c, -z.x, -z.y);
+    of::Polar z = of::polar_from_u32(r.x, r.y, c.bm_k2);
+    of::heston_euler_step(a, c, z.q, z.c, z.s);
+    if (ANTI) of::heston_euler_step(b, c, z.q, -z.c, -z.s);
     if (2 * q + 1 < steps) {
-      z = of::normal_pair_scaled_from_u32(r.z, r.w, c.bm_k2);
-      of::heston_euler_step(a, c, z.x, z.y);
-      if (ANTI) of::heston_euler_step(b, c, -z.x, -z.y);
+      z = of::polar_from_u32(r.z, r.w, c.bm_k2);
+      of::heston_euler_step(a, c, z.q, z.c, z.s);
+      if (ANTI) of::heston_euler_step(b, c, z.q, -z.c, -z.s);
     }
   } else {
     float u = of::uniform_from_u32(r.x), zx = of::normal_from_u32(r.y);
@@ -382,7 +437,7 @@ __global__ void __launch_bounds__(256, 5) strip_kernel_ws(const __grid_constant_
   }
   __syncthreads();
   float K[KPL];
-  of::Kahan32 s1[KPL], s2[KPL];
+  of::KahanSq32 acc[KPL];
 #pragma unroll
   for (int q = 0; q < KPL; ++q) {
     const int k = lane + 32 * q;
@@ -450,8 +505,7 @@ __global__ void __launch_bounds__(256, 5) strip_kernel_ws(const __grid_constant_
       for (int q = 0; q < KPL; ++q) {
         float x = fmaxf(call ? st - K[q] : K[q] - st, 0.0f);
         if (ANTI) x = 0.5f * (x + fmaxf(call ? sta - K[q] : K[q] - sta, 0.0f));
-        s1[q].add(x);
-        s2[q].add(x * x);
+        acc[q].add(x);
       }
     }
   }
@@ -461,8 +515,8 @@ __global__ void __launch_bounds__(256, 5) strip_kernel_ws(const __grid_constant_
   for (int q = 0; q < KPL; ++q) {
     const int k = lane + 32 * q;
     if (k < n) {
-      sh_strip[(warp * n + k) * 2] = s1[q].value();
-      sh_strip[(warp * n + k) * 2 + 1] = s2[q].value();
+      sh_strip[(warp * n + k) * 2] = acc[q].value();
+      sh_strip[(warp * n + k) * 2 + 1] = acc[q].square();
     }
   }
   __syncthreads();
@@ -497,8 +551,8 @@ StripKernelFn pick_strip_ilp(int kpl, int ilp, int model, bool anti);
 
 // The kernel, its dynamic shared memory and the samples one block covers per
 // round, for a strip tile shape: tile 1 or 2 = strip_kernel with that many
-// samples in flight per thread (0 = 1), tile 3 = the warp-specialised
-// strip_kernel_ws.
+// samples in flight per thread (0: strip_default_tile), tile 3 = the
+// warp-specialised strip_kernel_ws.
 struct StripShape {
   StripKernelFn fn;
   size_t smem;
@@ -506,25 +560,46 @@ struct StripShape {
   bool ws;
 };
 
-StripShape strip_shape(int tile, int64_t n_strikes, int model, bool anti, int block) {
-  const int kpl = (int)((n_strikes + 31) / 32);
+// tile 0: two samples per thread where the samples fill the resident threads
+// (four blocks per SM) twice over, one below that, where more warps matter,
+// and for QE, whose two samples run one after the other.  2^20 samples of 256
+// steps, one / two: Heston 529 / 475 us, GBM 234 / 217, QE 1160 / 1202; 2^19
+// antithetic pairs: Heston 329 / 311, GBM 133 / 125.
+int strip_default_tile(int64_t samples, int model, int sms) {
+  return model != OF_MODEL_HESTON_QE && samples >= (int64_t)sms * 4 * kStripThreads * 2 ? 2 : 1;
+}
+
+StripShape strip_shape(int tile, int64_t samples, int64_t n_strikes, int model, bool anti, int sms) {
+  constexpr int block = kStripThreads;
+  const int kpl = n_strikes == 1 ? 0 : (int)((n_strikes + 31) / 32);
   const size_t sums = (size_t)(block / 32) * (size_t)n_strikes * 2 * sizeof(double);
   if (tile == 3) {
     const StripKernelFn fn = kpl <= 1 ? pick_strip_ws_kpl<1>(model, anti)
                              : kpl <= 2 ? pick_strip_ws_kpl<2>(model, anti) : pick_strip_ws_kpl<4>(model, anti);
     return {fn, kWsRingBytes + sums, (int64_t)kWsPairs * 32, true};
   }
-  const int ilp = tile == 2 ? 2 : 1;
+  const int ilp = tile ? tile : strip_default_tile(samples, model, sms);
   return {pick_strip_ilp(kpl, ilp, model, anti), sums, (int64_t)block * ilp, false};
+}
+
+// Blocks: enough for the samples, at most the resident ones; few samples are
+// spread over all SMs, some warps of each block idle.
+int strip_grid(const StripShape& sh, int64_t samples, int sms, int per_sm) {
+  const int64_t want = (samples + sh.samples_per_block - 1) / sh.samples_per_block;
+  const int64_t rounds = (samples + 31) / 32;
+  const int64_t spread = sh.ws ? want : std::max(want, std::min<int64_t>(sms, rounds));
+  return (int)std::max<int64_t>(1, std::min(spread, (int64_t)sms * per_sm));
 }
 
 // Kernel for KPL strikes per lane and ILP samples in flight per thread.
 StripKernelFn pick_strip_ilp(int kpl, int ilp, int model, bool anti) {
   if (ilp == 2) {
+    if (kpl == 0) return pick_strip<0, 2>(model, anti);
     if (kpl <= 1) return pick_strip<1, 2>(model, anti);
     if (kpl <= 2) return pick_strip<2, 2>(model, anti);
     return pick_strip<4, 2>(model, anti);
   }
+  if (kpl == 0) return pick_strip<0>(model, anti);
   if (kpl <= 1) return pick_strip<1>(model, anti);
   if (kpl <= 2) return pick_strip<2>(model, anti);
   return pick_strip<4>(model, anti);
@@ -551,7 +626,6 @@ struct of_strip_plan {
   bool ws = false;  // warp-specialised kernel: clears and reads back the status word after the sums
   double discount = 1.0;
   int64_t samples = 0;
-  float* d_strikes = nullptr;
   double* d_partials = nullptr;
   double* d_sums = nullptr;
   double* h_sums = nullptr;
@@ -559,14 +633,16 @@ struct of_strip_plan {
   cudaGraphExec_t exec = nullptr;
 };
 
-// d_sums holds the 2n sums and one more double whose first word is the
-// status of the warp-specialised kernel.
+// The sums go to h_sums (pinned), from the kernel's last block or from the
+// reduction launch; behind the 2n sums follows one more double whose first
+// word is the status of the warp-specialised kernel (from d_sums).
 static of_status strip_enqueue(of_strip_plan* pl, cudaStream_t s) {
   const int64_t cols = 2 * (int64_t)pl->n_strikes;
   if (pl->ws) cudaMemsetAsync(pl->d_sums + cols, 0, sizeof(double), s);
   pl->fn<<<pl->grid, pl->block, pl->smem, s>>>(pl->P, pl->d_partials);
-  of_launch_reduce_rows(pl->d_partials, pl->grid, cols, pl->d_sums, s);
-  cudaMemcpyAsync(pl->h_sums, pl->d_sums, (cols + (pl->ws ? 1 : 0)) * sizeof(double), cudaMemcpyDeviceToHost, s);
+  if (!pl->P.ticket) of_launch_reduce_rows(pl->d_partials, pl->grid, cols, pl->h_sums, s);
+  if (pl->ws)
+    cudaMemcpyAsync(pl->h_sums + cols, pl->d_sums + cols, sizeof(double), cudaMemcpyDeviceToHost, s);
   return OF_OK;
 }
 
@@ -582,7 +658,6 @@ extern "C" void of_strip_plan_destroy(of_strip_plan* pl) {
   if (pl->ctx) cudaStreamSynchronize(pl->ctx->stream);
   if (pl->exec) cudaGraphExecDestroy(pl->exec);
   if (pl->graph) cudaGraphDestroy(pl->graph);
-  cudaFree(pl->d_strikes);
   cudaFree(pl->d_partials);
   cudaFree(pl->d_sums);
   if (pl->h_sums) cudaFreeHost(pl->h_sums);
@@ -637,14 +712,13 @@ static of_status strip_setup(of_ctx* ctx, const of_model* m, int32_t option_type
   P.antithetic = cfg->antithetic ? 1 : 0;
   P.s0 = (float)m->s0;
   P.keys = of::philox_keys(cfg->seed);
-  const StripShape sh = strip_shape(cfg->tile_ilp, n_strikes, m->kind, P.antithetic, pl->block);
+  for (int64_t k = 0; k < n_strikes; ++k) P.strikes[k] = (float)strikes[k];
+  const StripShape sh = strip_shape(cfg->tile_ilp, pl->samples, n_strikes, m->kind, P.antithetic, ctx->sm_count);
   pl->fn = sh.fn;
   pl->smem = sh.smem;
   pl->ws = sh.ws;
   const int per_sm = of_blocks_per_sm((const void*)pl->fn, pl->block, pl->smem);
-  const int64_t want = (pl->samples + sh.samples_per_block - 1) / sh.samples_per_block;
-  const int64_t cap = (int64_t)ctx->sm_count * per_sm;
-  pl->grid = (int)std::max<int64_t>(1, std::min(want, cap));
+  pl->grid = strip_grid(sh, pl->samples, ctx->sm_count, per_sm);
   return OF_OK;
 }
 
@@ -664,17 +738,16 @@ extern "C" of_status of_strip_plan_create(of_ctx* ctx, const of_model* m, int32_
     of_strip_plan_destroy(pl);
     return st;
   };
-  std::vector<float> ks((size_t)n_strikes);
-  for (int64_t k = 0; k < n_strikes; ++k) ks[(size_t)k] = (float)strikes[k];
-  if (cudaMalloc(&pl->d_strikes, ks.size() * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&pl->d_partials, (size_t)pl->grid * 2 * n_strikes * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&pl->d_sums, (2 * n_strikes + 1) * sizeof(double)) != cudaSuccess ||
+  if (cudaMalloc(&pl->d_partials, (size_t)pl->grid * 2 * n_strikes * sizeof(double)) != cudaSuccess ||
+      cudaMalloc(&pl->d_sums, (2 * n_strikes + 2) * sizeof(double)) != cudaSuccess ||
+      cudaMemset(pl->d_sums, 0, (2 * n_strikes + 2) * sizeof(double)) != cudaSuccess ||
       cudaMallocHost(&pl->h_sums, (2 * n_strikes + 1) * sizeof(double)) != cudaSuccess)
     return fail(of_fail(ctx, OF_ERR_ALLOC, "strip plan allocation failed"));
-  if (cudaMemcpy(pl->d_strikes, ks.data(), ks.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
-    return fail(of_fail(ctx, OF_ERR_CUDA, "strike upload failed"));
-  pl->P.strikes = pl->d_strikes;
   pl->P.status = (uint32_t*)(pl->d_sums + 2 * n_strikes);
+  if (!pl->ws && strip_fused(pl->grid, 2 * (int)n_strikes)) {
+    pl->P.ticket = (unsigned*)(pl->d_sums + 2 * n_strikes + 1);
+    pl->P.out = pl->h_sums;
+  }
   // Capture kernel + reduction + readback once; launches replay the graph.
   cudaStream_t cap_stream = nullptr;
   if (cudaStreamCreateWithFlags(&cap_stream, cudaStreamNonBlocking) != cudaSuccess)
@@ -718,19 +791,18 @@ extern "C" of_status of_mc_strip(of_ctx* ctx, const of_model* m, int32_t option_
   of_strip_plan pl;  // setup only; buffers come from the context
   OF_TRY(strip_setup(ctx, m, option_type, strikes, n_strikes, cfg, &pl));
   const int64_t cols = 2 * n_strikes;
-  void *d_k = nullptr, *d_part = nullptr, *d_sums = nullptr, *h = nullptr;
-  OF_TRY(of_scratch(ctx, SLOT_STRIKES, (size_t)n_strikes * sizeof(float), &d_k));
+  void *d_part = nullptr, *d_sums = nullptr, *h = nullptr;
   OF_TRY(of_scratch(ctx, SLOT_PARTIALS, (size_t)pl.grid * cols * sizeof(double), &d_part));
   OF_TRY(of_scratch(ctx, SLOT_SUMS, (size_t)(cols + 1) * sizeof(double), &d_sums));
-  OF_TRY(of_pinned(ctx, (size_t)(cols + 1) * sizeof(double) + (size_t)n_strikes * sizeof(float), &h));
-  float* hk = (float*)((double*)h + cols + 1);
-  for (int64_t k = 0; k < n_strikes; ++k) hk[k] = (float)strikes[k];
-  OF_CUDA_TRY(ctx, cudaMemcpyAsync(d_k, hk, (size_t)n_strikes * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
-  pl.P.strikes = (const float*)d_k;
+  OF_TRY(of_pinned(ctx, (size_t)(cols + 1) * sizeof(double), &h));
   pl.P.status = (uint32_t*)((double*)d_sums + cols);
   pl.d_partials = (double*)d_part;
   pl.d_sums = (double*)d_sums;
   pl.h_sums = (double*)h;
+  if (!pl.ws && strip_fused(pl.grid, (int)cols)) {
+    OF_TRY(of_ticket(ctx, &pl.P.ticket));
+    pl.P.out = pl.h_sums;
+  }
   OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
   strip_enqueue(&pl, ctx->stream);
   OF_CUDA_TRY(ctx, cudaGetLastError());
@@ -897,13 +969,15 @@ __device__ __forceinline__ void book_sample(const BookOpt& o, uint64_t i, const 
   for (int32_t j = 0; j < o.steps; j += SPC) {
     const uint4 r = of::philox4x32_10(make_uint4((uint32_t)(j / SPC), lo, hi, o.stream), K);
     const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
-    // Box-Muller normals of the two draw pairs (GBM and Heston Euler)
+    // Box-Muller normals of the two draw pairs (GBM), their polar form (Heston Euler)
     float2 p01 = make_float2(0.0f, 0.0f), p23 = make_float2(0.0f, 0.0f);
-    if (MODEL != OF_MODEL_HESTON_QE) {
-      // Heston Euler takes its normals scaled by sqrt(dt) (heston_euler_step)
-      const float k2 = MODEL == OF_MODEL_HESTON_EULER ? c.bm_k2 : of::kBoxMullerK2;
-      p01 = of::normal_pair_scaled_from_u32(r.x, r.y, k2);
-      p23 = of::normal_pair_scaled_from_u32(r.z, r.w, k2);
+    of::Polar h01{}, h23{};
+    if (MODEL == OF_MODEL_GBM) {
+      p01 = of::normal_pair_from_u32(r.x, r.y);
+      p23 = of::normal_pair_from_u32(r.z, r.w);
+    } else if (MODEL == OF_MODEL_HESTON_EULER) {
+      h01 = of::polar_from_u32(r.x, r.y, c.bm_k2);
+      h23 = of::polar_from_u32(r.z, r.w, c.bm_k2);
     }
 #pragma unroll
     for (int q = 0; q < SPC; ++q) {
@@ -918,10 +992,9 @@ __device__ __forceinline__ void book_sample(const BookOpt& o, uint64_t i, const 
           if (anti) b.y = book_dividend(d, b.y);
         }
       } else if (MODEL == OF_MODEL_HESTON_EULER) {
-        const float2 z = q == 0 ? p01 : p23;
-        const float z1 = z.x, z2 = z.y;
-        of::heston_euler_step(a, c, z1, z2);
-        if (anti) of::heston_euler_step(b, c, -z1, -z2);
+        const of::Polar z = q == 0 ? h01 : h23;
+        of::heston_euler_step(a, c, z.q, z.c, z.s);
+        if (anti) of::heston_euler_step(b, c, z.q, -z.c, -z.s);
       } else {
         const float u = of::uniform_from_u32(rr[2 * q]), zx = of::normal_from_u32(rr[2 * q + 1]);
         of::heston_qe_step(a, c, u, 1.0f, zx, rr[2 * q]);
@@ -2038,7 +2111,7 @@ of_status of_mc_run_fp32(of_ctx* ctx, const of_model* m, const of_payoff* p, con
 // For callers that cannot allocate device memory when they price: every
 // byte of scratch the strip kernel needs lives in the static array below,
 // which each GPU that loads this library holds until the process exits.
-// Layout: [strikes: MAX_STRIKES floats][sums: 2*MAX_STRIKES doubles]
+// Layout: [MAX_STRIKES floats unused][sums: 2*MAX_STRIKES doubles]
 //         [per-block partials: MAX_BLOCKS * 2*MAX_STRIKES doubles].
 // In host code `g_strip_noalloc_scratch` names a host-side stand-in, not the
 // device array: its device address is looked up with cudaGetSymbolAddress
@@ -2145,9 +2218,6 @@ extern "C" of_status of_mc_strip_noalloc(void* cuda_stream, const of_model* m, i
                 OF_STRIP_NOALLOC_MAX_STRIKES, (long long)n_strikes);
     return OF_ERR_INVALID_INPUT;
   }
-  float hk[OF_STRIP_NOALLOC_MAX_STRIKES];
-  for (int64_t k = 0; k < n_strikes; ++k) hk[k] = (float)strikes[k];
-
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) {
@@ -2170,7 +2240,6 @@ extern "C" of_status of_mc_strip_noalloc(void* cuda_stream, const of_model* m, i
     noalloc_msg(err, err_len, "device address of the static scratch: %s", cudaGetErrorString(e));
     return OF_ERR_CUDA;
   }
-  float* d_strikes = (float*)base;
   double* d_sums = (double*)((char*)base + OF_STRIP_NOALLOC_MAX_STRIKES * 4);
   double* d_status = d_sums + OF_STRIP_NOALLOC_MAX_STRIKES * 2;  // the warp-specialised kernel's status word
   double* d_partials = d_status + 1;
@@ -2184,31 +2253,31 @@ extern "C" of_status of_mc_strip_noalloc(void* cuda_stream, const of_model* m, i
   P.antithetic = cfg->antithetic ? 1 : 0;
   P.s0 = (float)m->s0;
   P.keys = of::philox_keys(cfg->seed);
-  P.strikes = d_strikes;
+  for (int64_t k = 0; k < n_strikes; ++k) P.strikes[k] = (float)strikes[k];
   P.status = (uint32_t*)d_status;
   // the kernel of_mc_strip picks for the same request (strikes per lane, tile shape)
-  const int block = 256;
-  const StripShape sh = strip_shape(cfg->tile_ilp, n_strikes, m->kind, P.antithetic, block);
-  const StripKernelFn fn = sh.fn;
-  const size_t smem = sh.smem;
+  const int block = kStripThreads;
   int sms = 0, per_sm = 0;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, block, smem)) != cudaSuccess) {
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) {
     noalloc_msg(err, err_len, "device query failed: %s", cudaGetErrorString(e));
     return OF_ERR_CUDA;
   }
-  const int64_t want = (P.samples + sh.samples_per_block - 1) / sh.samples_per_block;
-  int64_t grid = std::min<int64_t>(want, (int64_t)sms * std::max(per_sm, 1));
-  grid = std::max<int64_t>(1, std::min<int64_t>(grid, OF_STRIP_NOALLOC_MAX_BLOCKS));
+  const StripShape sh = strip_shape(cfg->tile_ilp, P.samples, n_strikes, m->kind, P.antithetic, sms);
+  const StripKernelFn fn = sh.fn;
+  const size_t smem = sh.smem;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, block, smem)) != cudaSuccess) {
+    noalloc_msg(err, err_len, "device query failed: %s", cudaGetErrorString(e));
+    return OF_ERR_CUDA;
+  }
+  const int64_t grid =
+      std::min<int64_t>(strip_grid(sh, P.samples, sms, std::max(per_sm, 1)), OF_STRIP_NOALLOC_MAX_BLOCKS);
 
   cudaStream_t s = (cudaStream_t)cuda_stream;
   const int64_t cols = 2 * n_strikes;
   double hs[2 * OF_STRIP_NOALLOC_MAX_STRIKES];
   uint32_t h_status = 0;
-  if ((e = cudaMemcpyAsync(d_strikes, hk, (size_t)n_strikes * sizeof(float), cudaMemcpyHostToDevice, s)) !=
-          cudaSuccess ||
-      (sh.ws && (e = cudaMemsetAsync(d_status, 0, sizeof(double), s)) != cudaSuccess)) {
-    noalloc_msg(err, err_len, "strike upload failed: %s", cudaGetErrorString(e));
+  if (sh.ws && (e = cudaMemsetAsync(d_status, 0, sizeof(double), s)) != cudaSuccess) {
+    noalloc_msg(err, err_len, "status reset failed: %s", cudaGetErrorString(e));
     return OF_ERR_CUDA;
   }
   fn<<<(unsigned)grid, block, smem, s>>>(P, d_partials);

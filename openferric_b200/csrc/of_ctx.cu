@@ -1,6 +1,7 @@
 // of_ctx.cu - context lifecycle, scratch pool, errors and shared host helpers.
 #include <cmath>
 #include <cstring>
+#include <mutex>
 
 #include "of_device.cuh"
 #include "of_internal.h"
@@ -81,8 +82,26 @@ of_status of_ticket(of_ctx* ctx, unsigned** out) {
 }
 
 int of_blocks_per_sm(const void* kernel, int block, size_t smem) {
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, smem) != cudaSuccess || n < 1) n = 1;
+  // The occupancy of a launch shape never changes: asked of the runtime once
+  // per device (about 2 us a call).
+  struct Known {
+    const void* kernel;
+    int device, block, n;
+    size_t smem;
+  };
+  static std::mutex mutex;
+  static std::vector<Known> known;
+  constexpr size_t kMost = 1024;  // dynamic shared memory sizes vary with the request
+  int device = 0, n = 0;
+  cudaGetDevice(&device);
+  {
+    std::lock_guard<std::mutex> guard(mutex);
+    for (const Known& k : known)
+      if (k.kernel == kernel && k.device == device && k.block == block && k.smem == smem) return k.n;
+  }
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, smem) != cudaSuccess || n < 1) return 1;
+  std::lock_guard<std::mutex> guard(mutex);
+  if (known.size() < kMost) known.push_back(Known{kernel, device, block, n, smem});
   return n;
 }
 

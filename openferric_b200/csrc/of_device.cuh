@@ -178,12 +178,79 @@ __device__ __forceinline__ uint4 philox4x32_10(uint4 c, const PhiloxKeys& K) {
   return c;
 }
 
+// Philox blocks {q, lo, hi, stream} of many samples that share hi, stream and
+// the sequence of q (every kernel's use): in the first three rounds all terms
+// but two depend on the sample alone or on q alone.
+//   round 1: c0, c1 of its output depend on (lo, hi), c2, c3 on q;
+//   round 2: M0 c0 on the sample, M1 c2 on q;
+//   round 3: M0 c0 on q (and hi), only M1 c2 on both.
+// philox_q makes the q terms (round keys folded in), once per q and block of
+// threads, into shared memory; philox_lane the sample's, once per sample; and
+// philox_block does what is left: 15 wide products and 17 XORs of 20 and 20.
+// A 32x32->64-bit product occupies its pipe for four cycles a warp (an FP32
+// FMA one, a XOR 1.4), so the 20 products, 80 cycles a call, bound the FP32
+// step loops: 150 cycles per pair of Heston samples and step, 100 per four GBM
+// steps.
+struct PhiloxLane {
+  uint32_t hi, lo;  // M0 x round 1's c0
+};
+
+__device__ __forceinline__ PhiloxLane philox_lane(uint32_t lo, uint32_t hi, const PhiloxKeys& K) {
+  const uint64_t p = (uint64_t)0xD2511F53u * (__umulhi(0xCD9E8D57u, hi) ^ lo ^ K.k0[0]);
+  return PhiloxLane{(uint32_t)(p >> 32), (uint32_t)p};
+}
+
+__device__ __forceinline__ uint4 philox_q(uint32_t q, uint32_t hi, uint32_t stream, const PhiloxKeys& K) {
+  const uint64_t u = (uint64_t)0xD2511F53u * q;
+  const uint64_t b = (uint64_t)0xCD9E8D57u * ((uint32_t)(u >> 32) ^ stream ^ K.k1[0]);
+  const uint64_t c = (uint64_t)0xD2511F53u * ((uint32_t)(b >> 32) ^ (0xCD9E8D57u * hi) ^ K.k0[1]);
+  return make_uint4((uint32_t)u ^ K.k1[1], (uint32_t)b ^ K.k0[2], (uint32_t)(c >> 32) ^ K.k1[2], (uint32_t)c);
+}
+
+__device__ __forceinline__ uint4 philox_block(const uint4 t, const PhiloxLane& s, const PhiloxKeys& K) {
+  const uint64_t p = (uint64_t)0xCD9E8D57u * (s.hi ^ t.x);
+  uint4 c = make_uint4((uint32_t)(p >> 32) ^ t.y, (uint32_t)p, s.lo ^ t.z, t.w);
+#pragma unroll
+  for (int r = 3; r < 10; ++r) {
+    const uint64_t p0 = (uint64_t)0xD2511F53u * c.x;
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * c.z;
+    c = make_uint4((uint32_t)(p1 >> 32) ^ c.y ^ K.k0[r], (uint32_t)p1, (uint32_t)(p0 >> 32) ^ c.w ^ K.k1[r],
+                   (uint32_t)p0);
+  }
+  return c;
+}
+
+// The q terms of one (hi, stream): a table of the first n in shared memory,
+// made by all threads of the block (philox_table_fill, then a barrier), and
+// past it computed in place.  A sample whose hi is not the table's takes n = 0.
+struct PhiloxTab {
+  const uint4* tab;
+  uint32_t n, hi, stream;
+};
+
+__device__ __forceinline__ void philox_table_fill(uint4* tab, uint32_t n, uint32_t hi, uint32_t stream,
+                                                  const PhiloxKeys& K) {
+  for (uint32_t q = threadIdx.x; q < n; q += blockDim.x) tab[q] = philox_q(q, hi, stream, K);
+}
+
+// FULL: q is known to be in the table.
+template <bool FULL = false>
+__device__ __forceinline__ uint4 philox_terms(const PhiloxTab& T, uint32_t q, const PhiloxKeys& K) {
+  return FULL || q < T.n ? T.tab[q] : philox_q(q, T.hi, T.stream, K);
+}
+
+// 1 + k 2^-23 with k the top 23 bits of r: 0x3F800000 | (r >> 9) as one funnel
+// shift (0x7F << 23 is 1.0's exponent field).
+__device__ __forceinline__ float unit_mantissa(uint32_t r) {
+  return __uint_as_float(__funnelshift_r(r, 0x7Fu, 9));
+}
+
 // u32 -> standard normal in FP32: u = (k + 0.5) 2^-23 with k the top 23 bits,
 // then Phi^-1(u) = x P(w), x = 2u-1, w = -log2((1+x)(1-x)) with the fitted
 // polynomials of invnorm_coeffs.h (one MUFU lg2 per draw; the tail branch,
 // w >= OF_INVN_W_SPLIT, is taken with probability 0.34 %).
 __device__ __forceinline__ float normal_from_u32(uint32_t r) {
-  const float f = __uint_as_float(0x3F800000u | (r >> 9));  // 1 + k 2^-23, exact
+  const float f = unit_mantissa(r);  // 1 + k 2^-23, exact
   const float x = fmaf(2.0f, f, -3.0f) + 1.1920928955078125e-7f;  // (2k + 1 - 2^23) 2^-23, exact
   const float t = fmaf(-x, x, 1.0f);  // 1 - x^2 = 4u(1-u), one rounding of the exact value
   const float w = -__log2f(t);
@@ -229,7 +296,7 @@ __device__ __forceinline__ float inv_normal_vq(float v, float q) {
 
 // u32 -> uniform in (0,1), the same grid as normal_from_u32: (k + 0.5) 2^-23.
 __device__ __forceinline__ float uniform_from_u32(uint32_t r) {
-  const float f = __uint_as_float(0x3F800000u | (r >> 9));
+  const float f = unit_mantissa(r);
   // f - (1 - 2^-24) = (2k + 1) 2^-24: one exact subtraction (Sterbenz), the
   // same value as (f - 1) + 2^-24
   return f - 0.999999940395355224609375f;
@@ -252,7 +319,7 @@ constexpr float kBoxMullerK2 = -1.3862943611198906f;  // -2 ln 2: unit scale
 __device__ __forceinline__ float2 normal_pair_scaled_from_u32(uint32_t a, uint32_t b, float k2) {
   const float u1 = uniform_from_u32(a);
   const float r = sqrtf(k2 * __log2f(u1));  // k2 log2(u1) = -2 s^2 ln(u1)
-  const float ang = fmaf(6.28318530717959f, __uint_as_float(0x3F800000u | (b >> 9)), -9.42477796076938f);
+  const float ang = fmaf(6.28318530717959f, unit_mantissa(b), -9.42477796076938f);
   float s, c;
   __sincosf(ang, &s, &c);
   return make_float2(r * c, r * s);
@@ -262,18 +329,51 @@ __device__ __forceinline__ float2 normal_pair_from_u32(uint32_t a, uint32_t b) {
   return normal_pair_scaled_from_u32(a, b, kBoxMullerK2);
 }
 
+// The pair before its square root: q = s^2 (-2 ln u1) and the angle's cosine
+// and sine, for steps that scale the normals by a square root of their own:
+// sqrt(v) s z = sqrt(v q) (cos, sin) takes one square root instead of two.
+struct Polar {
+  float q, c, s;
+};
+
+__device__ __forceinline__ Polar polar_from_u32(uint32_t a, uint32_t b, float k2) {
+  Polar p;
+  p.q = k2 * __log2f(uniform_from_u32(a));
+  __sincosf(fmaf(6.28318530717959f, unit_mantissa(b), -9.42477796076938f), &p.s, &p.c);
+  return p;
+}
+
+// polar_from_u32 of two samples' draw pairs (a0, b0) and (a1, b1) with the
+// FP32 arithmetic in packed pairs; each half is the scalar form bit for bit.
+struct Polar2 {
+  float2 q, c, s;
+};
+
+__device__ __forceinline__ Polar2 polars2_from_u32(uint32_t a0, uint32_t b0, uint32_t a1, uint32_t b1, float k2) {
+  Polar2 p;
+  const float2 u1 = sub2(make_float2(unit_mantissa(a0), unit_mantissa(a1)),
+                         splat2(0.999999940395355224609375f));
+  p.q = mul2(splat2(k2), make_float2(__log2f(u1.x), __log2f(u1.y)));
+  const float2 ang = fma2(splat2(6.28318530717959f),
+                          make_float2(unit_mantissa(b0), unit_mantissa(b1)),
+                          splat2(-9.42477796076938f));
+  __sincosf(ang.x, &p.s.x, &p.c.x);
+  __sincosf(ang.y, &p.s.y, &p.c.y);
+  return p;
+}
+
 // normal_pair_scaled_from_u32 of two samples' draw pairs (a0, b0) and (a1, b1)
 // with the FP32 arithmetic in packed pairs: w1 = (z1 of sample 0, z1 of
 // sample 1), w2 likewise for z2; each half is bit-identical to the scalar
 // transform (the same operations in the same order).
 __device__ __forceinline__ void normal_pairs_scaled2_from_u32(uint32_t a0, uint32_t b0, uint32_t a1, uint32_t b1,
                                                               float k2, float2& w1, float2& w2) {
-  const float2 u1 = sub2(make_float2(__uint_as_float(0x3F800000u | (a0 >> 9)), __uint_as_float(0x3F800000u | (a1 >> 9))),
+  const float2 u1 = sub2(make_float2(unit_mantissa(a0), unit_mantissa(a1)),
                          splat2(0.999999940395355224609375f));
   const float2 rr = mul2(splat2(k2), make_float2(__log2f(u1.x), __log2f(u1.y)));
   const float2 r = make_float2(sqrtf(rr.x), sqrtf(rr.y));
   const float2 ang = fma2(splat2(6.28318530717959f),
-                          make_float2(__uint_as_float(0x3F800000u | (b0 >> 9)), __uint_as_float(0x3F800000u | (b1 >> 9))),
+                          make_float2(unit_mantissa(b0), unit_mantissa(b1)),
                           splat2(-9.42477796076938f));
   float s0, c0, s1, c1;
   __sincosf(ang.x, &s0, &c0);
@@ -293,19 +393,19 @@ constexpr float kBoxMullerAngSum = -8.63937979737193f;
 __device__ __forceinline__ float normal_pair_sum_from_u32(uint32_t a, uint32_t b) {
   const float u1 = uniform_from_u32(a);
   const float r = sqrtf((2.0f * kBoxMullerK2) * __log2f(u1));
-  const float ang = fmaf(6.28318530717959f, __uint_as_float(0x3F800000u | (b >> 9)), kBoxMullerAngSum);
+  const float ang = fmaf(6.28318530717959f, unit_mantissa(b), kBoxMullerAngSum);
   return r * __sinf(ang);
 }
 
 // normal_pair_sum_from_u32 of two samples' draw pairs (a0, b0) and (a1, b1)
 // in packed pairs; each half is the scalar form bit for bit.
 __device__ __forceinline__ float2 normal_pair_sums2_from_u32(uint32_t a0, uint32_t b0, uint32_t a1, uint32_t b1) {
-  const float2 u1 = sub2(make_float2(__uint_as_float(0x3F800000u | (a0 >> 9)), __uint_as_float(0x3F800000u | (a1 >> 9))),
+  const float2 u1 = sub2(make_float2(unit_mantissa(a0), unit_mantissa(a1)),
                          splat2(0.999999940395355224609375f));
   const float2 rr = mul2(splat2(2.0f * kBoxMullerK2), make_float2(__log2f(u1.x), __log2f(u1.y)));
   const float2 r = make_float2(sqrtf(rr.x), sqrtf(rr.y));
   const float2 ang = fma2(splat2(6.28318530717959f),
-                          make_float2(__uint_as_float(0x3F800000u | (b0 >> 9)), __uint_as_float(0x3F800000u | (b1 >> 9))),
+                          make_float2(unit_mantissa(b0), unit_mantissa(b1)),
                           splat2(kBoxMullerAngSum));
   return mul2(r, make_float2(__sinf(ang.x), __sinf(ang.y)));
 }
@@ -340,6 +440,20 @@ __device__ __forceinline__ void block_sum(double (&v)[N], double* sh) {
     }
   }
 }
+
+// Compensated FP32 accumulators (Kahan) of a value and its square in one
+// packed pair; each half is Kahan32's arithmetic bit for bit.
+struct KahanSq32 {
+  float2 sum = make_float2(0.0f, 0.0f), comp = make_float2(0.0f, 0.0f);
+  __device__ __forceinline__ void add(float x) {
+    const float2 y = sub2(make_float2(x, x * x), comp);
+    const float2 t = add2(sum, y);
+    comp = sub2(sub2(t, sum), y);
+    sum = t;
+  }
+  __device__ __forceinline__ double value() const { return (double)sum.x - (double)comp.x; }
+  __device__ __forceinline__ double square() const { return (double)sum.y - (double)comp.y; }
+};
 
 // Compensated FP32 accumulator (Kahan); flushed to FP64 as sum - comp.
 struct Kahan32 {

@@ -17,8 +17,8 @@ struct StepConsts {
   // Heston Euler of the reference (src/models/stochastic.rs:56-71, with the
   // variance floored after every step as src/mc/simulation.rs:111-113 does):
   // y += mudt - half_dt v + sqrt(v) sqdt zs ; v = max(v + kdt_theta - kdt v + xi sqrt(v) sqdt z1, 0)
-  // The normals arrive as sqdt (z1, z2): bm_k2 = -2 ln(2) dt is the radius
-  // constant of normal_pair_scaled_from_u32.
+  // The normals arrive as a polar pair scaled by sqdt: bm_k2 = -2 ln(2) dt is
+  // the radius constant of polar_from_u32.
   float mudt, half_dt, sqdt, kdt, kdt_theta, xi, rho, rho_c, v0, y_floor, one_m_kdt, bm_k2;
   // Heston QE (Andersen 2008, gamma1 = gamma2 = 1/2, psi_c = 1.5)
   float qe_e, qe_c1, qe_c2, qe_theta, qe_k0, qe_k1, qe_k2, qe_k3, qe_k4;
@@ -29,13 +29,15 @@ struct LegState {
 };
 
 // Reference Heston Euler step in FP32 (variance kept >= 0 after each step).
-// w1, w2 = sqdt (z1, z2), the pair of normal_pair_scaled_from_u32(.., c.bm_k2).
-__device__ __forceinline__ void heston_euler_step(LegState& L, const StepConsts& c, float w1, float w2) {
-  const float sq = sqrtf(L.v);
-  const float ws = fmaf(c.rho, w1, c.rho_c * w2);  // sqdt zs
-  const float y = fmaf(sq, ws, fmaf(-c.half_dt, L.v, L.y + c.mudt));
+// sqdt (z1, z2) = sqrt(q) (cs, sn), the pair of polar_from_u32(.., c.bm_k2)
+// (negated cs and sn: the antithetic twin's).  Both normals enter scaled by
+// sqrt(v), so one square root, of v q, serves the pair.
+__device__ __forceinline__ void heston_euler_step(LegState& L, const StepConsts& c, float q, float cs, float sn) {
+  const float R = sqrtf(L.v * q);
+  const float ws = fmaf(c.rho, cs, c.rho_c * sn);
+  const float y = fmaf(R, ws, fmaf(-c.half_dt, L.v, L.y + c.mudt));
   // v + kappa (theta - v) dt = (1 - kappa dt) v + kappa theta dt
-  const float vn = fmaf(c.xi * sq, w1, fmaf(c.one_m_kdt, L.v, c.kdt_theta));
+  const float vn = fmaf(c.xi * R, cs, fmaf(c.one_m_kdt, L.v, c.kdt_theta));
   L.v = fmaxf(vn, 0.0f);
   L.y = fmaxf(y, c.y_floor);
 }
@@ -47,11 +49,12 @@ struct LegState2 {
   float2 y, v;
 };
 
-__device__ __forceinline__ void heston_euler_step2(LegState2& L, const StepConsts& c, float2 w1, float2 w2) {
-  const float2 sq = make_float2(sqrtf(L.v.x), sqrtf(L.v.y));
-  const float2 ws = fma2(splat2(c.rho), w1, mul2(splat2(c.rho_c), w2));
-  const float2 y = fma2(sq, ws, fma2(splat2(-c.half_dt), L.v, add2(L.y, splat2(c.mudt))));
-  const float2 vn = fma2(mul2(splat2(c.xi), sq), w1, fma2(splat2(c.one_m_kdt), L.v, splat2(c.kdt_theta)));
+__device__ __forceinline__ void heston_euler_step2(LegState2& L, const StepConsts& c, const Polar2& z) {
+  const float2 vq = mul2(L.v, z.q);
+  const float2 R = make_float2(sqrtf(vq.x), sqrtf(vq.y));
+  const float2 ws = fma2(splat2(c.rho), z.c, mul2(splat2(c.rho_c), z.s));
+  const float2 y = fma2(R, ws, fma2(splat2(-c.half_dt), L.v, add2(L.y, splat2(c.mudt))));
+  const float2 vn = fma2(mul2(splat2(c.xi), R), z.c, fma2(splat2(c.one_m_kdt), L.v, splat2(c.kdt_theta)));
   L.v = make_float2(fmaxf(vn.x, 0.0f), fmaxf(vn.y, 0.0f));
   L.y = make_float2(fmaxf(y.x, c.y_floor), fmaxf(y.y, c.y_floor));
 }
