@@ -139,18 +139,18 @@ struct GMath<double> {
 
 // The four draws of Philox block q of sample i: Box-Muller normals (the
 // book's draws for GBM steps) or uniforms (survival draws).
-template <typename R>
-__device__ __forceinline__ void gk_normals(const GreekConsts<R>& c, uint32_t q, uint32_t lo, uint32_t hi,
-                                           const PhiloxKeys& K, R (&z)[4]) {
-  const uint4 r = philox4x32_10(make_uint4(q, lo, hi, c.stream), K);
+template <typename R, typename GEN>
+__device__ __forceinline__ void gk_normals(const GreekConsts<R>& c, uint32_t q, const PhiloxLane& L,
+                                           const GEN& K, R (&z)[4]) {
+  const uint4 r = K.block(q, L);
   GMath<R>::pair(r.x, r.y, z[0], z[1]);
   GMath<R>::pair(r.z, r.w, z[2], z[3]);
 }
 
-template <typename R>
-__device__ __forceinline__ void gk_uniforms(const GreekConsts<R>& c, uint32_t q, uint32_t lo, uint32_t hi,
-                                            const PhiloxKeys& K, R (&u)[4]) {
-  const uint4 r = philox4x32_10(make_uint4(q, lo, hi, c.stream), K);
+template <typename R, typename GEN>
+__device__ __forceinline__ void gk_uniforms(const GreekConsts<R>& c, uint32_t q, const PhiloxLane& L,
+                                            const GEN& K, R (&u)[4]) {
+  const uint4 r = K.block(q, L);
   u[0] = GMath<R>::unif(r.x);
   u[1] = GMath<R>::unif(r.y);
   u[2] = GMath<R>::unif(r.z);
@@ -199,10 +199,10 @@ __device__ __forceinline__ void gk_discount(const GreekConsts<R>& c, R x, const 
 template <typename R, bool G, bool ANTI>
 __device__ __forceinline__ void gk_terminal_finish(const GreekConsts<R>& c, R w, GreekSample<R>& out);
 
-template <typename R, bool G, bool ANTI>
-__device__ __forceinline__ void gk_terminal(const GreekConsts<R>& c, uint64_t i, const PhiloxKeys& K,
+template <typename R, bool G, bool ANTI, typename GEN>
+__device__ __forceinline__ void gk_terminal(const GreekConsts<R>& c, uint64_t i, GEN K,
                                             GreekSample<R>& out) {
-  const uint32_t lo = (uint32_t)i, hi = (uint32_t)(i >> 32);
+  const PhiloxLane L = K.lane(i);
   R w = (R)0;  // sum of the path's normals
   const int32_t full = c.steps & ~3;
   if constexpr (std::is_same<R, float>::value) {
@@ -210,12 +210,12 @@ __device__ __forceinline__ void gk_terminal(const GreekConsts<R>& c, uint64_t i,
     // block of one or three steps adds its odd normal from the plain
     // transform.  The FP64 modes add the pair's two normals: the same draws.
     for (int32_t j = 0; j < full; j += 4) {
-      const uint4 r = philox4x32_10(make_uint4((uint32_t)(j >> 2), lo, hi, c.stream), K);
+      const uint4 r = K.block((uint32_t)(j >> 2), L);
       w += normal_pair_sum_from_u32(r.x, r.y) + normal_pair_sum_from_u32(r.z, r.w);
     }
     const int32_t rem = c.steps - full;
     if (rem > 0) {
-      const uint4 r = philox4x32_10(make_uint4((uint32_t)(full >> 2), lo, hi, c.stream), K);
+      const uint4 r = K.block((uint32_t)(full >> 2), L);
       if (rem == 1) {
         w += normal_pair_from_u32(r.x, r.y).x;
       } else {
@@ -226,12 +226,12 @@ __device__ __forceinline__ void gk_terminal(const GreekConsts<R>& c, uint64_t i,
   } else {
     for (int32_t j = 0; j < full; j += 4) {
       R z[4];
-      gk_normals(c, (uint32_t)(j >> 2), lo, hi, K, z);
+      gk_normals(c, (uint32_t)(j >> 2), L, K, z);
       w += (z[0] + z[1]) + (z[2] + z[3]);
     }
     if (full < c.steps) {
       R z[4];
-      gk_normals(c, (uint32_t)(full >> 2), lo, hi, K, z);
+      gk_normals(c, (uint32_t)(full >> 2), L, K, z);
       w += z[0];
       if (full + 1 < c.steps) w += z[1];
       if (full + 2 < c.steps) w += z[2];
@@ -363,10 +363,10 @@ __device__ __forceinline__ void gk_asian_finish(const GreekConsts<R>& c, const A
   for (int t = 0; t < 4; ++t) out.g[t] = h * gs[t];
 }
 
-template <typename R, bool G, bool ANTI, bool DAILY, bool NEED_ARITH, bool NEED_GEO>
-__device__ __forceinline__ void gk_asian(const GreekConsts<R>& c, uint64_t i, const PhiloxKeys& K,
+template <typename R, bool G, bool ANTI, bool DAILY, bool NEED_ARITH, bool NEED_GEO, typename GEN>
+__device__ __forceinline__ void gk_asian(const GreekConsts<R>& c, uint64_t i, GEN K,
                                          const float* __restrict__ obs_w, GreekSample<R>& out) {
-  const uint32_t lo = (uint32_t)i, hi = (uint32_t)(i >> 32);
+  const PhiloxLane L = K.lane(i);
   AsianLeg<R> A{}, B{};
   if (!DAILY) {  // an observation at t = 0: e^0 = 1, y = 0, i = 0
     const R w0 = (R)__ldg(obs_w + c.obs_offset);
@@ -386,7 +386,7 @@ __device__ __forceinline__ void gk_asian(const GreekConsts<R>& c, uint64_t i, co
   const int32_t full = c.steps & ~3;
   for (int32_t j = 0; j < full; j += 4) {
     R z[4];
-    gk_normals(c, (uint32_t)(j >> 2), lo, hi, K, z);
+    gk_normals(c, (uint32_t)(j >> 2), L, K, z);
     step(z[0], j);
     step(z[1], j + 1);
     step(z[2], j + 2);
@@ -394,7 +394,7 @@ __device__ __forceinline__ void gk_asian(const GreekConsts<R>& c, uint64_t i, co
   }
   if (full < c.steps) {
     R z[4];
-    gk_normals(c, (uint32_t)(full >> 2), lo, hi, K, z);
+    gk_normals(c, (uint32_t)(full >> 2), L, K, z);
     step(z[0], full);
     if (full + 1 < c.steps) step(z[1], full + 1);
     if (full + 2 < c.steps) step(z[2], full + 2);
@@ -405,22 +405,22 @@ __device__ __forceinline__ void gk_asian(const GreekConsts<R>& c, uint64_t i, co
 // gk_terminal<float, G, ANTI> of samples i0 and i1: the normals' sums in
 // packed pairs, in the scalar loop's order (each half bit for bit the scalar
 // sum).
-template <bool G, bool ANTI>
+template <bool G, bool ANTI, typename GEN>
 __device__ __forceinline__ void gk_terminal_pair(const GreekConsts<float>& c, uint64_t i0, uint64_t i1,
-                                                 const PhiloxKeys& K, GreekSample<float>& o0, GreekSample<float>& o1) {
-  const uint32_t lo0 = (uint32_t)i0, hi0 = (uint32_t)(i0 >> 32), lo1 = (uint32_t)i1, hi1 = (uint32_t)(i1 >> 32);
+                                                 GEN K, GreekSample<float>& o0, GreekSample<float>& o1) {
+  const PhiloxLane L0 = K.lane(i0), L1 = K.lane(i1);  // i0 and i1 share their high word
   float2 w = make_float2(0.0f, 0.0f);
   const int32_t full = c.steps & ~3;
   for (int32_t j = 0; j < full; j += 4) {
-    const uint4 r0 = philox4x32_10(make_uint4((uint32_t)(j >> 2), lo0, hi0, c.stream), K);
-    const uint4 r1 = philox4x32_10(make_uint4((uint32_t)(j >> 2), lo1, hi1, c.stream), K);
+    const uint4 qt = K.terms((uint32_t)(j >> 2));
+    const uint4 r0 = philox_block(qt, L0, *K.K), r1 = philox_block(qt, L1, *K.K);
     w = add2(w, add2(normal_pair_sums2_from_u32(r0.x, r0.y, r1.x, r1.y),
                      normal_pair_sums2_from_u32(r0.z, r0.w, r1.z, r1.w)));
   }
   const int32_t rem = c.steps - full;
   if (rem > 0) {
-    const uint4 r0 = philox4x32_10(make_uint4((uint32_t)(full >> 2), lo0, hi0, c.stream), K);
-    const uint4 r1 = philox4x32_10(make_uint4((uint32_t)(full >> 2), lo1, hi1, c.stream), K);
+    const uint4 qt = K.terms((uint32_t)(full >> 2));
+    const uint4 r0 = philox_block(qt, L0, *K.K), r1 = philox_block(qt, L1, *K.K);
     float2 a1, a2;
     if (rem == 1) {
       normal_pairs_scaled2_from_u32(r0.x, r0.y, r1.x, r1.y, kBoxMullerK2, a1, a2);
@@ -474,10 +474,10 @@ __device__ __forceinline__ AsianLeg<float> asian_half(const AsianLeg2& L, int e)
 // The step loop of gk_asian<float, G, ...> for two legs.  TWIN: sample i0 and
 // its antithetic twin (one stream, normals z and -z); otherwise samples i0
 // and i1.
-template <bool G, bool TWIN, bool DAILY, bool NEED_ARITH, bool NEED_GEO>
+template <bool G, bool TWIN, bool DAILY, bool NEED_ARITH, bool NEED_GEO, typename GEN>
 __device__ __forceinline__ void gk_asian_legs2(const GreekConsts<float>& c, uint64_t i0, uint64_t i1,
-                                               const PhiloxKeys& K, const float* __restrict__ obs_w, AsianLeg2& L) {
-  const uint32_t lo0 = (uint32_t)i0, hi0 = (uint32_t)(i0 >> 32), lo1 = (uint32_t)i1, hi1 = (uint32_t)(i1 >> 32);
+                                               GEN K, const float* __restrict__ obs_w, AsianLeg2& L) {
+  const PhiloxLane L0 = K.lane(i0), L1 = K.lane(i1);  // i0 and i1 share their high word
   L = AsianLeg2{};
   if (!DAILY) {
     const float w0 = __ldg(obs_w + c.obs_offset);
@@ -492,7 +492,8 @@ __device__ __forceinline__ void gk_asian_legs2(const GreekConsts<float>& c, uint
     if (DAILY || w != 0.0f) gk_observe2<G, NEED_ARITH, NEED_GEO>(L, w, idx);
   };
   for (int32_t j = 0; j < c.steps; j += 4) {
-    const uint4 r0 = philox4x32_10(make_uint4((uint32_t)(j >> 2), lo0, hi0, c.stream), K);
+    const uint4 qt = K.terms((uint32_t)(j >> 2));
+    const uint4 r0 = philox_block(qt, L0, *K.K);
     float2 w1, w2, w3, w4;
     if (TWIN) {  // w1 = (z_j, z_j+2), w2 = (z_j+1, z_j+3)
       normal_pairs_scaled2_from_u32(r0.x, r0.y, r0.z, r0.w, kBoxMullerK2, w1, w2);
@@ -501,7 +502,7 @@ __device__ __forceinline__ void gk_asian_legs2(const GreekConsts<float>& c, uint
       w1 = splat2(w1.x);
       w2 = splat2(w2.x);
     } else {
-      const uint4 r1 = philox4x32_10(make_uint4((uint32_t)(j >> 2), lo1, hi1, c.stream), K);
+      const uint4 r1 = philox_block(qt, L1, *K.K);
       normal_pairs_scaled2_from_u32(r0.x, r0.y, r1.x, r1.y, kBoxMullerK2, w1, w2);
       normal_pairs_scaled2_from_u32(r0.z, r0.w, r1.z, r1.w, kBoxMullerK2, w3, w4);
     }
@@ -512,17 +513,17 @@ __device__ __forceinline__ void gk_asian_legs2(const GreekConsts<float>& c, uint
   }
 }
 
-template <bool G, bool DAILY, bool NEED_ARITH, bool NEED_GEO>
-__device__ __forceinline__ void gk_asian_twin(const GreekConsts<float>& c, uint64_t i, const PhiloxKeys& K,
+template <bool G, bool DAILY, bool NEED_ARITH, bool NEED_GEO, typename GEN>
+__device__ __forceinline__ void gk_asian_twin(const GreekConsts<float>& c, uint64_t i, GEN K,
                                               const float* __restrict__ obs_w, GreekSample<float>& out) {
   AsianLeg2 L;
   gk_asian_legs2<G, true, DAILY, NEED_ARITH, NEED_GEO>(c, i, i, K, obs_w, L);
   gk_asian_finish<float, G, true, NEED_GEO>(c, asian_half(L, 0), asian_half(L, 1), out);
 }
 
-template <bool G, bool DAILY, bool NEED_ARITH, bool NEED_GEO>
+template <bool G, bool DAILY, bool NEED_ARITH, bool NEED_GEO, typename GEN>
 __device__ __forceinline__ void gk_asian_pair(const GreekConsts<float>& c, uint64_t i0, uint64_t i1,
-                                              const PhiloxKeys& K, const float* __restrict__ obs_w,
+                                              GEN K, const float* __restrict__ obs_w,
                                               GreekSample<float>& o0, GreekSample<float>& o1) {
   AsianLeg2 L;
   gk_asian_legs2<G, false, DAILY, NEED_ARITH, NEED_GEO>(c, i0, i1, K, obs_w, L);
@@ -656,16 +657,16 @@ __device__ __forceinline__ void surv_payoff(const SurvLeg<R, G>& s, const GreekC
   if (G) gk_discount(c, x, dx, g);
 }
 
-template <typename R, bool G, bool ANTI, bool IN>
-__device__ __forceinline__ void gk_barrier(const GreekConsts<R>& c, uint64_t i, const PhiloxKeys& K,
+template <typename R, bool G, bool ANTI, bool IN, typename GEN>
+__device__ __forceinline__ void gk_barrier(const GreekConsts<R>& c, uint64_t i, GEN K,
                                            GreekSample<R>& out) {
-  const uint32_t lo = (uint32_t)i, hi = (uint32_t)(i >> 32);
+  const PhiloxLane L = K.lane(i);
   SurvLeg<R, G> A, B;
   surv_init(A, c);
   if (ANTI) surv_init(B, c);
   for (int32_t j = 0; j < c.steps; j += 4) {
     R u[4];
-    gk_uniforms(c, (uint32_t)(j >> 2), lo, hi, K, u);
+    gk_uniforms(c, (uint32_t)(j >> 2), L, K, u);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (j + q >= c.steps) break;
@@ -702,9 +703,8 @@ __host__ __device__ __forceinline__ int gk_group(int kind) {
 // Two survival legs share each FP32 instruction (sm_100 f32x2): two
 // independent samples, or a sample and its antithetic twin (uniforms u and
 // 1 - u).  Every packed operation is the scalar step's operation in its order,
-// so each half is surv_step's arithmetic bit for bit; the table lookups of the
-// inverse normal (two fitted branches), the exponentials and the divisions
-// stay scalar per half.
+// so each half is surv_step's arithmetic bit for bit; the inverse normal's
+// tail branch, the exponentials and the divisions stay scalar per half.
 struct SurvLeg2 {
   float2 y, L, ypl;
   float2 e[3], le[3];
@@ -756,7 +756,7 @@ __device__ __forceinline__ void surv_step2(SurvLeg2& s, const GreekConsts<float>
   v.y = v.y > M::kTiny ? v.y : M::kTiny;
   q.x = q.x > M::kTiny ? q.x : M::kTiny;
   q.y = q.y > M::kTiny ? q.y : M::kTiny;
-  const float2 zeta = make_float2(M::icdf2(v.x, q.x), M::icdf2(v.y, q.y));
+  const float2 zeta = inv_normal_vq2(v, q);
   if (G) {
     const float2 zmh = sub2(zeta, h);
     const float2 d = mul2(mul2(splat2(0.5f), zmh), add2(zeta, h));
@@ -772,7 +772,7 @@ __device__ __forceinline__ void surv_step2(SurvLeg2& s, const GreekConsts<float>
   s.y = fma2(splat2(c.beta * c.sgn), zeta, add2(s.y, splat2(c.alpha)));
   s.L = mul2(s.L, p);
   if (IN) {
-    const float2 zp = make_float2(M::icdf2(u.x, 1.0f - u.x), M::icdf2(u.y, 1.0f - u.y));
+    const float2 zp = inv_normal_vq2(u, sub2(splat2(1.0f), u));
     s.ypl = fma2(splat2(c.beta), zp, add2(s.ypl, splat2(c.alpha)));
   }
 }
@@ -794,15 +794,15 @@ __device__ __forceinline__ SurvLeg<float, G> surv_half(const SurvLeg2& s, int e)
 
 // gk_barrier<float, G, true, IN>: the sample and its antithetic twin as the
 // two halves
-template <bool G, bool IN>
-__device__ __forceinline__ void gk_barrier_twin(const GreekConsts<float>& c, uint64_t i, const PhiloxKeys& K,
+template <bool G, bool IN, typename GEN>
+__device__ __forceinline__ void gk_barrier_twin(const GreekConsts<float>& c, uint64_t i, GEN K,
                                                 GreekSample<float>& out) {
-  const uint32_t lo = (uint32_t)i, hi = (uint32_t)(i >> 32);
+  const PhiloxLane L = K.lane(i);
   SurvLeg2 s;
   surv_init2(s, c);
   for (int32_t j = 0; j < c.steps; j += 4) {
     float u[4];
-    gk_uniforms(c, (uint32_t)(j >> 2), lo, hi, K, u);
+    gk_uniforms(c, (uint32_t)(j >> 2), L, K, u);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (j + q >= c.steps) break;
@@ -819,16 +819,16 @@ __device__ __forceinline__ void gk_barrier_twin(const GreekConsts<float>& c, uin
 }
 
 // gk_barrier<float, G, false, IN> of samples i0 and i1 in one packed loop
-template <bool G, bool IN>
+template <bool G, bool IN, typename GEN>
 __device__ __forceinline__ void gk_barrier_pair(const GreekConsts<float>& c, uint64_t i0, uint64_t i1,
-                                                const PhiloxKeys& K, GreekSample<float>& o0, GreekSample<float>& o1) {
-  const uint32_t lo0 = (uint32_t)i0, hi0 = (uint32_t)(i0 >> 32), lo1 = (uint32_t)i1, hi1 = (uint32_t)(i1 >> 32);
+                                                GEN K, GreekSample<float>& o0, GreekSample<float>& o1) {
+  const PhiloxLane L0 = K.lane(i0), L1 = K.lane(i1);  // i0 and i1 share their high word
   SurvLeg2 s;
   surv_init2(s, c);
   for (int32_t j = 0; j < c.steps; j += 4) {
     float u0[4], u1[4];
-    gk_uniforms(c, (uint32_t)(j >> 2), lo0, hi0, K, u0);
-    gk_uniforms(c, (uint32_t)(j >> 2), lo1, hi1, K, u1);
+    gk_uniforms(c, (uint32_t)(j >> 2), L0, K, u0);
+    gk_uniforms(c, (uint32_t)(j >> 2), L1, K, u1);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (j + q >= c.steps) break;
@@ -848,8 +848,8 @@ __device__ __forceinline__ void gk_barrier_pair(const GreekConsts<float>& c, uin
   for (int t = 0; t < 4; ++t) o1.g[t] = g[t];
 }
 
-template <typename R, bool G, int KG, bool ANTI>
-__device__ __forceinline__ void gk_sample_group_anti(const GreekConsts<R>& c, uint64_t i, const PhiloxKeys& K,
+template <typename R, bool G, int KG, bool ANTI, typename GEN>
+__device__ __forceinline__ void gk_sample_group_anti(const GreekConsts<R>& c, uint64_t i, GEN K,
                                                      const float* obs_w, GreekSample<R>& out) {
   if (KG == KG_TERMINAL) {
     gk_terminal<R, G, ANTI>(c, i, K, out);
@@ -888,18 +888,18 @@ __device__ __forceinline__ void gk_sample_group_anti(const GreekConsts<R>& c, ui
 
 // Two samples of a terminal-only option (FP32 modes; antithetic twins are
 // the negated sum of the same normals).
-template <bool G>
+template <bool G, typename GEN>
 __device__ __forceinline__ void gk_terminal_pair_group(const GreekConsts<float>& c, uint64_t i0, uint64_t i1,
-                                                       const PhiloxKeys& K, GreekSample<float>& o0,
+                                                       GEN K, GreekSample<float>& o0,
                                                        GreekSample<float>& o1) {
   if (c.flags & GF_ANTI) gk_terminal_pair<G, true>(c, i0, i1, K, o0, o1);
   else gk_terminal_pair<G, false>(c, i0, i1, K, o0, o1);
 }
 
 // Two samples of an Asian option without antithetic twins (FP32 modes).
-template <bool G>
+template <bool G, typename GEN>
 __device__ __forceinline__ void gk_asian_pair_group(const GreekConsts<float>& c, uint64_t i0, uint64_t i1,
-                                                    const PhiloxKeys& K, const float* __restrict__ obs_w,
+                                                    GEN K, const float* __restrict__ obs_w,
                                                     GreekSample<float>& o0, GreekSample<float>& o1) {
   if (c.kind == GK_ASIAN_DAILY) {
     if (c.flags & GF_GEOMETRIC) gk_asian_pair<G, true, false, true>(c, i0, i1, K, obs_w, o0, o1);
@@ -913,16 +913,16 @@ __device__ __forceinline__ void gk_asian_pair_group(const GreekConsts<float>& c,
 }
 
 // Two samples of a barrier option without antithetic twins (FP32 modes).
-template <bool G>
+template <bool G, typename GEN>
 __device__ __forceinline__ void gk_barrier_pair_group(const GreekConsts<float>& c, uint64_t i0, uint64_t i1,
-                                                      const PhiloxKeys& K, GreekSample<float>& o0,
+                                                      GEN K, GreekSample<float>& o0,
                                                       GreekSample<float>& o1) {
   if (c.kind == GK_BARRIER_OUT) gk_barrier_pair<G, false>(c, i0, i1, K, o0, o1);
   else gk_barrier_pair<G, true>(c, i0, i1, K, o0, o1);
 }
 
-template <typename R, bool G, int KG>
-__device__ __forceinline__ void gk_sample_group(const GreekConsts<R>& c, uint64_t i, const PhiloxKeys& K,
+template <typename R, bool G, int KG, typename GEN>
+__device__ __forceinline__ void gk_sample_group(const GreekConsts<R>& c, uint64_t i, GEN K,
                                                 const float* obs_w, GreekSample<R>& out) {
   if (c.flags & GF_ANTI) gk_sample_group_anti<R, G, KG, true>(c, i, K, obs_w, out);
   else gk_sample_group_anti<R, G, KG, false>(c, i, K, obs_w, out);

@@ -45,7 +45,9 @@ StepConsts make_consts(const of_model* m) {
   c.kdt_theta = (float)(m->kappa * m->theta * dt);
   c.one_m_kdt = (float)(1.0 - m->kappa * dt);
   c.xi = (float)m->xi;
-  c.bm_k2 = (float)(-2.0 * 0.69314718055994531 * dt);
+  // the radius constant of polar_from_u32: Heston's normals come scaled by
+  // sqrt(dt), GBM's by sigma sqrt(dt)
+  c.bm_k2 = (float)(-2.0 * 0.69314718055994531 * (m->kind == OF_MODEL_GBM ? m->sigma * m->sigma * dt : dt));
   c.rho = (float)m->rho;
   c.rho_c = (float)std::sqrt(1.0 - m->rho * m->rho);
   c.v0 = (float)m->v0;
@@ -884,6 +886,7 @@ struct BookParams {
   const BookDiv* divs;
   int32_t n_tiles;
   int32_t ppt;  // samples per thread per tile (tile = block * ppt samples)
+  uint32_t tab;  // entries of the q table in dynamic shared memory
   of::PhiloxKeys keys;
   int* counter;
   double* partials;  // [slot][5]
@@ -953,8 +956,8 @@ __device__ __forceinline__ float book_dividend(const BookDiv& d, float y) {
 
 // DIVS: the option has discrete dividends (GBM only); without them the step
 // loop carries no trigger check.
-template <int MODEL, bool DIVS = false>
-__device__ __forceinline__ void book_sample(const BookOpt& o, uint64_t i, const of::PhiloxKeys& K, const float* obs_w,
+template <int MODEL, bool DIVS, typename GEN>
+__device__ __forceinline__ void book_sample(const BookOpt& o, uint64_t i, GEN G, const float* obs_w,
                                             const BookDiv* divs, float& x, float& cvy) {
   const bool anti = o.flags & BF_ANTI;
   const StepConsts& c = o.c;
@@ -962,30 +965,32 @@ __device__ __forceinline__ void book_sample(const BookOpt& o, uint64_t i, const 
   PathObs oa{0.0f, 0.0f, 0.0f, false}, obb{0.0f, 0.0f, 0.0f, false};
   book_observe(o, oa, 0.0f, 0, obs_w);
   if (anti) book_observe(o, obb, 0.0f, 0, obs_w);
-  const uint32_t lo = (uint32_t)i, hi = (uint32_t)(i >> 32);
+  const of::PhiloxLane L = G.lane(i);
   int32_t ev = 0;  // next dividend trigger (GBM)
   const bool observe_each = (o.payoff != OF_PAYOFF_VANILLA) || (o.flags & (BF_NEED_ARITH | BF_NEED_GEO));
   constexpr int SPC = MODEL == OF_MODEL_GBM ? 4 : 2;  // steps per Philox call
   for (int32_t j = 0; j < o.steps; j += SPC) {
-    const uint4 r = of::philox4x32_10(make_uint4((uint32_t)(j / SPC), lo, hi, o.stream), K);
+    const uint4 r = G.block((uint32_t)(j / SPC), L);
     const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
-    // Box-Muller normals of the two draw pairs (GBM), their polar form (Heston Euler)
-    float2 p01 = make_float2(0.0f, 0.0f), p23 = make_float2(0.0f, 0.0f);
+    // polar normals of the two draw pairs (GBM and Heston Euler); for GBM .q
+    // becomes the radius sigma sqrt(dt) r, so that a step is one add and one fma
     of::Polar h01{}, h23{};
-    if (MODEL == OF_MODEL_GBM) {
-      p01 = of::normal_pair_from_u32(r.x, r.y);
-      p23 = of::normal_pair_from_u32(r.z, r.w);
-    } else if (MODEL == OF_MODEL_HESTON_EULER) {
+    if (MODEL != OF_MODEL_HESTON_QE) {
       h01 = of::polar_from_u32(r.x, r.y, c.bm_k2);
       h23 = of::polar_from_u32(r.z, r.w, c.bm_k2);
+    }
+    if (MODEL == OF_MODEL_GBM) {
+      h01.q = sqrtf(h01.q);
+      h23.q = sqrtf(h23.q);
     }
 #pragma unroll
     for (int q = 0; q < SPC; ++q) {
       if (j + q >= o.steps) break;
       if (MODEL == OF_MODEL_GBM) {
-        const float z = q == 0 ? p01.x : q == 1 ? p01.y : q == 2 ? p23.x : p23.y;
-        a.y = fmaf(c.diff, z, a.y + c.drift);
-        if (anti) b.y = fmaf(-c.diff, z, b.y + c.drift);
+        const of::Polar& h = q < 2 ? h01 : h23;
+        const float z = (q & 1) ? h.s : h.c;
+        a.y = fmaf(h.q, z, a.y + c.drift);
+        if (anti) b.y = fmaf(-h.q, z, b.y + c.drift);
         for (; DIVS && ev < o.n_div && divs[o.div_offset + ev].step == j + q; ++ev) {  // mc_engine.rs:157-167
           const BookDiv d = divs[o.div_offset + ev];
           a.y = book_dividend(d, a.y);
@@ -1022,8 +1027,8 @@ __device__ __forceinline__ void book_sample(const BookOpt& o, uint64_t i, const 
 // tested every step.  Whole Philox counter blocks (four steps) run without a
 // bounds test; the last, partial block follows.  BK_TERMINAL options take the
 // sum of their normals instead (book_terminal_sum).
-template <int KIND, bool TWIN>
-__device__ __forceinline__ void book_gbm_legs2(const BookOpt& o, uint64_t i0, uint64_t i1, const of::PhiloxKeys& K,
+template <int KIND, bool TWIN, typename GEN>
+__device__ __forceinline__ void book_gbm_legs2(const BookOpt& o, uint64_t i0, uint64_t i1, GEN G,
                                                float2& y, PathObs& oa, PathObs& ob);
 
 // Terminal-only options (BK_TERMINAL) need y_T alone: y_T = steps drift +
@@ -1035,17 +1040,18 @@ __device__ __forceinline__ void book_gbm_legs2(const BookOpt& o, uint64_t i0, ui
 // from the stepwise sum of the general loop by FP32 rounding only.  The
 // packed-pair form below sums in the same order, so each of its halves is
 // this scalar sum bit for bit.
-__device__ __forceinline__ float book_terminal_sum(const BookOpt& o, uint64_t i, const of::PhiloxKeys& K) {
-  const uint32_t lo = (uint32_t)i, hi = (uint32_t)(i >> 32);
+template <typename GEN>
+__device__ __forceinline__ float book_terminal_sum(const BookOpt& o, uint64_t i, GEN G) {
+  const of::PhiloxLane L = G.lane(i);
   float w = 0.0f;
   const int32_t full = o.steps & ~3;
   for (int32_t j = 0; j < full; j += 4) {
-    const uint4 r = of::philox4x32_10(make_uint4((uint32_t)(j >> 2), lo, hi, o.stream), K);
+    const uint4 r = G.block((uint32_t)(j >> 2), L);
     w += of::normal_pair_sum_from_u32(r.x, r.y) + of::normal_pair_sum_from_u32(r.z, r.w);
   }
   const int32_t rem = o.steps - full;
   if (rem > 0) {
-    const uint4 r = of::philox4x32_10(make_uint4((uint32_t)(full >> 2), lo, hi, o.stream), K);
+    const uint4 r = G.block((uint32_t)(full >> 2), L);
     if (rem == 1) {
       w += of::normal_pair_from_u32(r.x, r.y).x;
     } else {
@@ -1057,22 +1063,23 @@ __device__ __forceinline__ float book_terminal_sum(const BookOpt& o, uint64_t i,
 }
 
 // book_terminal_sum of samples i0 and i1 in packed pairs
+template <typename GEN>
 __device__ __forceinline__ float2 book_terminal_sums2(const BookOpt& o, uint64_t i0, uint64_t i1,
-                                                      const of::PhiloxKeys& K) {
+                                                      GEN G) {
   using of::add2;
-  const uint32_t lo0 = (uint32_t)i0, hi0 = (uint32_t)(i0 >> 32), lo1 = (uint32_t)i1, hi1 = (uint32_t)(i1 >> 32);
+  const of::PhiloxLane L0 = G.lane(i0), L1 = G.lane(i1);  // i0 and i1 share their high word
   float2 w = make_float2(0.0f, 0.0f);
   const int32_t full = o.steps & ~3;
   for (int32_t j = 0; j < full; j += 4) {
-    const uint4 r0 = of::philox4x32_10(make_uint4((uint32_t)(j >> 2), lo0, hi0, o.stream), K);
-    const uint4 r1 = of::philox4x32_10(make_uint4((uint32_t)(j >> 2), lo1, hi1, o.stream), K);
+    const uint4 qt = G.terms((uint32_t)(j >> 2));
+    const uint4 r0 = of::philox_block(qt, L0, *G.K), r1 = of::philox_block(qt, L1, *G.K);
     w = add2(w, add2(of::normal_pair_sums2_from_u32(r0.x, r0.y, r1.x, r1.y),
                      of::normal_pair_sums2_from_u32(r0.z, r0.w, r1.z, r1.w)));
   }
   const int32_t rem = o.steps - full;
   if (rem > 0) {
-    const uint4 r0 = of::philox4x32_10(make_uint4((uint32_t)(full >> 2), lo0, hi0, o.stream), K);
-    const uint4 r1 = of::philox4x32_10(make_uint4((uint32_t)(full >> 2), lo1, hi1, o.stream), K);
+    const uint4 qt = G.terms((uint32_t)(full >> 2));
+    const uint4 r0 = of::philox_block(qt, L0, *G.K), r1 = of::philox_block(qt, L1, *G.K);
     float2 a1, a2;
     if (rem == 1) {
       of::normal_pairs_scaled2_from_u32(r0.x, r0.y, r1.x, r1.y, of::kBoxMullerK2, a1, a2);
@@ -1103,17 +1110,17 @@ __device__ __forceinline__ void book_terminal_payoff(const BookOpt& o, float w, 
   }
 }
 
-template <int KIND, bool ANTI>
-__device__ __forceinline__ void book_sample_gbm(const BookOpt& o, uint64_t i, const of::PhiloxKeys& K, float& x,
+template <int KIND, bool ANTI, typename GEN>
+__device__ __forceinline__ void book_sample_gbm(const BookOpt& o, uint64_t i, GEN G, float& x,
                                                 float& cvy) {
   if (KIND == BK_TERMINAL) {
-    book_terminal_payoff<ANTI>(o, book_terminal_sum(o, i, K), x, cvy);
+    book_terminal_payoff<ANTI>(o, book_terminal_sum(o, i, G), x, cvy);
     return;
   }
   if (ANTI) {  // the sample and its antithetic twin as the two halves of packed pairs
     float2 y;
     PathObs oa, ob;
-    book_gbm_legs2<KIND, true>(o, i, i, K, y, oa, ob);
+    book_gbm_legs2<KIND, true>(o, i, i, G, y, oa, ob);
     float xb, yb2;
     book_payoff(o, oa, y.x, x, cvy);
     book_payoff(o, ob, y.y, xb, yb2);
@@ -1121,57 +1128,37 @@ __device__ __forceinline__ void book_sample_gbm(const BookOpt& o, uint64_t i, co
     cvy = 0.5f * (cvy + yb2);
     return;
   }
-  const float drift = o.c.drift, diff = o.c.diff;
-  // barrier test as sg*y >= sg*b: sg = +1 for an up barrier, -1 for a down one
-  const float sg = (o.flags & BF_UP) ? 1.0f : -1.0f, sgb = sg * o.barrier_y;
-  float ya = 0.0f, yb = 0.0f;
-  PathObs oa{0.0f, 0.0f, 0.0f, false}, ob{0.0f, 0.0f, 0.0f, false};
-  if (KIND == BK_BARRIER) oa.hit = ob.hit = 0.0f >= sgb;  // the scan includes path[0]
-  auto add_fixing = [](PathObs& p, float y) {  // Kahan sum of the daily fixings S/S0
-    const float yk = __expf(y) - p.arith_comp;
-    const float t = p.arith_sum + yk;
-    p.arith_comp = (t - p.arith_sum) - yk;
-    p.arith_sum = t;
-  };
-  auto step = [&](float z) {
-    ya = fmaf(diff, z, ya + drift);
-    if (ANTI) yb = fmaf(-diff, z, yb + drift);
+  // a barrier path runs with the sign that makes its barrier an upper one:
+  // sg y, sg drift, sg diff and sg b (sg = +1 up, -1 down; exact), one
+  // comparison per step
+  const float sg = KIND == BK_BARRIER && !(o.flags & BF_UP) ? -1.0f : 1.0f;
+  const float drift = sg * o.c.drift, sgb = sg * o.barrier_y, k2 = o.c.bm_k2;
+  float ya = 0.0f;
+  PathObs oa{0.0f, 0.0f, 0.0f, false};
+  if (KIND == BK_BARRIER) oa.hit = 0.0f >= sgb;  // the scan includes path[0]
+  auto step = [&](float R, float z) {
+    ya = fmaf(R, z, ya + drift);
     if (KIND == BK_BARRIER) {
-      oa.hit |= sg * ya >= sgb;
-      if (ANTI) ob.hit |= sg * yb >= sgb;
-    } else if (KIND == BK_ASIAN_DAILY || KIND == BK_ASIAN_DAILY_GEO) {
-      add_fixing(oa, ya);
-      if (ANTI) add_fixing(ob, yb);
-      if (KIND == BK_ASIAN_DAILY_GEO) {  // the general loop's fmaf(1, y, sum): one rounding
-        oa.geo_sum += ya;
-        if (ANTI) ob.geo_sum += yb;
-      }
+      oa.hit |= ya >= sgb;
+    } else {  // Kahan sum of the daily fixings S/S0
+      const float yk = __expf(ya) - oa.arith_comp;
+      const float t = oa.arith_sum + yk;
+      oa.arith_comp = (t - oa.arith_sum) - yk;
+      oa.arith_sum = t;
+      if (KIND == BK_ASIAN_DAILY_GEO) oa.geo_sum += ya;  // the general loop's fmaf(1, y, sum): one rounding
     }
   };
-  const uint32_t lo = (uint32_t)i, hi = (uint32_t)(i >> 32);
-  const int32_t full = o.steps & ~3;
-  for (int32_t j = 0; j < full; j += 4) {
-    const uint4 r = of::philox4x32_10(make_uint4((uint32_t)(j >> 2), lo, hi, o.stream), K);
-    const float2 p01 = of::normal_pair_from_u32(r.x, r.y), p23 = of::normal_pair_from_u32(r.z, r.w);
-    step(p01.x);
-    step(p01.y);
-    step(p23.x);
-    step(p23.y);
+  const of::PhiloxLane L = G.lane(i);
+  for (int32_t j = 0; j < o.steps; j += 4) {
+    const uint4 r = G.block((uint32_t)(j >> 2), L);
+    const of::Polar p = of::polar_from_u32(r.x, r.y, k2), q = of::polar_from_u32(r.z, r.w, k2);
+    const float Rp = sg * sqrtf(p.q), Rq = sg * sqrtf(q.q);
+    step(Rp, p.c);
+    if (j + 1 < o.steps) step(Rp, p.s);
+    if (j + 2 < o.steps) step(Rq, q.c);
+    if (j + 3 < o.steps) step(Rq, q.s);
   }
-  if (full < o.steps) {
-    const uint4 r = of::philox4x32_10(make_uint4((uint32_t)(full >> 2), lo, hi, o.stream), K);
-    const float2 p01 = of::normal_pair_from_u32(r.x, r.y), p23 = of::normal_pair_from_u32(r.z, r.w);
-    step(p01.x);
-    if (full + 1 < o.steps) step(p01.y);
-    if (full + 2 < o.steps) step(p23.x);
-  }
-  book_payoff(o, oa, ya, x, cvy);
-  if (ANTI) {
-    float xb, yb2;
-    book_payoff(o, ob, yb, xb, yb2);
-    x = 0.5f * (x + xb);
-    cvy = 0.5f * (cvy + yb2);
-  }
+  book_payoff(o, oa, sg * ya, x, cvy);
 }
 
 // Two legs of the specialised GBM loop in packed pairs (.x and .y), each half
@@ -1179,28 +1166,27 @@ __device__ __forceinline__ void book_sample_gbm(const BookOpt& o, uint64_t i, co
 // i0 and its antithetic twin (one Philox stream, normals z and -z); otherwise
 // the independent samples i0 and i1 (two streams, Box-Muller of both in packed
 // pairs).
-template <int KIND, bool TWIN>
-__device__ __forceinline__ void book_gbm_legs2(const BookOpt& o, uint64_t i0, uint64_t i1, const of::PhiloxKeys& K,
+template <int KIND, bool TWIN, typename GEN>
+__device__ __forceinline__ void book_gbm_legs2(const BookOpt& o, uint64_t i0, uint64_t i1, GEN G,
                                                float2& y, PathObs& oa, PathObs& ob) {
   using of::add2;
   using of::fma2;
   using of::mul2;
   using of::splat2;
   using of::sub2;
-  const float2 drift = splat2(o.c.drift);
-  const float2 diff = TWIN ? make_float2(o.c.diff, -o.c.diff) : splat2(o.c.diff);
-  const float sg = (o.flags & BF_UP) ? 1.0f : -1.0f, sgb = sg * o.barrier_y;
+  const float sg = KIND == BK_BARRIER && !(o.flags & BF_UP) ? -1.0f : 1.0f;
+  const float2 drift = splat2(sg * o.c.drift);
+  const float sgb = sg * o.barrier_y, k2 = o.c.bm_k2;
   y = make_float2(0.0f, 0.0f);
   float2 as = make_float2(0.0f, 0.0f), ac = make_float2(0.0f, 0.0f);  // Kahan sums of the daily fixings
   float2 ag = make_float2(0.0f, 0.0f);                                 // geometric sums
   bool ha = false, hb = false;
   if (KIND == BK_BARRIER) ha = hb = 0.0f >= sgb;  // the scan includes path[0]
-  auto step = [&](float2 z) {
-    y = fma2(diff, z, add2(y, drift));
+  auto step = [&](float2 R, float2 z) {
+    y = fma2(R, z, add2(y, drift));
     if (KIND == BK_BARRIER) {
-      const float2 t = mul2(splat2(sg), y);
-      ha |= t.x >= sgb;
-      hb |= t.y >= sgb;
+      ha |= y.x >= sgb;
+      hb |= y.y >= sgb;
     } else if (KIND == BK_ASIAN_DAILY || KIND == BK_ASIAN_DAILY_GEO) {
       const float2 yk = sub2(make_float2(__expf(y.x), __expf(y.y)), ac);
       const float2 t = add2(as, yk);
@@ -1209,44 +1195,56 @@ __device__ __forceinline__ void book_gbm_legs2(const BookOpt& o, uint64_t i0, ui
       if (KIND == BK_ASIAN_DAILY_GEO) ag = add2(ag, y);
     }
   };
-  const uint32_t lo0 = (uint32_t)i0, hi0 = (uint32_t)(i0 >> 32), lo1 = (uint32_t)i1, hi1 = (uint32_t)(i1 >> 32);
+  const of::PhiloxLane L0 = G.lane(i0), L1 = G.lane(i1);  // i0 and i1 share their high word
   for (int32_t j = 0; j < o.steps; j += 4) {
-    const uint4 r0 = of::philox4x32_10(make_uint4((uint32_t)(j >> 2), lo0, hi0, o.stream), K);
-    float2 w1, w2, w3, w4;
-    if (TWIN) {  // w1 = (z_j, z_j+2), w2 = (z_j+1, z_j+3)
-      of::normal_pairs_scaled2_from_u32(r0.x, r0.y, r0.z, r0.w, of::kBoxMullerK2, w1, w2);
-      w3 = splat2(w1.y);
-      w4 = splat2(w2.y);
-      w1 = splat2(w1.x);
-      w2 = splat2(w2.x);
-    } else {  // wk = step j+k-1 of (i0, i1)
-      const uint4 r1 = of::philox4x32_10(make_uint4((uint32_t)(j >> 2), lo1, hi1, o.stream), K);
-      of::normal_pairs_scaled2_from_u32(r0.x, r0.y, r1.x, r1.y, of::kBoxMullerK2, w1, w2);
-      of::normal_pairs_scaled2_from_u32(r0.z, r0.w, r1.z, r1.w, of::kBoxMullerK2, w3, w4);
+    const uint4 qt = G.terms((uint32_t)(j >> 2));
+    const uint4 r0 = of::philox_block(qt, L0, *G.K);
+    // steps j, j+1 take the radius Ra, steps j+2, j+3 Rb
+    float2 Ra, Rb, z1, z2, z3, z4;
+    if (TWIN) {
+      const of::Polar2 p = of::polars2_from_u32(r0.x, r0.y, r0.z, r0.w, k2);
+      const float ra = sg * sqrtf(p.q.x), rb = sg * sqrtf(p.q.y);
+      Ra = make_float2(ra, -ra);
+      Rb = make_float2(rb, -rb);
+      z1 = splat2(p.c.x);
+      z2 = splat2(p.s.x);
+      z3 = splat2(p.c.y);
+      z4 = splat2(p.s.y);
+    } else {
+      const uint4 r1 = of::philox_block(qt, L1, *G.K);
+      const of::Polar2 p = of::polars2_from_u32(r0.x, r0.y, r1.x, r1.y, k2),
+                       q = of::polars2_from_u32(r0.z, r0.w, r1.z, r1.w, k2);
+      Ra = make_float2(sg * sqrtf(p.q.x), sg * sqrtf(p.q.y));
+      Rb = make_float2(sg * sqrtf(q.q.x), sg * sqrtf(q.q.y));
+      z1 = p.c;
+      z2 = p.s;
+      z3 = q.c;
+      z4 = q.s;
     }
     if (j + 4 <= o.steps) {
-      step(w1);
-      step(w2);
-      step(w3);
-      step(w4);
+      step(Ra, z1);
+      step(Ra, z2);
+      step(Rb, z3);
+      step(Rb, z4);
     } else {
-      step(w1);
-      if (j + 1 < o.steps) step(w2);
-      if (j + 2 < o.steps) step(w3);
+      step(Ra, z1);
+      if (j + 1 < o.steps) step(Ra, z2);
+      if (j + 2 < o.steps) step(Rb, z3);
     }
   }
+  if (KIND == BK_BARRIER) y = mul2(splat2(sg), y);
   oa = PathObs{as.x, ac.x, ag.x, ha};
   ob = PathObs{as.y, ac.y, ag.y, hb};
 }
 
 // book_sample_gbm<KIND, false> of two samples in one packed loop.
-template <int KIND>
+template <int KIND, typename GEN>
 __device__ __forceinline__ void book_sample_gbm_pair(const BookOpt& o, uint64_t i0, uint64_t i1,
-                                                     const of::PhiloxKeys& K, float& x0, float& cv0, float& x1,
+                                                     GEN G, float& x0, float& cv0, float& x1,
                                                      float& cv1) {
   float2 y;
   PathObs oa, ob;
-  book_gbm_legs2<KIND, false>(o, i0, i1, K, y, oa, ob);
+  book_gbm_legs2<KIND, false>(o, i0, i1, G, y, oa, ob);
   book_payoff(o, oa, y.x, x0, cv0);
   book_payoff(o, ob, y.y, x1, cv1);
 }
@@ -1254,53 +1252,78 @@ __device__ __forceinline__ void book_sample_gbm_pair(const BookOpt& o, uint64_t 
 // book_sample_gbm<BK_TERMINAL, ANTI> of samples i0 and i1: their sums of
 // normals in packed pairs (two Philox streams per thread), then each sample's
 // payoff (and its twin's) as the scalar form takes it.
-template <bool ANTI>
-__device__ __forceinline__ void book_terminal_pair(const BookOpt& o, uint64_t i0, uint64_t i1, const of::PhiloxKeys& K,
+template <bool ANTI, typename GEN>
+__device__ __forceinline__ void book_terminal_pair(const BookOpt& o, uint64_t i0, uint64_t i1, GEN G,
                                                    float& x0, float& cv0, float& x1, float& cv1) {
-  const float2 w = book_terminal_sums2(o, i0, i1, K);
+  const float2 w = book_terminal_sums2(o, i0, i1, G);
   book_terminal_payoff<ANTI>(o, w.x, x0, cv0);
   book_terminal_payoff<ANTI>(o, w.y, x1, cv1);
 }
 
 // One sample of option o: the specialised GBM loop when the option has one,
 // the general loop otherwise.
-__device__ __forceinline__ void book_dispatch(const BookOpt& o, uint64_t i, const BookParams& P, float& x, float& y) {
+template <typename GEN>
+__device__ __forceinline__ void book_dispatch(const BookOpt& o, uint64_t i, const BookParams& P, const GEN& G,
+                                              float& x, float& y) {
   const bool anti = o.flags & BF_ANTI;
   switch (o.kind) {
     case BK_TERMINAL:
-      if (anti) book_sample_gbm<BK_TERMINAL, true>(o, i, P.keys, x, y);
-      else book_sample_gbm<BK_TERMINAL, false>(o, i, P.keys, x, y);
+      if (anti) book_sample_gbm<BK_TERMINAL, true>(o, i, G, x, y);
+      else book_sample_gbm<BK_TERMINAL, false>(o, i, G, x, y);
       return;
     case BK_BARRIER:
-      if (anti) book_sample_gbm<BK_BARRIER, true>(o, i, P.keys, x, y);
-      else book_sample_gbm<BK_BARRIER, false>(o, i, P.keys, x, y);
+      if (anti) book_sample_gbm<BK_BARRIER, true>(o, i, G, x, y);
+      else book_sample_gbm<BK_BARRIER, false>(o, i, G, x, y);
       return;
     case BK_ASIAN_DAILY:
-      if (anti) book_sample_gbm<BK_ASIAN_DAILY, true>(o, i, P.keys, x, y);
-      else book_sample_gbm<BK_ASIAN_DAILY, false>(o, i, P.keys, x, y);
+      if (anti) book_sample_gbm<BK_ASIAN_DAILY, true>(o, i, G, x, y);
+      else book_sample_gbm<BK_ASIAN_DAILY, false>(o, i, G, x, y);
       return;
     case BK_ASIAN_DAILY_GEO:
-      if (anti) book_sample_gbm<BK_ASIAN_DAILY_GEO, true>(o, i, P.keys, x, y);
-      else book_sample_gbm<BK_ASIAN_DAILY_GEO, false>(o, i, P.keys, x, y);
+      if (anti) book_sample_gbm<BK_ASIAN_DAILY_GEO, true>(o, i, G, x, y);
+      else book_sample_gbm<BK_ASIAN_DAILY_GEO, false>(o, i, G, x, y);
       return;
     default:
       break;
   }
   if (o.model == OF_MODEL_GBM) {
-    if (o.n_div) book_sample<OF_MODEL_GBM, true>(o, i, P.keys, P.obs_w, P.divs, x, y);
-    else book_sample<OF_MODEL_GBM, false>(o, i, P.keys, P.obs_w, P.divs, x, y);
+    if (o.n_div) book_sample<OF_MODEL_GBM, true>(o, i, G, P.obs_w, P.divs, x, y);
+    else book_sample<OF_MODEL_GBM, false>(o, i, G, P.obs_w, P.divs, x, y);
   } else if (o.model == OF_MODEL_HESTON_EULER) {
-    book_sample<OF_MODEL_HESTON_EULER>(o, i, P.keys, P.obs_w, P.divs, x, y);
+    book_sample<OF_MODEL_HESTON_EULER, false>(o, i, G, P.obs_w, P.divs, x, y);
   } else {
-    book_sample<OF_MODEL_HESTON_QE>(o, i, P.keys, P.obs_w, P.divs, x, y);
+    book_sample<OF_MODEL_HESTON_QE, false>(o, i, G, P.obs_w, P.divs, x, y);
   }
+}
+
+// The generator of a tile's option, its table (`cap` entries) filled by the
+// block (called by all threads).  FULL launches have a table that covers every
+// option's counter blocks and samples below 2^32; the others compute the terms
+// past the table, or past the tile's first high word, in place.  The loops run
+// at the integer-multiply rate (a wide multiply takes four issue cycles a warp
+// on sm_100); the table saves five of a counter block's twenty.  With the
+// radius folded into the path's fma and the packed sums of squares, 384 options
+// of 2^14..2^17 paths by 25..1260 daily steps took 10.58 ms (antithetic 6.36)
+// against 11.58 (6.98); with the range test left in the loop, 11.2.
+constexpr uint32_t kBookTab = 2048;  // largest table (32 KB, three blocks an SM): 8,192 GBM steps
+
+template <bool FULL>
+__device__ __forceinline__ of::PhiloxGen<FULL> book_gen(uint4* qtab, uint32_t cap, int steps_per_block, int32_t steps,
+                                                        int64_t first, uint32_t stream, const of::PhiloxKeys& K) {
+  const uint32_t nq = ((uint32_t)steps + steps_per_block - 1) / steps_per_block;
+  const of::PhiloxTab T{qtab, nq < cap ? nq : cap, (uint32_t)((uint64_t)first >> 32), stream};
+  of::philox_table_fill(qtab, T.n, T.hi, T.stream, K);
+  __syncthreads();
+  return of::PhiloxGen<FULL>{&K, T};
 }
 
 // Three 256-thread blocks per SM: ptxas's own choice without the hint is 64
 // registers with spills in the step loop.
+template <bool FULL>
 __global__ void __launch_bounds__(256, 3) book_kernel(const __grid_constant__ BookParams P) {
   __shared__ int tile_sh;
   __shared__ double red_sh[5 * 8];
+  extern __shared__ uint4 qtab[];
   for (;;) {
     if (threadIdx.x == 0) tile_sh = atomicAdd(P.counter, 1);
     __syncthreads();
@@ -1308,13 +1331,14 @@ __global__ void __launch_bounds__(256, 3) book_kernel(const __grid_constant__ Bo
     if (t >= P.n_tiles) break;
     const BookTile tile = P.tiles[t];
     const BookOpt o = P.opts[tile.opt];
-    of::Kahan32 acc[5];
+    const of::PhiloxGen<FULL> G =
+        book_gen<FULL>(qtab, P.tab, o.model == OF_MODEL_GBM ? 4 : 2, o.steps, tile.first, o.stream, P.keys);
+    of::KahanSq32 ax, ay;
+    of::Kahan32 axy;
     auto add = [&](float x, float y) {
-      acc[0].add(x);
-      acc[1].add(x * x);
-      acc[2].add(y);
-      acc[3].add(x * y);
-      acc[4].add(y * y);
+      ax.add(x);
+      ay.add(y);
+      axy.add(x * y);
     };
     // specialised GBM kinds without antithetic twins, and terminal-only
     // options with them, run two samples at a time in packed pairs; the sums
@@ -1325,27 +1349,25 @@ __global__ void __launch_bounds__(256, 3) book_kernel(const __grid_constant__ Bo
       if (local >= tile.count) break;
       const uint64_t i = (uint64_t)(tile.first + local);
       float x, y;
-      if (pairs && k + 1 < P.ppt && local + (int)blockDim.x < tile.count) {
-        const uint64_t i1 = i + blockDim.x;
+      if (const uint64_t i1 = i + blockDim.x;
+          pairs && k + 1 < P.ppt && local + (int)blockDim.x < tile.count && (FULL || (i >> 32) == (i1 >> 32))) {
         float x1, y1;
         if (o.kind == BK_TERMINAL) {
-          if (o.flags & BF_ANTI) book_terminal_pair<true>(o, i, i1, P.keys, x, y, x1, y1);
-          else book_terminal_pair<false>(o, i, i1, P.keys, x, y, x1, y1);
+          if (o.flags & BF_ANTI) book_terminal_pair<true>(o, i, i1, G, x, y, x1, y1);
+          else book_terminal_pair<false>(o, i, i1, G, x, y, x1, y1);
         }
-        else if (o.kind == BK_BARRIER) book_sample_gbm_pair<BK_BARRIER>(o, i, i1, P.keys, x, y, x1, y1);
-        else if (o.kind == BK_ASIAN_DAILY_GEO) book_sample_gbm_pair<BK_ASIAN_DAILY_GEO>(o, i, i1, P.keys, x, y, x1, y1);
-        else book_sample_gbm_pair<BK_ASIAN_DAILY>(o, i, i1, P.keys, x, y, x1, y1);
+        else if (o.kind == BK_BARRIER) book_sample_gbm_pair<BK_BARRIER>(o, i, i1, G, x, y, x1, y1);
+        else if (o.kind == BK_ASIAN_DAILY_GEO) book_sample_gbm_pair<BK_ASIAN_DAILY_GEO>(o, i, i1, G, x, y, x1, y1);
+        else book_sample_gbm_pair<BK_ASIAN_DAILY>(o, i, i1, G, x, y, x1, y1);
         add(x, y);
         add(x1, y1);
         ++k;
         continue;
       }
-      book_dispatch(o, i, P, x, y);
+      book_dispatch(o, i, P, G, x, y);
       add(x, y);
     }
-    double v[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) v[k] = acc[k].value();
+    double v[5] = {ax.value(), ax.square(), ay.value(), axy.value(), ay.square()};
     of::block_sum<5>(v, red_sh);
     if (threadIdx.x == 0)
       for (int k = 0; k < 5; ++k) P.partials[(int64_t)tile.slot * 5 + k] = v[k];
@@ -1435,14 +1457,14 @@ struct GreekAcc<double, false> {
 // per tile); <double, false>: FP64 prices on the same draws.  FP32 Greeks:
 // the terminal group at four blocks per SM (64 registers), the Asian and
 // survival-barrier groups at three (the survival step's 91 registers capped
-// at 80, with a 4-byte spill: 351 ms for the 4096-option book against
-// 368 ms at two blocks); the FP64 modes at two.
-template <typename R, bool G, int KG>
+// at 80 spill 64 bytes: two blocks cost 5 % more); the FP64 modes at two.
+template <typename R, bool G, int KG, bool FULL>
 __global__ void __launch_bounds__(256, (!G || sizeof(R) == 8) ? 2 : (KG == of::KG_TERMINAL ? 4 : 3))
     book_greeks_kernel(const __grid_constant__ BookParams P, const of::GreekConsts<R>* __restrict__ gc) {
   constexpr int NC = G ? 13 : 5;
   __shared__ int tile_sh;
   __shared__ double red_sh[NC * 8];
+  extern __shared__ uint4 qtab[];
   for (;;) {
     if (threadIdx.x == 0) tile_sh = atomicAdd(P.counter, 1);
     __syncthreads();
@@ -1450,6 +1472,7 @@ __global__ void __launch_bounds__(256, (!G || sizeof(R) == 8) ? 2 : (KG == of::K
     if (t >= P.n_tiles) break;
     const BookTile tile = P.tiles[t];
     const of::GreekConsts<R>& c = gc[tile.opt];
+    const of::PhiloxGen<FULL> gen = book_gen<FULL>(qtab, P.tab, 4, c.steps, tile.first, c.stream, P.keys);
     GreekAcc<R, G> acc;
     // FP32: two samples at a time in packed pairs (terminal-only options, and
     // Asian and barrier options without antithetic twins, whose twins pair
@@ -1460,12 +1483,12 @@ __global__ void __launch_bounds__(256, (!G || sizeof(R) == 8) ? 2 : (KG == of::K
       const int local = k * blockDim.x + threadIdx.x;
       if (local >= tile.count) break;
       if constexpr (kPairs) {
-        if (pairs && k + 1 < P.ppt && local + (int)blockDim.x < tile.count) {
+        const uint64_t i0 = (uint64_t)(tile.first + local), i1 = i0 + blockDim.x;
+        if (pairs && k + 1 < P.ppt && local + (int)blockDim.x < tile.count && (FULL || (i0 >> 32) == (i1 >> 32))) {
           of::GreekSample<float> v0, v1;
-          const uint64_t i0 = (uint64_t)(tile.first + local), i1 = i0 + blockDim.x;
-          if constexpr (KG == of::KG_BARRIER) of::gk_barrier_pair_group<G>(c, i0, i1, P.keys, v0, v1);
-          else if constexpr (KG == of::KG_ASIAN) of::gk_asian_pair_group<G>(c, i0, i1, P.keys, P.obs_w, v0, v1);
-          else of::gk_terminal_pair_group<G>(c, i0, i1, P.keys, v0, v1);
+          if constexpr (KG == of::KG_BARRIER) of::gk_barrier_pair_group<G>(c, i0, i1, gen, v0, v1);
+          else if constexpr (KG == of::KG_ASIAN) of::gk_asian_pair_group<G>(c, i0, i1, gen, P.obs_w, v0, v1);
+          else of::gk_terminal_pair_group<G>(c, i0, i1, gen, v0, v1);
           acc.add(v0);
           acc.add(v1);
           ++k;
@@ -1473,7 +1496,7 @@ __global__ void __launch_bounds__(256, (!G || sizeof(R) == 8) ? 2 : (KG == of::K
         }
       }
       of::GreekSample<R> v;
-      of::gk_sample_group<R, G, KG>(c, (uint64_t)(tile.first + local), P.keys, P.obs_w, v);
+      of::gk_sample_group<R, G, KG>(c, (uint64_t)(tile.first + local), gen, P.obs_w, v);
       acc.add(v);
     }
     double v[NC];
@@ -1643,33 +1666,37 @@ struct of_book_plan {
   double* d_sums = nullptr;
   double* h_sums = nullptr;
   bool use_graph = true;
+  bool full = true;  // the q table covers every option (PhiloxGen<true>)
+  size_t smem() const { return (size_t)P.tab * sizeof(uint4); }
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 };
 
-template <typename R, bool G>
+template <typename R, bool G, bool FULL>
 static const void* book_greeks_kernel_for(int kg) {
-  return kg == of::KG_TERMINAL ? (const void*)book_greeks_kernel<R, G, of::KG_TERMINAL>
-         : kg == of::KG_ASIAN  ? (const void*)book_greeks_kernel<R, G, of::KG_ASIAN>
-                               : (const void*)book_greeks_kernel<R, G, of::KG_BARRIER>;
+  return kg == of::KG_TERMINAL ? (const void*)book_greeks_kernel<R, G, of::KG_TERMINAL, FULL>
+         : kg == of::KG_ASIAN  ? (const void*)book_greeks_kernel<R, G, of::KG_ASIAN, FULL>
+                               : (const void*)book_greeks_kernel<R, G, of::KG_BARRIER, FULL>;
 }
 
+template <bool FULL>
 static const void* book_kernel_for(int mode, int kg) {
-  if (mode == OF_BOOK_GREEKS) return book_greeks_kernel_for<float, true>(kg);
-  if (mode == OF_BOOK_PRICE_FP64) return book_greeks_kernel_for<double, false>(kg);
-  if (mode == OF_BOOK_GREEKS_FP64) return book_greeks_kernel_for<double, true>(kg);
-  return (const void*)book_kernel;
+  if (mode == OF_BOOK_GREEKS) return book_greeks_kernel_for<float, true, FULL>(kg);
+  if (mode == OF_BOOK_PRICE_FP64) return book_greeks_kernel_for<double, false, FULL>(kg);
+  if (mode == OF_BOOK_GREEKS_FP64) return book_greeks_kernel_for<double, true, FULL>(kg);
+  return (const void*)book_kernel<FULL>;
 }
 
-template <typename R, bool G>
+static const void* book_kernel_for(const of_book_plan* pl, int kg) {
+  return pl->full ? book_kernel_for<true>(pl->mode, kg) : book_kernel_for<false>(pl->mode, kg);
+}
+
 static void book_greeks_enqueue(of_book_plan* pl, cudaStream_t s) {
-  const of::GreekConsts<R>* gc = (const of::GreekConsts<R>*)pl->d_gc;
   for (int kg = 0; kg < of::KG_COUNT; ++kg) {
     if (pl->Pg[kg].n_tiles == 0) continue;
-    const dim3 grid((unsigned)pl->grid_g[kg]);
-    if (kg == of::KG_TERMINAL) book_greeks_kernel<R, G, of::KG_TERMINAL><<<grid, pl->block, 0, s>>>(pl->Pg[kg], gc);
-    else if (kg == of::KG_ASIAN) book_greeks_kernel<R, G, of::KG_ASIAN><<<grid, pl->block, 0, s>>>(pl->Pg[kg], gc);
-    else book_greeks_kernel<R, G, of::KG_BARRIER><<<grid, pl->block, 0, s>>>(pl->Pg[kg], gc);
+    void* args[] = {(void*)&pl->Pg[kg], (void*)&pl->d_gc};
+    cudaLaunchKernel(book_kernel_for(pl, kg), dim3((unsigned)pl->grid_g[kg]), dim3((unsigned)pl->block), args,
+                     pl->smem(), s);
   }
 }
 
@@ -1677,16 +1704,17 @@ static void book_enqueue(of_book_plan* pl, cudaStream_t s) {
   cudaMemsetAsync(pl->d_counter, 0, of::KG_COUNT * sizeof(int), s);
   const unsigned rgrid = (unsigned)((pl->n + 7) / 8);
   if (pl->mode == OF_BOOK_GREEKS) {
-    book_greeks_enqueue<float, true>(pl, s);
+    book_greeks_enqueue(pl, s);
     book_reduce_kernel<13><<<rgrid, 256, 0, s>>>(pl->d_partials, pl->d_begin, (int)pl->n, pl->d_sums);
   } else if (pl->mode == OF_BOOK_PRICE_FP64) {
-    book_greeks_enqueue<double, false>(pl, s);
+    book_greeks_enqueue(pl, s);
     book_reduce_kernel<5><<<rgrid, 256, 0, s>>>(pl->d_partials, pl->d_begin, (int)pl->n, pl->d_sums);
   } else if (pl->mode == OF_BOOK_GREEKS_FP64) {
-    book_greeks_enqueue<double, true>(pl, s);
+    book_greeks_enqueue(pl, s);
     book_reduce_kernel<13><<<rgrid, 256, 0, s>>>(pl->d_partials, pl->d_begin, (int)pl->n, pl->d_sums);
   } else {
-    book_kernel<<<pl->grid, pl->block, 0, s>>>(pl->P);
+    void* args[] = {(void*)&pl->P};
+    cudaLaunchKernel(book_kernel_for(pl, 0), dim3((unsigned)pl->grid), dim3((unsigned)pl->block), args, pl->smem(), s);
     book_reduce_kernel<5><<<rgrid, 256, 0, s>>>(pl->d_partials, pl->d_begin, (int)pl->n, pl->d_sums);
   }
   cudaMemcpyAsync(pl->h_sums, pl->d_sums, (size_t)pl->n * pl->nc * sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -1950,10 +1978,18 @@ static of_status book_plan_create(of_ctx* ctx, const of_book_entry* e, int64_t n
   P.divs = pl->d_divs;
   P.n_tiles = (int32_t)nt;
   P.ppt = pl->ppt;
+  uint32_t most = 1;  // counter blocks of the longest option
+  for (int64_t o = 0; o < n; ++o) {
+    const uint32_t spb = opts[(size_t)o].model == OF_MODEL_GBM ? 4 : 2;
+    most = std::max(most, ((uint32_t)opts[(size_t)o].steps + spb - 1) / spb);
+    if (pl->samples[(size_t)o] >> 32) pl->full = false;
+  }
+  if (most > kBookTab) pl->full = false;
+  P.tab = std::min(most, kBookTab);
   P.keys = of::philox_keys(cfg->seed);
   P.counter = pl->d_counter;
   P.partials = pl->d_partials;
-  const int per_sm = of_blocks_per_sm(book_kernel_for(pl->mode, of::KG_TERMINAL), pl->block, 0);
+  const int per_sm = of_blocks_per_sm(book_kernel_for(pl, of::KG_TERMINAL), pl->block, pl->smem());
   const int64_t cap = (int64_t)ctx->sm_count * per_sm;
   pl->grid = (int)std::max<int64_t>(1, std::min<int64_t>(cap, (int64_t)nt));
   if (pl->mode != OF_BOOK_PRICE) {
@@ -1966,7 +2002,7 @@ static of_status book_plan_create(of_ctx* ctx, const of_book_entry* e, int64_t n
       Q.tiles = pl->d_tiles + start;
       Q.n_tiles = (int32_t)(end - start);
       Q.counter = pl->d_counter + kg;
-      const int per = of_blocks_per_sm(book_kernel_for(pl->mode, kg), pl->block, 0);
+      const int per = of_blocks_per_sm(book_kernel_for(pl, kg), pl->block, pl->smem());
       pl->grid_g[kg] = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->sm_count * per, (int64_t)(end - start)));
       start = end;
     }

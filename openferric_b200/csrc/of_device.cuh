@@ -239,6 +239,31 @@ __device__ __forceinline__ uint4 philox_terms(const PhiloxTab& T, uint32_t q, co
   return FULL || q < T.n ? T.tab[q] : philox_q(q, T.hi, T.stream, K);
 }
 
+// The counter blocks of one stream for a block of threads: the keys and the
+// stream's table.  lane(i) is sample i's part; a copy serves the samples of
+// one high word.  FULL: the table covers every counter block and every
+// sample's high word is 0; otherwise lane(i) moves the generator to the high
+// word of i (without a table where that is not the table's).  The test costs
+// the book's step loops 6 %, so its launches use FULL whenever they can.
+template <bool FULL>
+struct PhiloxGen {
+  const PhiloxKeys* K;
+  PhiloxTab T;
+  __device__ __forceinline__ PhiloxLane lane(uint64_t i) {
+    if constexpr (FULL) return philox_lane((uint32_t)i, 0u, *K);
+    const uint32_t hi = (uint32_t)(i >> 32);
+    if (hi != T.hi) {
+      T.hi = hi;
+      T.n = 0;
+    }
+    return philox_lane((uint32_t)i, hi, *K);
+  }
+  __device__ __forceinline__ uint4 terms(uint32_t q) const { return philox_terms<FULL>(T, q, *K); }
+  __device__ __forceinline__ uint4 block(uint32_t q, const PhiloxLane& L) const {
+    return philox_block(terms(q), L, *K);
+  }
+};
+
 // 1 + k 2^-23 with k the top 23 bits of r: 0x3F800000 | (r >> 9) as one funnel
 // shift (0x7F << 23 is 1.0's exponent field).
 __device__ __forceinline__ float unit_mantissa(uint32_t r) {
@@ -292,6 +317,26 @@ __device__ __forceinline__ float inv_normal_vq(float v, float q) {
     for (int i = OF_INVN_DEG_T - 1; i >= 0; --i) p = fmaf(p, s, kInvnTail[i]);
   }
   return x * p;
+}
+
+// inv_normal_vq of two arguments: the central polynomial in packed pairs, each
+// half the scalar form bit for bit; a half in the tail (0.3 % of unconditioned
+// draws) is taken again in scalar form.  The survival step of the barrier
+// Greeks issues 62 % of its cycles to the FMA pipe: the Greeks of 192
+// options of 2^13..2^15 paths by 25..1260 steps took 4.02 ms (antithetic 4.38)
+// with the pair, 4.12 (4.55) with two scalar calls.
+__device__ __forceinline__ float2 inv_normal_vq2(float2 v, float2 q) {
+  const float2 t = mul2(mul2(splat2(4.0f), v), q);
+  const float2 x = sub2(v, q);
+  const float2 w = make_float2(-__log2f(t.x), -__log2f(t.y));
+  const float2 s = sub2(w, splat2(OF_INVN_C_CENTER));
+  float2 p = splat2(kInvnCentral[OF_INVN_DEG_C]);
+#pragma unroll
+  for (int i = OF_INVN_DEG_C - 1; i >= 0; --i) p = fma2(p, s, splat2(kInvnCentral[i]));
+  float2 z = mul2(x, p);
+  if (!(w.x < OF_INVN_W_SPLIT)) z.x = inv_normal_vq(v.x, q.x);
+  if (!(w.y < OF_INVN_W_SPLIT)) z.y = inv_normal_vq(v.y, q.y);
+  return z;
 }
 
 // u32 -> uniform in (0,1), the same grid as normal_from_u32: (k + 0.5) 2^-23.
