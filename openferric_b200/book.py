@@ -153,14 +153,28 @@ class BookPlan:
             pass
 
 
+def _price_once(entries, seed, block, paths_per_thread, device, greeks):
+    """One launch in the context's cached buffers: raw results and Greeks (or None), and the volatilities."""
+    ctx = context(device)
+    n = len(entries)
+    arr, keep, vols = book_entries_abi(entries)
+    cfg = A.OfBookConfig(seed=int(seed) & 0xFFFFFFFFFFFFFFFF, block=block, paths_per_thread=paths_per_thread)
+    out = (A.OfMcResult * n)()
+    gr = (A.OfBookGreeks * n)() if greeks else None
+    with ctx.lock:
+        if greeks:
+            ctx.check(ctx._L.of_mc_price_book_greeks(ctx.handle, arr, n, C.byref(cfg), out, gr))
+        else:
+            ctx.check(ctx._L.of_mc_price_book(ctx.handle, arr, n, C.byref(cfg), out))
+    del keep
+    return out, gr, vols
+
+
 def price_book(entries: Sequence[BookEntry], seed: int, block: int = 0, paths_per_thread: int = 0,
                device: int = 0) -> List[PricingResult]:
-    plan = BookPlan(entries, seed, block, paths_per_thread, use_graph=False, device=device)
-    try:
-        plan.launch()
-        return plan.results()
-    finally:
-        plan.close()
+    out, _, vols = _price_once(entries, seed, block, paths_per_thread, device, False)
+    return [PricingResult(price=r.price, stderr=r.stderr_, diagnostics=_diagnostics(e.num_paths, e.num_steps, vol))
+            for e, r, vol in zip(entries, out, vols)]
 
 
 def price_book_greeks(entries: Sequence[BookEntry], seed: int, block: int = 0, paths_per_thread: int = 0,
@@ -169,12 +183,14 @@ def price_book_greeks(entries: Sequence[BookEntry], seed: int, block: int = 0, p
     one persistent launch (of_mc_price_book_greeks).  GBM options without
     discrete dividends; barrier options are priced by one-step survival (no
     control variate), the other payoffs by the book's own estimator."""
-    plan = BookPlan(entries, seed, block, paths_per_thread, use_graph=False, device=device, mode=A.OF_BOOK_GREEKS)
-    try:
-        plan.launch()
-        return plan.greeks_results()
-    finally:
-        plan.close()
+    out, gr, vols = _price_once(entries, seed, block, paths_per_thread, device, True)
+    results = []
+    for e, r, g, vol in zip(entries, out, gr, vols):
+        res = PricingResult(price=r.price, stderr=r.stderr_,
+                            diagnostics=_diagnostics(e.num_paths, e.num_steps, vol))
+        res.greeks, se = _greeks_of(g)
+        results.append(BookGreeksResult(res, se))
+    return results
 
 
 def price_book_greeks_fp64(entries: Sequence[BookEntry], seed: int, block: int = 0, paths_per_thread: int = 0,

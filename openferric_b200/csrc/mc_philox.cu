@@ -1509,12 +1509,14 @@ __global__ void __launch_bounds__(256, (!G || sizeof(R) == 8) ? 2 : (KG == of::K
 }
 
 // Per-option sums over its tile slots [begin[o], begin[o+1]) in fixed order;
-// NC sums per slot.
+// NC sums per slot, written to pinned host memory.  It runs after the launch's
+// last tile, so it also clears the tile counters for the next one.
 template <int NC>
 __global__ void book_reduce_kernel(const double* __restrict__ partials, const int32_t* __restrict__ begin, int n_opts,
-                                   double* __restrict__ sums) {
+                                   double* __restrict__ sums, int* __restrict__ counter) {
   const int o = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
+  if (blockIdx.x == 0 && threadIdx.x < of::KG_COUNT) counter[threadIdx.x] = 0;
   if (o >= n_opts) return;
   double acc[NC];
 #pragma unroll
@@ -1661,10 +1663,10 @@ struct of_book_plan {
   BookDiv* d_divs = nullptr;
   void* d_gc = nullptr;  // GreekConsts<float> (Greeks mode) or <double> (FP64 mode)
   int* d_counter = nullptr;
-  double* d_partials = nullptr;
   int32_t* d_begin = nullptr;
-  double* d_sums = nullptr;
-  double* h_sums = nullptr;
+  char* d_image = nullptr;  // one allocation and one upload: the six tables above and the counters
+  double* d_partials = nullptr;
+  double* h_sums = nullptr;  // pinned, written by the reduction
   bool use_graph = true;
   bool full = true;  // the q table covers every option (PhiloxGen<true>)
   size_t smem() const { return (size_t)P.tab * sizeof(uint4); }
@@ -1701,23 +1703,17 @@ static void book_greeks_enqueue(of_book_plan* pl, cudaStream_t s) {
 }
 
 static void book_enqueue(of_book_plan* pl, cudaStream_t s) {
-  cudaMemsetAsync(pl->d_counter, 0, of::KG_COUNT * sizeof(int), s);
-  const unsigned rgrid = (unsigned)((pl->n + 7) / 8);
-  if (pl->mode == OF_BOOK_GREEKS) {
-    book_greeks_enqueue(pl, s);
-    book_reduce_kernel<13><<<rgrid, 256, 0, s>>>(pl->d_partials, pl->d_begin, (int)pl->n, pl->d_sums);
-  } else if (pl->mode == OF_BOOK_PRICE_FP64) {
-    book_greeks_enqueue(pl, s);
-    book_reduce_kernel<5><<<rgrid, 256, 0, s>>>(pl->d_partials, pl->d_begin, (int)pl->n, pl->d_sums);
-  } else if (pl->mode == OF_BOOK_GREEKS_FP64) {
-    book_greeks_enqueue(pl, s);
-    book_reduce_kernel<13><<<rgrid, 256, 0, s>>>(pl->d_partials, pl->d_begin, (int)pl->n, pl->d_sums);
-  } else {
+  if (pl->mode == OF_BOOK_PRICE) {
     void* args[] = {(void*)&pl->P};
     cudaLaunchKernel(book_kernel_for(pl, 0), dim3((unsigned)pl->grid), dim3((unsigned)pl->block), args, pl->smem(), s);
-    book_reduce_kernel<5><<<rgrid, 256, 0, s>>>(pl->d_partials, pl->d_begin, (int)pl->n, pl->d_sums);
+  } else {
+    book_greeks_enqueue(pl, s);
   }
-  cudaMemcpyAsync(pl->h_sums, pl->d_sums, (size_t)pl->n * pl->nc * sizeof(double), cudaMemcpyDeviceToHost, s);
+  const unsigned rgrid = (unsigned)((pl->n + 7) / 8);
+  if (pl->nc == 13)
+    book_reduce_kernel<13><<<rgrid, 256, 0, s>>>(pl->d_partials, pl->d_begin, (int)pl->n, pl->h_sums, pl->d_counter);
+  else
+    book_reduce_kernel<5><<<rgrid, 256, 0, s>>>(pl->d_partials, pl->d_begin, (int)pl->n, pl->h_sums, pl->d_counter);
 }
 
 extern "C" void of_book_plan_destroy(of_book_plan* pl) {
@@ -1729,15 +1725,8 @@ extern "C" void of_book_plan_destroy(of_book_plan* pl) {
     delete pl;
     return;
   }
-  cudaFree(pl->d_opts);
-  cudaFree(pl->d_tiles);
-  cudaFree(pl->d_obs);
-  cudaFree(pl->d_divs);
-  cudaFree(pl->d_gc);
-  cudaFree(pl->d_counter);
+  cudaFree(pl->d_image);
   cudaFree(pl->d_partials);
-  cudaFree(pl->d_begin);
-  cudaFree(pl->d_sums);
   if (pl->h_sums) cudaFreeHost(pl->h_sums);
   delete pl;
 }
@@ -1785,13 +1774,6 @@ static of_status book_plan_create(of_ctx* ctx, const of_book_entry* e, int64_t n
   pl->cv_kind.resize((size_t)n);
   pl->cv_expected.resize((size_t)n);
   pl->discount.resize((size_t)n);
-  struct Pending {
-    int32_t opt;
-    int64_t first;
-    int32_t count;
-    double cost;
-  };
-  std::vector<Pending> pend;
   const int64_t tile_samples = (int64_t)pl->block * pl->ppt;
   for (int64_t o = 0; o < n; ++o) {
     const of_book_entry& b = e[o];
@@ -1888,89 +1870,100 @@ static of_status book_plan_create(of_ctx* ctx, const of_book_entry* e, int64_t n
     pl->cv_expected[(size_t)o] = b.cv_expected;
     pl->discount[(size_t)o] = b.discount_factor;
     pl->path_steps += (double)b.num_paths * (double)b.model.steps;
-    for (int64_t first = 0; first < samples; first += tile_samples) {
-      const int32_t cnt = (int32_t)std::min<int64_t>(tile_samples, samples - first);
-      const double legs = b.antithetic ? 2.0 : 1.0;
-      pend.push_back({(int32_t)o, first, cnt, (double)cnt * legs * (double)b.model.steps});
-    }
   }
-  if (pend.size() > (size_t)2147483647) return fail(of_fail(ctx, OF_ERR_INVALID_INPUT, "too many tiles"));
-  // Slots in option-major order, schedule longest tile first.
-  std::vector<int32_t> begin((size_t)n + 1, 0);
-  for (size_t k = 0; k < pend.size(); ++k) begin[(size_t)pend[k].opt + 1]++;
-  for (int64_t o = 0; o < n; ++o) begin[(size_t)o + 1] += begin[(size_t)o];
-  // The schedule: the Greeks modes' kind groups in turn, longest tile first
-  // within a group, ties in slot order (a stable sort of the tiles by group,
-  // then cost descending).  An option's tiles are consecutive slots; all but
-  // its last share one cost, and the last may be shorter.  So the schedule is
-  // built from runs of equal-cost tiles, at most two per option, sorted
-  // stably: the same order as sorting the tiles, at O(n log n + tiles)
-  // instead of O(tiles log tiles) (a million tiles for a book of long-dated
-  // options at 2^25 paths each).
+  // Slots in option-major order, schedule longest tile first: the Greeks
+  // modes' kind groups in turn, longest tile first within a group, ties in
+  // slot order (a stable sort of the tiles by group, then cost descending).
+  // An option's tiles are consecutive slots; all but its last share one cost,
+  // and the last may be shorter.  So the schedule is built from runs of
+  // equal-cost tiles, at most two per option, sorted stably: the same order as
+  // sorting the tiles, at O(n log n + tiles) instead of O(tiles log tiles) (a
+  // million tiles for a book of long-dated options at 2^25 paths each).
   struct Run {
-    size_t begin, end;
+    int32_t opt, count;  // samples of each of its tiles
+    int64_t slot, tiles, first;
     int group;
     double cost;
   };
   std::vector<Run> runs;
   runs.reserve((size_t)n * 2);
-  for (size_t k = 0; k < pend.size();) {
-    const int32_t o = pend[k].opt;
+  std::vector<int64_t> begin((size_t)n + 1, 0);
+  int64_t group_tiles[of::KG_COUNT] = {0, 0, 0};
+  for (int64_t o = 0; o < n; ++o) {
     const int group = pl->mode != OF_BOOK_PRICE ? of::gk_group(gcs[(size_t)o].kind) : 0;
-    size_t e = k;
-    while (e < pend.size() && pend[e].opt == o && pend[e].cost == pend[k].cost) ++e;
-    runs.push_back({k, e, group, pend[k].cost});
-    k = e;
+    const double per = (e[o].antithetic ? 2.0 : 1.0) * (double)e[o].model.steps;
+    const int64_t samples = pl->samples[(size_t)o], whole = samples / tile_samples, rest = samples % tile_samples;
+    int64_t slot = begin[(size_t)o];
+    if (whole)
+      runs.push_back({(int32_t)o, (int32_t)tile_samples, slot, whole, 0, group, (double)tile_samples * per});
+    slot += whole;
+    if (rest) runs.push_back({(int32_t)o, (int32_t)rest, slot++, 1, whole * tile_samples, group, (double)rest * per});
+    group_tiles[group] += slot - begin[(size_t)o];
+    begin[(size_t)o + 1] = slot;
+    if (slot > 2147483647) return fail(of_fail(ctx, OF_ERR_INVALID_INPUT, "too many tiles"));
   }
   std::stable_sort(runs.begin(), runs.end(), [](const Run& a, const Run& b) {
     return a.group != b.group ? a.group < b.group : a.cost > b.cost;
   });
-  std::vector<BookTile> sorted;
-  sorted.reserve(pend.size());
-  for (const Run& r : runs)
-    for (size_t k = r.begin; k < r.end; ++k)
-      sorted.push_back({pend[k].opt, pend[k].count, pend[k].first, (int32_t)k, 0});
-  pl->n_tiles = (int64_t)sorted.size();
-
-  const size_t nt = sorted.size();
-  // A plan that lives inside one call borrows the context's cached buffers:
-  // no cudaMalloc / cudaFree / cudaMallocHost per call.
-  auto dalloc = [&](void** p, size_t bytes, int slot) {
-    if (pl->scratch) return of_scratch(ctx, slot, bytes, p) == OF_OK;
-    return cudaMalloc(p, bytes) == cudaSuccess;
+  const size_t nt = (size_t)begin[(size_t)n];
+  pl->n_tiles = (int64_t)nt;
+  // The tables in one image, uploaded once: [options | tiles | weights |
+  // dividends | Greek constants | slot ranges | counters].  A plan that lives
+  // inside one call borrows the context's cached buffers (no cudaMalloc,
+  // cudaFree or cudaMallocHost per call) and stages images of up to 8 MB, a
+  // quarter of a million tiles, in its pinned buffer behind the sums; larger
+  // ones go from pageable memory, so that the buffer stays small.  A call on
+  // 384 options (21,000 tiles) spends 0.6 ms beside its kernels, against 2.0
+  // and up with nine allocations, six uploads and their frees.
+  size_t bytes = 0;
+  auto place = [&](size_t size) {
+    const size_t at = bytes;
+    bytes += (size + 255) & ~(size_t)255;
+    return at;
   };
-  const size_t sum_bytes = (size_t)n * pl->nc * sizeof(double);
-  bool ok = dalloc((void**)&pl->d_opts, opts.size() * sizeof(BookOpt), SLOT_BOOK) &&
-            dalloc((void**)&pl->d_tiles, nt * sizeof(BookTile), SLOT_TILES) &&
-            dalloc((void**)&pl->d_obs, std::max<size_t>(1, obs.size()) * sizeof(float), SLOT_BOOK_OBS) &&
-            dalloc((void**)&pl->d_divs, std::max<size_t>(1, divs.size()) * sizeof(BookDiv), SLOT_BOOK_DIVS) &&
-            dalloc((void**)&pl->d_counter, of::KG_COUNT * sizeof(int), SLOT_BOOK_COUNTER) &&
-            dalloc((void**)&pl->d_partials, nt * pl->nc * sizeof(double), SLOT_BOOK_PARTIALS) &&
-            dalloc((void**)&pl->d_begin, begin.size() * sizeof(int32_t), SLOT_BOOK_BEGIN) &&
-            dalloc((void**)&pl->d_sums, sum_bytes, SLOT_BOOK_SUMS);
-  if (ok) ok = pl->scratch ? of_pinned(ctx, sum_bytes, (void**)&pl->h_sums) == OF_OK
+  const size_t gc_size = pl->mode == OF_BOOK_PRICE    ? 0
+                         : pl->mode == OF_BOOK_GREEKS ? sizeof(of::GreekConsts<float>)
+                                                      : sizeof(of::GreekConsts<double>);
+  const size_t at_opts = place(opts.size() * sizeof(BookOpt)), at_tiles = place(nt * sizeof(BookTile)),
+               at_obs = place(obs.size() * sizeof(float)), at_divs = place(divs.size() * sizeof(BookDiv)),
+               at_gc = place((size_t)n * gc_size), at_begin = place(begin.size() * sizeof(int32_t)),
+               at_counter = place(of::KG_COUNT * sizeof(int));
+  const size_t sum_bytes = ((size_t)n * pl->nc * sizeof(double) + 255) & ~(size_t)255;
+  const bool staged = pl->scratch && bytes <= ((size_t)8 << 20);
+  auto dalloc = [&](void** p, size_t size, int slot) {
+    if (pl->scratch) return of_scratch(ctx, slot, size, p) == OF_OK;
+    return cudaMalloc(p, size) == cudaSuccess;
+  };
+  bool ok = dalloc((void**)&pl->d_image, bytes, SLOT_BOOK) &&
+            dalloc((void**)&pl->d_partials, nt * pl->nc * sizeof(double), SLOT_BOOK_PARTIALS);
+  if (ok) ok = pl->scratch ? of_pinned(ctx, sum_bytes + (staged ? bytes : 0), (void**)&pl->h_sums) == OF_OK
                            : cudaMallocHost(&pl->h_sums, sum_bytes) == cudaSuccess;
   if (!ok) return fail(of_fail(ctx, OF_ERR_ALLOC, "book plan allocation failed"));
-  if (pl->mode == OF_BOOK_GREEKS) {  // the constants rounded once to FP32
-    std::vector<of::GreekConsts<float>> gf(gcs.size());
-    for (size_t k = 0; k < gcs.size(); ++k) gf[k] = round_greek_consts(gcs[k]);
-    if (!dalloc(&pl->d_gc, gf.size() * sizeof(gf[0]), SLOT_BOOK_GC))
-      return fail(of_fail(ctx, OF_ERR_ALLOC, "book plan allocation failed"));
-    if (cudaMemcpy(pl->d_gc, gf.data(), gf.size() * sizeof(gf[0]), cudaMemcpyHostToDevice) != cudaSuccess)
-      return fail(of_fail(ctx, OF_ERR_CUDA, "book upload failed"));
-  } else if (pl->mode == OF_BOOK_PRICE_FP64 || pl->mode == OF_BOOK_GREEKS_FP64) {
-    if (!dalloc(&pl->d_gc, gcs.size() * sizeof(gcs[0]), SLOT_BOOK_GC))
-      return fail(of_fail(ctx, OF_ERR_ALLOC, "book plan allocation failed"));
-    if (cudaMemcpy(pl->d_gc, gcs.data(), gcs.size() * sizeof(gcs[0]), cudaMemcpyHostToDevice) != cudaSuccess)
-      return fail(of_fail(ctx, OF_ERR_CUDA, "book upload failed"));
-  }
-  if (cudaMemcpy(pl->d_opts, opts.data(), opts.size() * sizeof(BookOpt), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(pl->d_tiles, sorted.data(), nt * sizeof(BookTile), cudaMemcpyHostToDevice) != cudaSuccess ||
-      (!obs.empty() && cudaMemcpy(pl->d_obs, obs.data(), obs.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) ||
-      (!divs.empty() &&
-       cudaMemcpy(pl->d_divs, divs.data(), divs.size() * sizeof(BookDiv), cudaMemcpyHostToDevice) != cudaSuccess) ||
-      cudaMemcpy(pl->d_begin, begin.data(), begin.size() * sizeof(int32_t), cudaMemcpyHostToDevice) != cudaSuccess)
+  std::vector<char> heap(staged ? 0 : bytes);
+  char* const image = staged ? (char*)pl->h_sums + sum_bytes : heap.data();
+  std::copy(opts.begin(), opts.end(), (BookOpt*)(image + at_opts));
+  std::copy(obs.begin(), obs.end(), (float*)(image + at_obs));
+  std::copy(divs.begin(), divs.end(), (BookDiv*)(image + at_divs));
+  std::copy(begin.begin(), begin.end(), (int32_t*)(image + at_begin));
+  std::fill_n((int*)(image + at_counter), (int)of::KG_COUNT, 0);
+  if (pl->mode == OF_BOOK_GREEKS)  // the constants rounded once to FP32
+    for (size_t k = 0; k < gcs.size(); ++k) ((of::GreekConsts<float>*)(image + at_gc))[k] = round_greek_consts(gcs[k]);
+  else
+    std::copy(gcs.begin(), gcs.end(), (of::GreekConsts<double>*)(image + at_gc));
+  BookTile* tile = (BookTile*)(image + at_tiles);
+  for (const Run& r : runs)
+    for (int64_t k = 0; k < r.tiles; ++k)
+      *tile++ = {r.opt, r.count, r.first + k * tile_samples, (int32_t)(r.slot + k), 0};
+  // (from pageable memory the call returns once the bytes have left it)
+  if (cudaMemcpyAsync(pl->d_image, image, bytes, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
     return fail(of_fail(ctx, OF_ERR_CUDA, "book upload failed"));
+  pl->d_opts = (BookOpt*)(pl->d_image + at_opts);
+  pl->d_tiles = (BookTile*)(pl->d_image + at_tiles);
+  pl->d_obs = (float*)(pl->d_image + at_obs);
+  pl->d_divs = (BookDiv*)(pl->d_image + at_divs);
+  pl->d_gc = pl->d_image + at_gc;
+  pl->d_begin = (int32_t*)(pl->d_image + at_begin);
+  pl->d_counter = (int*)(pl->d_image + at_counter);
   BookParams& P = pl->P;
   P.opts = pl->d_opts;
   P.tiles = pl->d_tiles;
@@ -1993,17 +1986,16 @@ static of_status book_plan_create(of_ctx* ctx, const of_book_entry* e, int64_t n
   const int64_t cap = (int64_t)ctx->sm_count * per_sm;
   pl->grid = (int)std::max<int64_t>(1, std::min<int64_t>(cap, (int64_t)nt));
   if (pl->mode != OF_BOOK_PRICE) {
-    size_t start = 0;
+    int64_t start = 0;
     for (int kg = 0; kg < of::KG_COUNT; ++kg) {
-      size_t end = start;
-      while (end < nt && of::gk_group(gcs[(size_t)sorted[end].opt].kind) == kg) ++end;
+      const int64_t end = start + group_tiles[kg];
       BookParams& Q = pl->Pg[kg];
       Q = P;
       Q.tiles = pl->d_tiles + start;
       Q.n_tiles = (int32_t)(end - start);
       Q.counter = pl->d_counter + kg;
       const int per = of_blocks_per_sm(book_kernel_for(pl, kg), pl->block, pl->smem());
-      pl->grid_g[kg] = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->sm_count * per, (int64_t)(end - start)));
+      pl->grid_g[kg] = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->sm_count * per, end - start));
       start = end;
     }
   }

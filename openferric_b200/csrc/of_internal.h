@@ -20,8 +20,7 @@ enum OfSlot {
   SLOT_OBS = 2,        // per-step observation weights
   SLOT_INJECT = 3,     // injected normals (test hook)
   SLOT_STRIKES = 4,    // strike strip
-  SLOT_BOOK = 5,       // batched-book option table
-  SLOT_TILES = 6,      // batched-book tile table
+  SLOT_BOOK = 5,       // batched-book tables of a plan run inside one call
   SLOT_DIVIDENDS = 7,  // discrete dividend triggers
   SLOT_LSM_PATHS = 8,  // LSM path store (time-major)
   SLOT_LSM_VALUES = 9, // LSM cash flows
@@ -34,14 +33,8 @@ enum OfSlot {
   SLOT_LSM_PATHS_B = 16,   // second LSM buffer set: the next batch generates into it
   SLOT_LSM_VALUES_B = 17,  // while the current one runs its passes
   SLOT_LSM_AUX_B = 18,
-  SLOT_BOOK_DIVS = 19,     // book plans run inside one call (of_mc_price_book, the SE driver):
-  SLOT_BOOK_GC = 20,       // their device tables and sums come from these slots
-  SLOT_BOOK_COUNTER = 21,
-  SLOT_BOOK_PARTIALS = 22,
-  SLOT_BOOK_BEGIN = 23,
-  SLOT_BOOK_SUMS = 24,
-  SLOT_BOOK_OBS = 25,
-  SLOT_COUNT = 26
+  SLOT_BOOK_PARTIALS = 19,   // and its per-tile sums
+  SLOT_COUNT = 20
 };
 
 struct of_ctx {

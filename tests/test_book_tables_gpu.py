@@ -13,7 +13,8 @@ import pytest
 
 from openferric_b200 import (AsianOption, AsianSpec, Averaging, BarrierDirection, BarrierOption, BarrierSpec,
                              BarrierStyle, Market, OptionType, StrikeType, VanillaOption, VarianceReduction)
-from openferric_b200.book import BookEntry, price_book, price_book_greeks
+from openferric_b200 import _abi as A
+from openferric_b200.book import BookEntry, BookPlan, price_book, price_book_greeks
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +44,24 @@ def test_a_book_keeps_its_draws_beside_a_longer_option(price, steps):
     bs = 100.0 * math.exp(-0.01) * cdf(d1) - 100.0 * math.exp(-0.03) * cdf(d1 - 0.3)
     last = beside[-1]
     assert abs(last.price - bs) <= 4.5 * last.stderr
+
+
+@pytest.mark.parametrize("greeks", [False, True])
+@pytest.mark.parametrize("paths", [1, 31, 1 << 13, 9_000_000])
+def test_a_call_and_a_plan_give_the_same_results(greeks, paths):
+    """The call stages its tables in pinned memory up to 8 MB (262,144 tiles;
+    9,000,000 samples in tiles of 32 are past it), the plan uploads its own."""
+    mk, book = _book(1, paths)
+    book = book[:2] + _book(5, 100)[1]
+    kw = dict(seed=23, block=32, paths_per_thread=1)
+    plan = BookPlan(book, mode=A.OF_BOOK_GREEKS if greeks else A.OF_BOOK_PRICE, **kw)
+    for _ in range(2):  # the second launch finds its tile counters cleared
+        plan.launch()
+        want = plan.greeks_results() if greeks else plan.results()
+    plan.close()
+    got = price_book_greeks(book, **kw) if greeks else price_book(book, **kw)
+    for g, w in zip(got, want):
+        if greeks:
+            assert (g.result.greeks, g.greeks_stderr) == (w.result.greeks, w.greeks_stderr)
+            g, w = g.result, w.result
+        assert (g.price, g.stderr) == (w.price, w.stderr)
