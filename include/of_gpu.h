@@ -555,7 +555,7 @@ of_status of_xoshiro_jump(of_ctx* ctx, uint64_t seed, const uint64_t* draws, int
 of_status of_test_bounded_wait(of_ctx* ctx, int32_t arrive, uint32_t limit_us, int32_t* waited_ok,
                                double* elapsed_us);
 
-/* ---- Heston pathwise adjoint (FP32, checkpointed) ------------------------ */
+/* ---- Heston pathwise Greeks (FP32) ---------------------------------------- */
 typedef struct of_heston_adjoint_params {
   double spot, strike, rate, dividend_yield, expiry;
   double kappa, theta, xi, rho, v0;
@@ -565,7 +565,7 @@ typedef struct of_heston_adjoint_params {
   int32_t payoff;           /* OF_PAYOFF_VANILLA, or OF_PAYOFF_ASIAN: arithmetic average of
                                the spot at every step 1..num_steps */
   int32_t scheme;           /* OF_MODEL_HESTON_QE or OF_MODEL_HESTON_EULER */
-  int32_t checkpoint_every; /* path-state checkpoint interval (32) */
+  int32_t checkpoint_every; /* path-state checkpoint interval of the backward sweep (32) */
   int32_t forward_only;     /* 0: price + adjoint Greeks; 1: price only (FP32); 2: price only
                                in FP64 arithmetic on the same draws (bump-and-revalue with
                                common random numbers: a 1e-4 relative bump is below the FP32
@@ -592,9 +592,11 @@ typedef struct of_adjoint_result {
   double kernel_ms;
 } of_adjoint_result;
 
-/* Price and all seven Heston sensitivities from one forward pass (path state
- * checkpointed every `checkpoint_every` steps) and one backward sweep that
- * recomputes each segment and regenerates its counter-based draws.  The
+/* Price and all seven Heston sensitivities: the pathwise derivative of every
+ * path, carried along with the path, or, where few paths are expected in the
+ * money, from a forward pass (path state checkpointed every
+ * `checkpoint_every` steps) and a backward sweep over the paths in the money
+ * that recomputes each segment and regenerates its counter-based draws.  The
  * reference has forward-mode Heston delta only (heston_price_delta_aad,
  * src/engines/monte_carlo/mc_aad.rs:280-342); the other six have no
  * reference counterpart. */

@@ -3,8 +3,9 @@ torch.autograd.Function.
 
 `price_with_adjoint` prices a European or daily-fixing arithmetic Asian option
 under Heston (Andersen QE, FP32 paths) and returns the price with
-d/d(S0, r, v0, kappa, theta, xi, rho) from one forward pass and one backward
-sweep.  `HestonAdjointFunction.apply(params, spec)` exposes the same call to
+d/d(S0, r, v0, kappa, theta, xi, rho) from one pass that carries the pathwise
+derivatives along, or a forward pass and a backward sweep over the paths in the
+money where those are few.  `HestonAdjointFunction.apply(params, spec)` exposes the same call to
 autograd: the forward returns the price, the backward multiplies the incoming
 gradient by the adjoint Greeks computed in the forward.
 """

@@ -294,6 +294,30 @@ __device__ __forceinline__ float normal_from_u32(uint32_t r) {
   return x * p;
 }
 
+// The tail polynomial of normal_from_u32 (w >= OF_INVN_W_SPLIT).
+__device__ __forceinline__ float invn_tail(float w) {
+  const float s = sqrtf(w) - OF_INVN_T_CENTER;
+  float p = kInvnTail[OF_INVN_DEG_T];
+#pragma unroll
+  for (int i = OF_INVN_DEG_T - 1; i >= 0; --i) p = fmaf(p, s, kInvnTail[i]);
+  return p;
+}
+
+// normal_from_u32 of two draws: the central polynomial in packed pairs, each
+// half the scalar form bit for bit.
+__device__ __forceinline__ float2 normals2_from_u32(uint32_t a, uint32_t b) {
+  const float2 f = make_float2(unit_mantissa(a), unit_mantissa(b));
+  const float2 x = add2(fma2(splat2(2.0f), f, splat2(-3.0f)), splat2(1.1920928955078125e-7f));
+  const float2 w = make_float2(-__log2f(fmaf(-x.x, x.x, 1.0f)), -__log2f(fmaf(-x.y, x.y, 1.0f)));
+  const float2 s = sub2(w, splat2(OF_INVN_C_CENTER));
+  float2 p = splat2(kInvnCentral[OF_INVN_DEG_C]);
+#pragma unroll
+  for (int i = OF_INVN_DEG_C - 1; i >= 0; --i) p = fma2(p, s, splat2(kInvnCentral[i]));
+  if (!(w.x < OF_INVN_W_SPLIT)) p.x = invn_tail(w.x);
+  if (!(w.y < OF_INVN_W_SPLIT)) p.y = invn_tail(w.y);
+  return mul2(x, p);
+}
+
 // Phi^-1(v) for v in (0,1) given q = 1 - v (each exact or rounded once, so
 // that either tail keeps its relative precision): the polynomials of
 // normal_from_u32 on x = v - q = 2v - 1 and w = -log2(4 v q), whose fit
