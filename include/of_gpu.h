@@ -537,6 +537,11 @@ typedef struct of_lsm_barrier_contract {
 of_status of_lsm_barrier(of_ctx* ctx, const of_lsm_barrier_contract* contract, const of_lsm_config* cfg,
                          of_lsm_result* result);
 
+/* sum_i sum_j min(t_i, t_j) of n fixing times, on the host: the covariance sum
+ * of the geometric-Asian closed form (src/pricing/asian.rs:86-136), bit for bit
+ * the sum of its double loop (i outer, j inner). */
+of_status of_min_sum_in_order(const double* times, int64_t n, double* out);
+
 /* xoshiro256++ jump-ahead: the state of the stream seeded with `seed`
  * (Xoshiro256PlusPlus::seed_from_u64, src/math/fast_rng.rs:36-48) after
  * `draws` calls of next_u64, computed on the device by GF(2) matrix powers.

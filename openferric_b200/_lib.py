@@ -25,7 +25,7 @@ EXPORTED = [
     "of_lsm_price", "of_xoshiro_jump", "of_heston_price_adjoint", "of_mc_european_gpu", "of_mc_strip_noalloc",
     "of_measure_device_peaks", "of_lsm_bermudan", "of_mc_european_qmc", "of_autotune_strip", "of_autotune_book",
     "of_test_bounded_wait", "of_book_price_to_stderr", "of_book_plan_greeks", "of_mc_price_book_greeks",
-    "of_book_price_to_stderr_greeks", "of_lsm_barrier",
+    "of_book_price_to_stderr_greeks", "of_lsm_barrier", "of_min_sum_in_order",
 ]
 
 
@@ -84,6 +84,8 @@ def _declare(L):
     L.of_lsm_barrier.restype = C.c_int
     L.of_xoshiro_jump.argtypes = [vp, C.c_uint64, P(C.c_uint64), C.c_int64, P(C.c_uint64)]
     L.of_xoshiro_jump.restype = C.c_int
+    L.of_min_sum_in_order.argtypes = [vp, C.c_int64, P(C.c_double)]
+    L.of_min_sum_in_order.restype = C.c_int
     L.of_heston_price_adjoint.argtypes = [vp, P(A.OfHestonAdjointParams), P(A.OfAdjointResult)]
     L.of_heston_price_adjoint.restype = C.c_int
     L.of_mc_european_gpu.argtypes = [vp, C.c_double, C.c_double, C.c_double, C.c_double, C.c_double, C.c_int64,

@@ -7,11 +7,15 @@ and geometric_asian_discrete_fixed_closed_form (src/pricing/asian.rs:86-136).
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
+import os
+from array import array
 from typing import Sequence
 
 import numpy as np
 
+from . import _lib
 from .core import OptionType
 
 _INV_SQRT_2PI = 0.3989422804014327
@@ -97,12 +101,29 @@ def bs_greeks(option_type: OptionType, spot: float, strike: float, rate: float, 
     return dict(delta=delta, gamma=gamma, vega=vega, theta=theta, rho=rho)
 
 
+def fixing_array(times) -> np.ndarray:
+    """Fixing times as a contiguous FP64 array.  array('d') reads a list of
+    floats in half the time of np.asarray (10 us against 18 at 640 fixings)."""
+    if isinstance(times, (list, tuple)) and times:
+        try:
+            return np.frombuffer(array("d", times), dtype=np.float64)
+        except TypeError:  # not plain numbers: numpy's own conversion, or its error
+            pass
+    return np.ascontiguousarray(times, dtype=np.float64)
+
+
 def min_sum_in_order(times: Sequence[float], rows_per_block: int = 256) -> float:
     """sum_i sum_j min(t_i, t_j) added in the reference's order (i outer, j
     inner, one FP64 add at a time: src/pricing/asian.rs:86-136), so the
-    result is bit-identical to its double loop.  np.cumsum adds strictly left
-    to right; blocks of rows bound the temporary to rows_per_block x n."""
-    t = np.asarray(times, dtype=np.float64)
+    result is bit-identical to its double loop.  The library's host code takes
+    whole rows at a time (of_min_sum_in_order: 22 us at 252 fixings, 300 for
+    the cumsum below); without the library, np.cumsum adds strictly left to
+    right, in blocks of rows that bound the temporary to rows_per_block x n."""
+    t = fixing_array(times)
+    if t.ndim == 1 and os.path.exists(_lib.LIB_PATH):
+        out = C.c_double()
+        _lib.raise_for(_lib.load().of_min_sum_in_order(t.ctypes.data, t.size, C.byref(out)))
+        return out.value
     total = 0.0
     for a in range(0, t.size, rows_per_block):
         block = np.minimum.outer(t[a:a + rows_per_block], t).ravel()
@@ -146,6 +167,6 @@ def geometric_asian_cov_sum_sorted(observation_times: Sequence[float]) -> float:
     is the minimum of 2(n - i) - 1 ordered pairs, so the sum is one dot
     product (within about 1e-15 relative of the exact sum), used for long
     fixing schedules."""
-    ts = np.sort(np.asarray(observation_times, dtype=np.float64))
+    ts = np.sort(fixing_array(observation_times))
     n = ts.size
     return float(np.dot(ts, (2 * (n - np.arange(n)) - 1).astype(np.float64)))

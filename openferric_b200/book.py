@@ -46,11 +46,12 @@ def book_entries_abi(entries: Sequence[BookEntry]):
     keep, vols = [], []
     for k, e in enumerate(entries):
         inst, m = e.instrument, e.market
-        inst.validate()
+        # an Asian's fixings are converted once, by its validation
+        times = inst._validated_times() if type(inst) is AsianOption else inst.validate()
         vol = m.vol_for(max(reference_strike(inst, m.spot), 1e-12), inst.expiry)
         gen = GbmPathGenerator(Gbm(m.rate - m.dividend_yield, vol), m.spot, inst.expiry, e.num_steps,
                                m.dividend_schedule if m.has_discrete_dividends() else None)
-        payoff, held = _payoff_abi(inst)
+        payoff, held = _payoff_abi(inst, times)
         keep.append(held)
         keep.append(gen)  # holds the dividend array the model points to
         vols.append(vol)

@@ -21,7 +21,7 @@ import numpy as np
 
 from . import _abi as A
 from ._lib import context
-from .analytic import bs_price, geometric_asian_discrete_fixed
+from .analytic import bs_price, fixing_array, geometric_asian_discrete_fixed
 from .core import (Averaging, BarrierDirection, BarrierStyle, Diagnostics, OptionType, PricingError,
                    PricingResult, StrikeType)
 from .instruments import AsianOption, BarrierOption, VanillaOption
@@ -154,7 +154,8 @@ class ControlVariate:
 # ---------------------------------------------------------------------------
 # Payoff descriptors (MonteCarloInstrument, mc_engine.rs:44-584)
 # ---------------------------------------------------------------------------
-def _payoff_abi(instrument) -> Tuple[A.OfPayoff, Optional[np.ndarray]]:
+def _payoff_abi(instrument, times: Optional[np.ndarray] = None) -> Tuple[A.OfPayoff, Optional[np.ndarray]]:
+    """times: an Asian's fixing times, where the caller has converted them."""
     p = A.OfPayoff()
     p.option_type = instrument.option_type.value
     p.strike = float(instrument.strike)
@@ -174,7 +175,7 @@ def _payoff_abi(instrument) -> Tuple[A.OfPayoff, Optional[np.ndarray]]:
         s = instrument.asian
         p.averaging = A.OF_AVG_ARITHMETIC if s.averaging is Averaging.Arithmetic else A.OF_AVG_GEOMETRIC
         p.strike_type = A.OF_STRIKE_FIXED if s.strike_type is StrikeType.Fixed else A.OF_STRIKE_FLOATING
-        keep = np.ascontiguousarray(s.observation_times, dtype=np.float64)
+        keep = fixing_array(s.observation_times) if times is None else times
         p.observation_times = keep.ctypes.data_as(C.POINTER(C.c_double))
         p.n_observations = len(keep)
     else:

@@ -8,6 +8,7 @@ from typing import List, Sequence, Tuple
 
 import numpy as np
 
+from .analytic import fixing_array
 from .core import (AsianSpec, Averaging, BarrierDirection, BarrierSpec, BarrierStyle, ExerciseStyle, OptionType,
                    PricingError, StrikeType)
 
@@ -69,15 +70,20 @@ class AsianOption:
         return "AsianOption"
 
     def validate(self) -> None:
+        self._validated_times()
+
+    def _validated_times(self) -> np.ndarray:
+        """validate(), returning the fixing times it converted."""
         if self.expiry < 0.0:
             raise PricingError.InvalidInput("asian expiry must be >= 0")
         if self.strike <= 0.0:
             raise PricingError.InvalidInput("asian strike must be > 0")
         if not self.asian.observation_times:
             raise PricingError.InvalidInput("asian observation_times cannot be empty")
-        obs = np.asarray(self.asian.observation_times, dtype=np.float64)
+        obs = fixing_array(self.asian.observation_times)
         if np.any((obs < 0.0) | (obs > self.expiry)):  # asian.rs:55-64; NaN compares false there too
             raise PricingError.InvalidInput("asian observation_times must lie in [0, expiry]")
+        return obs
 
 
 @dataclass
