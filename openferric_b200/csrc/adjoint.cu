@@ -56,8 +56,8 @@ constexpr float kLn2 = 0.69314718055994531f;
 constexpr int kPathThreads = 128;
 // The sweep back runs where fewer than kSweepShare of at least kSweepPathsPerSm
 // paths an SM are expected in the money.  1,048,576 paths of 512 steps, Asian:
-// 3.90 ms for the tangent pass whatever the share; forward pass and sweep 4.2
-// at a share of 0.13, 3.5 at 0.07, 3.1 at 0.  One round of sweeps takes 0.75 ms
+// 3.82 ms for the tangent pass whatever the share; forward pass and sweep 4.1
+// at a share of 0.13, 3.4 at 0.07, 3.0 at 0.  One round of sweeps takes 0.75 ms
 // however few they are, which the tangent pass undercuts below 2^20 paths:
 // 32,768 paths take 0.22 ms against 2.06 at the money.
 constexpr double kSweepShare = 0.10;
@@ -69,6 +69,12 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   return r;
 }
 
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 __device__ __forceinline__ float rcp_approx(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -77,9 +83,8 @@ __device__ __forceinline__ float rcp_approx(float x) {
 
 struct AdjC {
   // step
-  float e, one_m_e, c1, c2, theta, c0 /* (r-q) dt + K0 */, K1, K2, K12 /* K1 + K2 */, k34, half_k34, dt;
-  float sw_lo, sw_inv_width;  // smoothed switch band [lo, hi] of psi
-  float t_lo, t_hi;           // 2 / hi and 2 / lo
+  float e, one_m_e, c1, c2, theta, c0 /* (r-q) dt + K0 */, K1, K2, k34, half_k34, dt;
+  float sw_lo, sw_hi, sw_inv_width;  // smoothed switch band [lo, hi] of psi
   // parameter partials of the step constants
   float de_dk, c1_k, c2_k, c2_t, m2_over_xi;
   float K0_k, K0_t, K0_x, K0_r, K1_k, K1_x, K1_r, K2_k, K2_x, K2_r, k34_r;
@@ -108,69 +113,69 @@ __device__ __forceinline__ QeDraw draw_of(uint32_t a, uint32_t b) {
   return QeDraw{of::uniform_from_u32(a), z.x, z.y};
 }
 
-// Both branches are functions of m and t alone.  JAC: A1 = dv'/dm at fixed t
-// and At = dv'/dt.  Roots come with their reciprocals, x rsqrt(x).
+// Both branches are functions of m and t = 2 / psi alone.  JAC: A1 = dv'/dm at
+// fixed t and At = dv'/dt.
 //
 // quadratic: dv'/db^2 = a bz/b - a bz^2/(1+b^2) = a bz (1 - b Zv) / (b (1+b^2)),
 // without the cancellation of the two terms; db^2/dt = 1 + (t - 1/2)/root.
 template <bool JAC>
 __device__ __forceinline__ float quad_branch(float m, float t, float zv, float& A1, float& At) {
   const float tm = t - 1.0f, x = t * tm;
-  const float rs = rsqrt_approx(x), root = x * rs;
+  const float rs = rsqrt_approx(x), root = sqrt_approx(x);
   const float b2 = tm + root;
-  const float rb = rsqrt_approx(b2), b = b2 * rb;
-  const float d = fmaf(b, b, 1.0f), i0 = rcp_approx(d), inv = fmaf(i0, fmaf(-d, i0, 1.0f), i0);
-  const float a = m * inv, bz = b + zv, da = bz * bz;
+  const float rb = rsqrt_approx(b2), b = sqrt_approx(b2);
+  const float inv = rcp_approx(1.0f + b2);
+  const float a = m * inv, bz = b + zv;
   if (JAC) {
-    A1 = da * inv;
-    At = a * inv * (rb * bz) * fmaf(-b, zv, 1.0f) * fmaf(t - 0.5f, rs, 1.0f);
+    // 1 / (1 + b^2) of the b in use, refined once: E[(b + Zv)^2] / (1 + b^2)
+    // is 1 to a rounding, and an error of one sign would build up over the
+    // steps that the variance remembers (1e-5 of a Greek)
+    const float g = fmaf(inv, fmaf(-fmaf(b, b, 1.0f), inv, 1.0f), inv);
+    A1 = bz * bz * g;
+    At = a * g * (rb * bz) * fmaf(-b, zv, 1.0f) * fmaf(t - 0.5f, rs, 1.0f);
   }
-  return a * da;
+  return a * bz * bz;
 }
 
-// exponential, with (1-p)/(1-U) = 2t / ((2+t)(1-U)) and 1/(1-p) = 1/t + 1/2:
-// v' = m L (1/t + 1/2), dv'/dt = m (1 - L) / t^2
+// exponential: with 1/(1-p) = 1/t + 1/2, v' = m L (1/t + 1/2) and
+// dv'/dt = m (1 - L) / t^2, 1/t = psi / 2
 template <bool JAC>
-__device__ __forceinline__ float exp_branch(float m, float t, float u, float it, float& A1, float& At) {
-  const float tp = 2.0f + t;
-  float ve = 0.0f;
+__device__ __forceinline__ float exp_branch(float m, float psi, float u, float& A1, float& At) {
+  const float p = __fdividef(psi - 1.0f, psi + 1.0f);
   if (JAC) A1 = At = 0.0f;
-  if (u * tp > 2.0f - t) {  // U > p
-    const float L = fmaxf(__log2f((t + t) * rcp_approx(tp * (1.0f - u))) * kLn2, 0.0f);
-    const float k = it + 0.5f;
-    ve = m * L * k;
-    if (JAC) {
-      A1 = L * k;
-      At = m * (1.0f - L) * (it * it);
-    }
+  if (u <= p) return 0.0f;
+  const float L = (__log2f(1.0f - p) - __log2f(1.0f - u)) * kLn2;
+  if (JAC) {
+    const float it = 0.5f * psi;
+    A1 = L * (it + 0.5f);
+    At = m * (1.0f - L) * (it * it);
   }
-  return ve;
+  return __fdividef(m * L, 1.0f - p);
 }
 
 // The variance step with the (optional) smoothed switch.  JAC: the partial of
-// v' by m, and P and r = 1/s2 of that by s2, -P r (dt/dm = 4 m / s2,
+// v' by m, and P and r = 1/s2 of that by s2, -P r (dt/dm = 2 t / m,
 // dt/ds2 = -t / s2).
 template <bool JAC>
 __device__ __forceinline__ float qe_vnext(const AdjC& c, float v, const QeDraw& d, float& Bm, float& P, float& r) {
-  const float m = fmaf(c.theta - v, c.one_m_e, v);
+  const float m = fmaf(v - c.theta, c.e, c.theta);
   const float s2 = fmaf(v, c.c1, c.c2);
-  r = rcp_approx(s2);
-  const float q = m * r;
-  const float t = (m + m) * q;
+  const float inv_m = rcp_approx(m);
+  const float psi = s2 * inv_m * inv_m;
+  const float t = __fdividef(2.0f, psi);
   // each branch inlined once: quadratic below the band's top, exponential
   // above its bottom, blended inside the band
-  const bool need_q = t >= c.t_lo, need_e = t < c.t_hi;
+  const bool need_q = psi <= c.sw_hi, need_e = psi > c.sw_lo;
   float vn = 0.0f, A1 = 0.0f, At = 0.0f;
   if (need_q) vn = quad_branch<JAC>(m, t, d.zv, A1, At);
   if (need_e) {
-    const float it = rcp_approx(t);
     float e1 = 0.0f, et = 0.0f;
-    const float ve = exp_branch<JAC>(m, t, d.u, it, e1, et);
+    const float ve = exp_branch<JAC>(m, psi, d.u, e1, et);
     if (need_q) {
-      const float s = fmaf(2.0f, it, -c.sw_lo) * c.sw_inv_width;
+      const float s = (psi - c.sw_lo) * c.sw_inv_width;
       const float w = s * s * fmaf(-2.0f, s, 3.0f);
-      if (JAC) {  // dw/dt = dw/dpsi dpsi/dt, dpsi/dt = -2 / t^2
-        const float dw = -12.0f * s * (1.0f - s) * c.sw_inv_width * (it * it);
+      if (JAC) {  // dw/dt = dw/dpsi dpsi/dt, dpsi/dt = -psi^2 / 2
+        const float dw = -3.0f * s * (1.0f - s) * c.sw_inv_width * (psi * psi);
         A1 = fmaf(w, e1 - A1, A1);
         At = fmaf(ve - vn, dw, fmaf(w, et - At, At));
       }
@@ -182,8 +187,9 @@ __device__ __forceinline__ float qe_vnext(const AdjC& c, float v, const QeDraw& 
     }
   }
   if (JAC) {
-    Bm = fmaf(At, 4.0f * q, A1);
     P = At * t;
+    Bm = fmaf(P, 2.0f * inv_m, A1);
+    r = 0.5f * t * inv_m * inv_m;
   }
   return vn;
 }
@@ -192,16 +198,11 @@ __device__ __forceinline__ float qe_vnext(const AdjC& c, float v, const QeDraw& 
 __device__ __forceinline__ float vol_of(const AdjC& c, float v, float vn, float& inv) {
   const float var = c.k34 * (v + vn);
   inv = var > 0.0f ? rsqrt_approx(var) : 0.0f;
-  return var * inv;
+  return sqrt_approx(var);
 }
 
-// Two roundings of one sign are kept out of the 512 steps' sum.  K1 v + K2 v'
-// is taken as (K1 + K2) v + K2 (v' - v): K1 and K2 are -rho/xi and rho/xi to a
-// small rest, and the difference of their FP32 roundings would drift y by
-// 1e-7 sum v.  And y is added last: y + c0 would round the same part of c0
-// away at every step (y's grid is fixed within a binade), 1e-6 in the mean of y.
 __device__ __forceinline__ float qe_ynext(const AdjC& c, float y, float v, float vn, float sq, float zx) {
-  return y + fmaf(sq, zx, fmaf(c.K2, vn - v, fmaf(c.K12, v, c.c0)));
+  return fmaf(sq, zx, fmaf(c.K2, vn, fmaf(c.K1, v, y + c.c0)));
 }
 
 // ---- the pass over the paths ---------------------------------------------------
@@ -227,18 +228,17 @@ struct Tangents {
                                        float inv, float zx) {
     using of::fma2;
     using of::splat2;
-    using of::sub2;
     const float vm = v - c.theta, Bs = -P * r;
     const float2 dvn_v = splat2(fmaf(Bm, c.e, Bs * c.c1));
     // direct parts; s2 is proportional to xi^2, so that of xi needs no s2
     const float2 direct[2] = {{0.0f, fmaf(Bm * c.de_dk, vm, Bs * fmaf(v, c.c1_k, c.c2_k))},
                               {fmaf(Bm, c.one_m_e, Bs * c.c2_t), c.m2_over_xi * P}};
     const float kh = c.half_k34 * (zx * inv);
-    const float2 D2 = splat2(c.K2 + kh), D12 = splat2(fmaf(2.0f, kh, c.K12));  // dy/dv' and dy/dv + dy/dv'
+    const float2 D1 = splat2(c.K1 + kh), D2 = splat2(c.K2 + kh);  // dy/dv and dy/dv'
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
       const float2 n = fma2(dvn_v, dv[p], direct[p]);
-      Y[p] = fma2(D2, sub2(n, dv[p]), fma2(D12, dv[p], Y[p]));
+      Y[p] = fma2(D2, n, fma2(D1, dv[p], Y[p]));
       dv[p] = n;
     }
     W = fmaf(sq, zx, W);
@@ -260,12 +260,12 @@ struct Tangents {
 // partial round spreads over all SMs.  16 sums (price 2, Greeks 7 + 7); without
 // Greeks 14 of them are 0, and the price is added in the same order.
 //
-// Issue-bound: 197 instructions a warp and step with the tangents (130 for the
-// price), 140 (75) of them on the FMA pipe, issued at 68 % of the peak; a step
-// has 8 special functions (32 issue cycles of their unit a warp are 64 of 250)
-// and half a Philox block from the table of its counter terms.  1,048,576
-// paths of 512 steps, Asian: price and Greeks 3.90 ms against 8.43 for the
-// forward pass and the sweep before it, price alone 2.68 against 2.84.
+// Issue-bound: about 200 instructions a warp and step with the tangents (130
+// for the price), 140 (75) of them on the FMA pipe, issued at 68 % of the peak;
+// a step has 12 (9) special functions, 8 cycles of their unit each, and half a
+// Philox block from the table of its counter terms.  1,048,576 paths of 512
+// steps, Asian: price and Greeks 3.82 ms against 8.43 for the forward pass and
+// the sweep before it, price alone 2.58 against 2.84.
 template <int PASS, bool ASIAN, bool FULL>
 __global__ void __launch_bounds__(kPathThreads, 5) adjoint_paths(const __grid_constant__ AdjC c,
                                                                  double* __restrict__ partials, unsigned* ticket,
@@ -635,20 +635,18 @@ extern "C" of_status of_heston_price_adjoint(of_ctx* ctx, const of_heston_adjoin
   } else {
     AdjC c{};
     c.e = (float)e;
-    c.one_m_e = (float)(1.0 - e);
+    c.one_m_e = 1.0f - c.e;  // of the e the path takes
     c.c1 = (float)c1;
     c.c2 = (float)c2;
     c.theta = (float)th;
     c.c0 = (float)((p->rate - p->dividend_yield) * dt + K0);
     c.K1 = (float)K1;
     c.K2 = (float)K2;
-    c.K12 = (float)(dt * (k * r / x - 0.5));
     c.k34 = (float)k34;
     c.half_k34 = (float)(0.5 * k34);
     c.dt = (float)dt;
     c.sw_lo = (float)sw_lo;
-    c.t_lo = (float)(2.0 / sw_hi);
-    c.t_hi = (float)(2.0 / sw_lo);
+    c.sw_hi = (float)sw_hi;
     c.sw_inv_width = (float)sw_inv_width;
     c.de_dk = (float)de_dk;
     c.c1_k = (float)(x * x * de_dk * (1.0 - 2.0 * e) / k - c1 / k);
@@ -685,11 +683,12 @@ extern "C" of_status of_heston_price_adjoint(of_ctx* ctx, const of_heston_adjoin
     c.paths = p->num_paths;
     c.keys = of::philox_keys(p->seed);
     const double* Ks[4] = {K_k, K_t, K_x, K_r};
-    const double sumV[4] = {dt * r / x, 0.0, -dt * k * r / (x * x), dt * k / x};  // K1_p + K2_p, the 1/x parts cancelled
+    // of the FP32 constants, as the path takes them
     for (int q = 0; q < 4; ++q) {
-      c.linV[q] = sumV[q];
-      c.linK[q] = Ks[q][2];
-      c.lin0[q] = Ks[q][0] + sumV[q] * p->v0;
+      const double k0 = (float)Ks[q][0], k1 = (float)Ks[q][1], k2 = (float)Ks[q][2];
+      c.linV[q] = k1 + k2;
+      c.linK[q] = k2;
+      c.lin0[q] = k0 + c.linV[q] * (double)c.v0;
     }
     c.rho_w = -r / (1.0 - r * r);
     const bool greeks = p->forward_only == 0;
