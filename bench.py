@@ -51,25 +51,25 @@ PATHS, STEPS, SEED = 1 << 20, 256, 7
 PATH_STEPS = float(PATHS) * STEPS
 # Declared algorithmic work of one Heston Euler path-step in the FP32 kernel:
 # one Box-Muller pair (u1 2, radius constant 1, angle fma 2, r cos / r sin 2:
-# 7 flops; lg2, sqrt, sin, cos on the MUFU unit; sqrt(dt) rides in the radius
+# 7 flops; lg2, sin, cos on the MUFU unit; sqrt(dt) rides in the radius
 # constant) and the step (correlation 3, log-spot 5, variance 5, floors 2: 15
-# flops; one sqrt): 22 FP32 flops (FMA = 2) and 5 MUFU operations.  The
-# Philox rounds (integer multiply and xor, ~20 instructions per step) use
-# neither pipe's budget in this count.
+# flops; one sqrt, of variance times squared radius): 22 FP32 flops (FMA = 2)
+# and 4 MUFU operations.  The Philox rounds (integer multiply and xor, ~18
+# instructions per step) use neither pipe's budget in this count.
 FLOPS_PER_STEP = 22.0
-SFU_PER_STEP = 5.0
+SFU_PER_STEP = 4.0
 # Issued thread instructions per path-step of the strip kernel, Philox
 # included, from ncu captures (smsp__inst_executed.sum x 32 / path-steps) of
 # the bench's kernel at 2^20 paths, by samples in flight per thread.  With the
 # sampled SM clock they give the issue fraction: warp instructions per second
 # over 148 SMs x 4 schedulers x 1 instruction per cycle.
-INSTR_PER_STEP = {1: 48.8, 2: 40.0}
-INSTR_SOURCE = ("ncu smsp__inst_executed.sum of strip_kernel at 2^20 paths (profiles/strip_kernel_heston_euler_ilp2_2p20.md "
-                "for two samples per thread, profiles/strip_kernel_pipe_mix_2p20.md for one)")
+INSTR_PER_STEP = {1: 48.1, 2: 37.8}
+INSTR_SOURCE = ("ncu smsp__inst_executed.sum of strip_kernel at 2^20 paths "
+                "(profiles/strip_kernel_heston_euler_ilp2_2p20.md)")
 # DRAM bytes (read + write) of one strip launch from an ncu capture of the
 # kernel; the kernel reads no input from HBM, so the figure does not grow
 # with the path count.
-STRIP_DRAM_BYTES = 30720
+STRIP_DRAM_BYTES = 39680
 STRIP_DRAM_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of strip_kernel<ILP=2> at 2^20 paths "
                      "(the kernel reads no HBM input; the figure does not grow with paths)")
 CONFIG = {"workload": "heston_euler_strike_strip", "paths": PATHS, "steps": STEPS, "strikes": 41,
@@ -248,7 +248,7 @@ ADJ_HESTON = dict(spot=100.0, rate=0.03, v0=0.04, kappa=2.0, theta=0.04, xi=0.5,
 def greeks_comparison(paths=PATHS, steps=512, reps=3):
     """Priced + full-Greeks options/s for one Heston arithmetic Asian call
     (K=100, T=2, daily fixings at all 512 steps, the parameters of the strip):
-    FP32 QE + checkpointed adjoint (one call) against the plain FP64 engine
+    FP32 QE + pathwise Greeks (one call) against the plain FP64 engine
     (the reference-stream Euler engine) with the 7 Greeks by central bumps
     with common random numbers (15 runs).  Both at the same path count; the
     standard error of both is below 1e-4 S0 = 0.01."""
@@ -402,7 +402,7 @@ def leg_config1(steps, warmup, peaks, threads):
                              "note": "declared flops: Acklam central region + log-Euler update per path-step; the "
                                      "FP64 exp/log/div routines are multi-instruction and not counted, so the pipe "
                                      "is busier than this fraction"},
-                "gpu_launches_per_step": 2}
+                "gpu_launches_per_step": 1}
     out["clocks"] = clocks.summary()
     out["workload"] = ("european_call_gbm_100k_x_252 (S0=100 K=100 r=0.05 q=0 sigma=0.2 T=1 seed 42; "
                        "benches/pricing_bench.rs:89-109)")
@@ -432,7 +432,7 @@ def leg_config1(steps, warmup, peaks, threads):
 # ---------------------------------------------------------------------------
 # Issued thread instructions per path-step of book_kernel on the synthetic
 # mixed book, from the ncu capture of 256 options (profiles/book_kernel_book256.md).
-BOOK_INSTR_PER_STEP = 19.0
+BOOK_INSTR_PER_STEP = 16.8
 BOOK_SEED = 20261203
 
 
@@ -906,9 +906,8 @@ def main():
                                                           tile_ilp_ms={str(k): v for k, v in tune_ms.items()}),
         "roofline": dict(main_line, bound=bound, traffic=STRIP_DRAM_BYTES, traffic_source=STRIP_DRAM_SOURCE,
                          issue=issue_line, **{other_name: other_line},
-                         # the workload's declared algorithmic count: a single-log inverse normal per
-                         # draw (2 lg2 per step) + sqrt + ex2 = 4 MUFU per path-step; Box-Muller issues
-                         # 5 (lg2, sqrt, sin, cos per pair of normals, sqrt of the variance)
+                         # 4 MUFU per path-step: lg2, sin, cos per pair of normals, sqrt of the variance
+                         # times the squared radius
                          frac_at_4_mufu_per_step=per_gpu * 4.0 / sfu_peak),
         "e2e": {"value": world * PATH_STEPS * args.steps / e2e_s, "unit": UNIT,
                 "h2d_bytes_per_step": 41 * 4, "d2h_bytes_per_step": 41 * 2 * 8},

@@ -260,8 +260,8 @@ struct Tangents {
 // partial round spreads over all SMs.  16 sums (price 2, Greeks 7 + 7); without
 // Greeks 14 of them are 0, and the price is added in the same order.
 //
-// Issue-bound: about 200 instructions a warp and step with the tangents (130
-// for the price), 140 (75) of them on the FMA pipe, issued at 68 % of the peak;
+// Issue-bound: 183 instructions a warp and step with the tangents (130 for the
+// price), two thirds of them on the FMA pipe, issued at 70 % of the peak;
 // a step has 12 (9) special functions, 8 cycles of their unit each, and half a
 // Philox block from the table of its counter terms.  1,048,576 paths of 512
 // steps, Asian: price and Greeks 3.82 ms against 8.43 for the forward pass and
