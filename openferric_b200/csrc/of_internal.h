@@ -19,14 +19,12 @@ enum OfSlot {
   SLOT_SUMS = 1,       // final FP64 sums
   SLOT_OBS = 2,        // per-step observation weights
   SLOT_INJECT = 3,     // injected normals (test hook)
-  SLOT_STRIKES = 4,    // strike strip
   SLOT_BOOK = 5,       // batched-book tables of a plan run inside one call
   SLOT_DIVIDENDS = 7,  // discrete dividend triggers
   SLOT_LSM_PATHS = 8,  // LSM path store (time-major)
   SLOT_LSM_VALUES = 9, // LSM cash flows
   SLOT_LSM_AUX = 10,   // LSM betas / counters
   SLOT_ADJ_CKPT = 11,  // adjoint checkpoints
-  SLOT_ADJ_AUX = 12,
   SLOT_TICKET = 13,    // last-block-done counter of grid_sum, zero between launches
   SLOT_MISC = 14,
   SLOT_JUMP = 15,      // xoshiro256++ GF(2) jump tables
