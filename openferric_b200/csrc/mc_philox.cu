@@ -45,9 +45,7 @@ StepConsts make_consts(const of_model* m) {
   c.kdt_theta = (float)(m->kappa * m->theta * dt);
   c.one_m_kdt = (float)(1.0 - m->kappa * dt);
   c.xi = (float)m->xi;
-  // the radius constant of polar_from_u32: Heston's normals come scaled by
-  // sqrt(dt), GBM's by sigma sqrt(dt)
-  c.bm_k2 = (float)(-2.0 * 0.69314718055994531 * (m->kind == OF_MODEL_GBM ? m->sigma * m->sigma * dt : dt));
+  c.bm_k2 = (float)(-2.0 * 0.69314718055994531 * dt);
   c.rho = (float)m->rho;
   c.rho_c = (float)std::sqrt(1.0 - m->rho * m->rho);
   c.v0 = (float)m->v0;
@@ -972,25 +970,23 @@ __device__ __forceinline__ void book_sample(const BookOpt& o, uint64_t i, GEN G,
   for (int32_t j = 0; j < o.steps; j += SPC) {
     const uint4 r = G.block((uint32_t)(j / SPC), L);
     const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
-    // polar normals of the two draw pairs (GBM and Heston Euler); for GBM .q
-    // becomes the radius sigma sqrt(dt) r, so that a step is one add and one fma
+    // Box-Muller normals of the two draw pairs (GBM), their polar form (Heston Euler)
+    float2 p01 = make_float2(0.0f, 0.0f), p23 = make_float2(0.0f, 0.0f);
     of::Polar h01{}, h23{};
-    if (MODEL != OF_MODEL_HESTON_QE) {
+    if (MODEL == OF_MODEL_GBM) {
+      p01 = of::normal_pair_from_u32(r.x, r.y);
+      p23 = of::normal_pair_from_u32(r.z, r.w);
+    } else if (MODEL == OF_MODEL_HESTON_EULER) {
       h01 = of::polar_from_u32(r.x, r.y, c.bm_k2);
       h23 = of::polar_from_u32(r.z, r.w, c.bm_k2);
-    }
-    if (MODEL == OF_MODEL_GBM) {
-      h01.q = sqrtf(h01.q);
-      h23.q = sqrtf(h23.q);
     }
 #pragma unroll
     for (int q = 0; q < SPC; ++q) {
       if (j + q >= o.steps) break;
       if (MODEL == OF_MODEL_GBM) {
-        const of::Polar& h = q < 2 ? h01 : h23;
-        const float z = (q & 1) ? h.s : h.c;
-        a.y = fmaf(h.q, z, a.y + c.drift);
-        if (anti) b.y = fmaf(-h.q, z, b.y + c.drift);
+        const float z = q == 0 ? p01.x : q == 1 ? p01.y : q == 2 ? p23.x : p23.y;
+        a.y = fmaf(c.diff, z, a.y + c.drift);
+        if (anti) b.y = fmaf(-c.diff, z, b.y + c.drift);
         for (; DIVS && ev < o.n_div && divs[o.div_offset + ev].step == j + q; ++ev) {  // mc_engine.rs:157-167
           const BookDiv d = divs[o.div_offset + ev];
           a.y = book_dividend(d, a.y);
@@ -1132,12 +1128,12 @@ __device__ __forceinline__ void book_sample_gbm(const BookOpt& o, uint64_t i, GE
   // sg y, sg drift, sg diff and sg b (sg = +1 up, -1 down; exact), one
   // comparison per step
   const float sg = KIND == BK_BARRIER && !(o.flags & BF_UP) ? -1.0f : 1.0f;
-  const float drift = sg * o.c.drift, sgb = sg * o.barrier_y, k2 = o.c.bm_k2;
+  const float drift = sg * o.c.drift, diff = sg * o.c.diff, sgb = sg * o.barrier_y;
   float ya = 0.0f;
   PathObs oa{0.0f, 0.0f, 0.0f, false};
   if (KIND == BK_BARRIER) oa.hit = 0.0f >= sgb;  // the scan includes path[0]
-  auto step = [&](float R, float z) {
-    ya = fmaf(R, z, ya + drift);
+  auto step = [&](float z) {
+    ya = fmaf(diff, z, ya + drift);
     if (KIND == BK_BARRIER) {
       oa.hit |= ya >= sgb;
     } else {  // Kahan sum of the daily fixings S/S0
@@ -1151,12 +1147,11 @@ __device__ __forceinline__ void book_sample_gbm(const BookOpt& o, uint64_t i, GE
   const of::PhiloxLane L = G.lane(i);
   for (int32_t j = 0; j < o.steps; j += 4) {
     const uint4 r = G.block((uint32_t)(j >> 2), L);
-    const of::Polar p = of::polar_from_u32(r.x, r.y, k2), q = of::polar_from_u32(r.z, r.w, k2);
-    const float Rp = sg * sqrtf(p.q), Rq = sg * sqrtf(q.q);
-    step(Rp, p.c);
-    if (j + 1 < o.steps) step(Rp, p.s);
-    if (j + 2 < o.steps) step(Rq, q.c);
-    if (j + 3 < o.steps) step(Rq, q.s);
+    const float2 p01 = of::normal_pair_from_u32(r.x, r.y), p23 = of::normal_pair_from_u32(r.z, r.w);
+    step(p01.x);
+    if (j + 1 < o.steps) step(p01.y);
+    if (j + 2 < o.steps) step(p23.x);
+    if (j + 3 < o.steps) step(p23.y);
   }
   book_payoff(o, oa, sg * ya, x, cvy);
 }
@@ -1176,14 +1171,15 @@ __device__ __forceinline__ void book_gbm_legs2(const BookOpt& o, uint64_t i0, ui
   using of::sub2;
   const float sg = KIND == BK_BARRIER && !(o.flags & BF_UP) ? -1.0f : 1.0f;
   const float2 drift = splat2(sg * o.c.drift);
-  const float sgb = sg * o.barrier_y, k2 = o.c.bm_k2;
+  const float2 diff = TWIN ? make_float2(sg * o.c.diff, -sg * o.c.diff) : splat2(sg * o.c.diff);
+  const float sgb = sg * o.barrier_y;
   y = make_float2(0.0f, 0.0f);
   float2 as = make_float2(0.0f, 0.0f), ac = make_float2(0.0f, 0.0f);  // Kahan sums of the daily fixings
   float2 ag = make_float2(0.0f, 0.0f);                                 // geometric sums
   bool ha = false, hb = false;
   if (KIND == BK_BARRIER) ha = hb = 0.0f >= sgb;  // the scan includes path[0]
-  auto step = [&](float2 R, float2 z) {
-    y = fma2(R, z, add2(y, drift));
+  auto step = [&](float2 z) {
+    y = fma2(diff, z, add2(y, drift));
     if (KIND == BK_BARRIER) {
       ha |= y.x >= sgb;
       hb |= y.y >= sgb;
@@ -1199,37 +1195,27 @@ __device__ __forceinline__ void book_gbm_legs2(const BookOpt& o, uint64_t i0, ui
   for (int32_t j = 0; j < o.steps; j += 4) {
     const uint4 qt = G.terms((uint32_t)(j >> 2));
     const uint4 r0 = of::philox_block(qt, L0, *G.K);
-    // steps j, j+1 take the radius Ra, steps j+2, j+3 Rb
-    float2 Ra, Rb, z1, z2, z3, z4;
-    if (TWIN) {
-      const of::Polar2 p = of::polars2_from_u32(r0.x, r0.y, r0.z, r0.w, k2);
-      const float ra = sg * sqrtf(p.q.x), rb = sg * sqrtf(p.q.y);
-      Ra = make_float2(ra, -ra);
-      Rb = make_float2(rb, -rb);
-      z1 = splat2(p.c.x);
-      z2 = splat2(p.s.x);
-      z3 = splat2(p.c.y);
-      z4 = splat2(p.s.y);
-    } else {
+    float2 w1, w2, w3, w4;
+    if (TWIN) {  // w1 = (z_j, z_j+2), w2 = (z_j+1, z_j+3)
+      of::normal_pairs_scaled2_from_u32(r0.x, r0.y, r0.z, r0.w, of::kBoxMullerK2, w1, w2);
+      w3 = splat2(w1.y);
+      w4 = splat2(w2.y);
+      w1 = splat2(w1.x);
+      w2 = splat2(w2.x);
+    } else {  // wk = step j+k-1 of (i0, i1)
       const uint4 r1 = of::philox_block(qt, L1, *G.K);
-      const of::Polar2 p = of::polars2_from_u32(r0.x, r0.y, r1.x, r1.y, k2),
-                       q = of::polars2_from_u32(r0.z, r0.w, r1.z, r1.w, k2);
-      Ra = make_float2(sg * sqrtf(p.q.x), sg * sqrtf(p.q.y));
-      Rb = make_float2(sg * sqrtf(q.q.x), sg * sqrtf(q.q.y));
-      z1 = p.c;
-      z2 = p.s;
-      z3 = q.c;
-      z4 = q.s;
+      of::normal_pairs_scaled2_from_u32(r0.x, r0.y, r1.x, r1.y, of::kBoxMullerK2, w1, w2);
+      of::normal_pairs_scaled2_from_u32(r0.z, r0.w, r1.z, r1.w, of::kBoxMullerK2, w3, w4);
     }
     if (j + 4 <= o.steps) {
-      step(Ra, z1);
-      step(Ra, z2);
-      step(Rb, z3);
-      step(Rb, z4);
+      step(w1);
+      step(w2);
+      step(w3);
+      step(w4);
     } else {
-      step(Ra, z1);
-      if (j + 1 < o.steps) step(Ra, z2);
-      if (j + 2 < o.steps) step(Rb, z3);
+      step(w1);
+      if (j + 1 < o.steps) step(w2);
+      if (j + 2 < o.steps) step(w3);
     }
   }
   if (KIND == BK_BARRIER) y = mul2(splat2(sg), y);
@@ -1302,8 +1288,8 @@ __device__ __forceinline__ void book_dispatch(const BookOpt& o, uint64_t i, cons
 // past the table, or past the tile's first high word, in place.  The loops run
 // at the integer-multiply rate (a wide multiply takes four issue cycles a warp
 // on sm_100); the table saves five of a counter block's twenty.  With the
-// radius folded into the path's fma and the packed sums of squares, 384 options
-// of 2^14..2^17 paths by 25..1260 daily steps took 10.58 ms (antithetic 6.36)
+// signed barrier path and the packed sums of squares, 384 options of
+// 2^14..2^17 paths by 25..1260 daily steps took 10.60 ms (antithetic 6.36)
 // against 11.58 (6.98); with the range test left in the loop, 11.2.
 constexpr uint32_t kBookTab = 2048;  // largest table (32 KB, three blocks an SM): 8,192 GBM steps
 
