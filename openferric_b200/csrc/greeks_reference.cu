@@ -116,23 +116,23 @@ __global__ void __launch_bounds__(kGreekThreads) heston_delta_kernel(const __gri
   const int lane = threadIdx.x & 31;
   double acc[2] = {0, 0};
   const int64_t stride = (int64_t)gridDim.x * kGreekThreads;
-  constexpr double kVFloor = 1e-290;  // in place of 0, for the square root
   const double mudt = P.mu * P.dt, hdt = 0.5 * P.dt, omk = 1.0 - P.kappa * P.dt, kth = P.kappa * P.theta * P.dt;
   const double xsd = P.xi * P.sqrt_dt, r1 = P.rho * P.sqrt_dt, r2 = P.rho2 * P.sqrt_dt;
   for (int64_t first = (int64_t)blockIdx.x * kGreekThreads; first < P.samples; first += stride) {
     const int64_t i = first + threadIdx.x;
     of::Xoshiro256pp rng;
     rng.seed(P.seed + (uint64_t)i * 7919ULL);
-    double y = 0.0, v = fmax(P.v0, kVFloor);
+    double y = 0.0, v = P.v0;
     for (int64_t left = P.steps; left > 0; left -= of::kDrawBatch / 2) {
       of::stream_normals(rng, buf, lane);
       const int n = left < of::kDrawBatch / 2 ? (int)left : of::kDrawBatch / 2;
 #pragma unroll 2
       for (int k = 0; k < n; ++k) {
         const double z1 = buf.z[2 * k * 32 + lane], z2 = buf.z[(2 * k + 1) * 32 + lane];
-        const double sq = of::sqrt64(v);
+        const double sq = of::sqrt64_from0(v);
         y = fma(sq, fma(r1, z1, r2 * z2), fma(-hdt, v, y + mudt));
-        v = fmax(fma(sq, xsd * z1, fma(omk, v, kth)), kVFloor);
+        const double v_next = fma(sq, xsd * z1, fma(omk, v, kth));
+        v = v_next > 0.0 ? v_next : 0.0;
       }
       __syncwarp();
     }

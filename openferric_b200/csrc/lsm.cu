@@ -460,7 +460,6 @@ __global__ void __launch_bounds__(kGenThreads) lsm_gen_stream(const __grid_const
   const LsmStep* st = B.st + (size_t)c * (B.steps + 1);
   double* S = (double*)B.S + (size_t)c * B.steps * B.npad;
   constexpr int kDraws = DYN == DYN_HESTON ? 2 : 1;
-  constexpr double kVFloor = 1e-290;  // in place of 0, for the square root (its terms vanish in every sum)
   const double drift = C.drift, vol = C.step_vol, spot = C.spot, y_floor = C.y_floor;
   const double mudt = C.mu * C.dt, hdt = 0.5 * C.dt, omk = 1.0 - C.kappa * C.dt, kth = C.kappa * C.theta * C.dt;
   const double xsd = C.xi * C.sqrt_dt, r1 = C.rho * C.sqrt_dt, r2 = sqrt(1.0 - C.rho * C.rho) * C.sqrt_dt;
@@ -468,7 +467,7 @@ __global__ void __launch_bounds__(kGenThreads) lsm_gen_stream(const __grid_const
   for (int q = 0; q < m; ++q) {
     const bool in = p0 + q < B.n;
     double* out = S + p0 + q;
-    double y = 0.0, var = fmax(C.v0, kVFloor), s = spot;
+    double y = 0.0, var = C.v0, s = spot;
     for (int t = 0; t < B.steps;) {
       if (at == of::kDrawBatch) {
         __syncwarp();
@@ -490,9 +489,10 @@ __global__ void __launch_bounds__(kGenThreads) lsm_gen_stream(const __grid_const
           y = fmax(y + fma(sigma * C.sqrt_dt, z, fma(-hdt * sigma, sigma, mudt)), y_floor);
         } else {
           // Heston::step_euler (src/models/stochastic.rs:56-71), :259-275
-          const double zs = fma(r1, z, r2 * zb[32]), sq = of::sqrt64(var);
+          const double zs = fma(r1, z, r2 * zb[32]), sq = of::sqrt64_from0(var);
           y = fmin(fmax(fma(sq, zs, fma(-hdt, var, y + mudt)), y_floor), 680.0);
-          var = fmax(fma(sq, xsd * z, fma(omk, var, kth)), kVFloor);
+          const double v_next = fma(sq, xsd * z, fma(omk, var, kth));
+          var = v_next > 0.0 ? v_next : 0.0;
         }
         s = spot * of::exp64(y, tab);
         if (in) *out = s;

@@ -316,21 +316,19 @@ __global__ void __launch_bounds__(kRefThreads) mc_ref_heston(const __grid_consta
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   const int64_t stride = (int64_t)gridDim.x * kRefThreads;
   const int32_t steps = (int32_t)P.steps;
-  // the variance is floored at a positive 1e-290 for the square root's sake:
-  // its terms are lost in every sum, as those of 0 are
-  constexpr double kVFloor = 1e-290;
   const double mudt = P.mu * P.dt, hdt = 0.5 * P.dt, omk = 1.0 - P.kappa * P.dt, kth = P.kappa * P.theta * P.dt;
   const double xsd = P.xi * P.sqrt_dt, r1 = P.rho * P.sqrt_dt, r2 = P.rho_c * P.sqrt_dt;
   auto step = [&](double& y, double& v, double z1, double zs) {
-    const double sq = of::sqrt64(v);
-    y = fmax(fma(sq, zs, fma(-hdt, v, y + mudt)), P.y_floor);
-    v = fmax(fma(sq, xsd * z1, fma(omk, v, kth)), kVFloor);
+    const double sq = of::sqrt64_from0(v);
+    const double y_next = fma(sq, zs, fma(-hdt, v, y + mudt)), v_next = fma(sq, xsd * z1, fma(omk, v, kth));
+    y = y_next > P.y_floor ? y_next : P.y_floor;
+    v = v_next > 0.0 ? v_next : 0.0;
   };
   for (int64_t first = (int64_t)blockIdx.x * kRefThreads; first < P.samples; first += stride) {
     const int64_t i = first + threadIdx.x;
     RNG rng;
     rng.seed(P.seed + (uint64_t)i * 7919ULL);
-    double ya = 0.0, yb = 0.0, va = fmax(P.v0, kVFloor), vb = va;
+    double ya = 0.0, yb = 0.0, va = P.v0, vb = va;
     for (int32_t j0 = 0; j0 < steps; j0 += of::kDrawBatch / 2) {
       of::stream_normals(rng, buf, lane);
       const int n = steps - j0 < of::kDrawBatch / 2 ? steps - j0 : of::kDrawBatch / 2;

@@ -40,6 +40,21 @@ __device__ __forceinline__ double sqrt64(double x) {
   return fma(s * e, fma(e, 0.375, 0.5), s);
 }
 
+// sqrt64 for any x >= 0: y is taken of at least the smallest normal number (one
+// integer maximum, of the high words), so that it stays finite and 0 gives
+// s = 0 y = 0.  The Heston steps need it: a variance that has reached 0 stays
+// there under kappa theta = 0, and a positive stand-in for 0 would grow back,
+// for each positive normal takes its root (1e-290, 1e-146, 1e-74, ...).
+__device__ __forceinline__ double sqrt64_from0(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;"
+      : "=d"(y)
+      : "d"(__hiloint2double(max(__double2hiint(x), 0x00100000), __double2loint(x))));
+  const double s = x * y;
+  const double e = fma(-s, y, 1.0);
+  return fma(s * e, fma(e, 0.375, 0.5), s);
+}
+
 // exp(x) for |x| < 690 by table lookup (P. T. P. Tang, "Table-driven
 // implementation of the exponential function in IEEE floating-point
 // arithmetic", ACM TOMS 15, 1989): x = (64 m + j) ln2/64 + r, |r| <= ln2/128,
