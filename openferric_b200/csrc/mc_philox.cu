@@ -740,7 +740,6 @@ extern "C" of_status of_strip_plan_create(of_ctx* ctx, const of_model* m, int32_
   };
   if (cudaMalloc(&pl->d_partials, (size_t)pl->grid * 2 * n_strikes * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&pl->d_sums, (2 * n_strikes + 2) * sizeof(double)) != cudaSuccess ||
-      cudaMemset(pl->d_sums, 0, (2 * n_strikes + 2) * sizeof(double)) != cudaSuccess ||
       cudaMallocHost(&pl->h_sums, (2 * n_strikes + 1) * sizeof(double)) != cudaSuccess)
     return fail(of_fail(ctx, OF_ERR_ALLOC, "strip plan allocation failed"));
   pl->P.status = (uint32_t*)(pl->d_sums + 2 * n_strikes);
@@ -749,10 +748,14 @@ extern "C" of_status of_strip_plan_create(of_ctx* ctx, const of_model* m, int32_
     pl->P.out = pl->h_sums;
   }
   // Capture kernel + reduction + readback once; launches replay the graph.
+  // The first launch finds the ticket zeroed: the memset has finished here,
+  // whatever the legacy stream holds and whichever stream replays the graph.
   cudaStream_t cap_stream = nullptr;
   if (cudaStreamCreateWithFlags(&cap_stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(of_fail(ctx, OF_ERR_CUDA, "capture stream creation failed"));
-  cudaError_t e = cudaStreamBeginCapture(cap_stream, cudaStreamCaptureModeThreadLocal);
+  cudaError_t e = cudaMemsetAsync(pl->d_sums, 0, (2 * n_strikes + 2) * sizeof(double), cap_stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cap_stream);
+  if (e == cudaSuccess) e = cudaStreamBeginCapture(cap_stream, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     strip_enqueue(pl, cap_stream);
     e = cudaStreamEndCapture(cap_stream, &pl->graph);
