@@ -1944,8 +1944,18 @@ static of_status book_plan_create(of_ctx* ctx, const of_book_entry* e, int64_t n
     for (int64_t k = 0; k < r.tiles; ++k)
       *tile++ = {r.opt, r.count, r.first + k * tile_samples, (int32_t)(r.slot + k), 0};
   // (from pageable memory the call returns once the bytes have left it)
-  if (cudaMemcpyAsync(pl->d_image, image, bytes, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
-    return fail(of_fail(ctx, OF_ERR_CUDA, "book upload failed"));
+  cudaStream_t up = ctx->stream;
+  // A plan of its own is uploaded when it is returned, on a stream that no
+  // caller captures: in a capture of the context's stream the copy would
+  // become a node of the caller's graph that reads `heap` long after it is gone.
+  if (!pl->scratch && cudaStreamCreateWithFlags(&up, cudaStreamNonBlocking) != cudaSuccess)
+    return fail(of_fail(ctx, OF_ERR_CUDA, "upload stream creation failed"));
+  cudaError_t up_err = cudaMemcpyAsync(pl->d_image, image, bytes, cudaMemcpyHostToDevice, up);
+  if (!pl->scratch) {
+    if (up_err == cudaSuccess) up_err = cudaStreamSynchronize(up);
+    cudaStreamDestroy(up);
+  }
+  if (up_err != cudaSuccess) return fail(of_fail(ctx, OF_ERR_CUDA, "book upload failed"));
   pl->d_opts = (BookOpt*)(pl->d_image + at_opts);
   pl->d_tiles = (BookTile*)(pl->d_image + at_tiles);
   pl->d_obs = (float*)(pl->d_image + at_obs);
