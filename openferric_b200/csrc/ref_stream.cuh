@@ -221,6 +221,10 @@ __device__ __forceinline__ double tail_normal(double q) {
 // ---------------------------------------------------------------------------
 constexpr int kTailCap = 24;
 
+// Whole groups of four draws: 64 bits, since the pathwise Greeks take any
+// positive step count.
+__host__ __device__ constexpr int64_t draw_groups(int64_t steps) { return steps >> 2; }
+
 template <typename RNG>
 __device__ __forceinline__ double stream_normal_sum(RNG& rng, int64_t steps, double* list, int stride) {
   double sum = 0.0;
@@ -244,7 +248,7 @@ __device__ __forceinline__ double stream_normal_sum(RNG& rng, int64_t steps, dou
   uint64_t r[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) r[k] = rng.next_u64();
-  for (uint32_t g = (uint32_t)(steps >> 2); g; --g) {
+  for (int64_t g = draw_groups(steps); g; --g) {
     double n[4], d[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
