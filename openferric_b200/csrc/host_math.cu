@@ -2,6 +2,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <new>
+#include <stdexcept>
 #include <vector>
 
 #include "of_gpu.h"
@@ -19,8 +21,7 @@
 // rest times k(t_i).  Rows that leave the binade, binades with a tie and
 // fixings that are not finite and non-negative are added one by one.  Daily
 // fixings tie only in the low binades, the first eighth of the rows: 17 us.
-extern "C" of_status of_min_sum_in_order(const double* times, int64_t n, double* out) {
-  if (!out || n < 0 || (n > 0 && !times)) return OF_ERR_INVALID_INPUT;
+static double min_sum_in_order(const double* times, int64_t n) {
   double s = 0.0;
   std::vector<double> sorted(times, times + n);
   bool plain = false;
@@ -67,6 +68,18 @@ extern "C" of_status of_min_sum_in_order(const double* times, int64_t n, double*
     const double ti = times[i];
     for (int64_t j = 0; j < n; ++j) s += times[j] < ti ? times[j] : ti;
   }
-  *out = s;
+  return s;
+}
+
+// No exception leaves the C entry: its tables (5 n words) are what can fail.
+extern "C" of_status of_min_sum_in_order(const double* times, int64_t n, double* out) {
+  if (!out || n < 0 || (n > 0 && !times)) return OF_ERR_INVALID_INPUT;
+  try {
+    *out = min_sum_in_order(times, n);
+  } catch (const std::bad_alloc&) {
+    return OF_ERR_ALLOC;
+  } catch (const std::length_error&) {
+    return OF_ERR_ALLOC;
+  }
   return OF_OK;
 }
