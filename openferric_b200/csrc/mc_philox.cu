@@ -66,6 +66,31 @@ StepConsts make_consts(const of_model* m) {
   return c;
 }
 
+// A GBM sample's sum of normals grows by a counter block's four at a time, two
+// Box-Muller pair sums in one product and one fma, and by the last, partial
+// block's `rem`.  Every rounding is written out, for the compiler contracts
+// packed and scalar products with the sum that follows differently: the same
+// bits in every strip shape, one sample (gbm_add_block) or two in packed pairs
+// (gbm_add_block2).
+__device__ __forceinline__ float gbm_add_block(float w, const uint4 r) {
+  float2 q, s;
+  of::normal_pair_sum_factors2_from_u32(r.x, r.y, r.z, r.w, q, s);
+  return __fadd_rn(w, fmaf(q.y, s.y, __fmul_rn(q.x, s.x)));
+}
+
+__device__ __forceinline__ float2 gbm_add_block2(float2 w, const uint4 r0, const uint4 r1) {
+  float2 q01, s01, q23, s23;
+  of::normal_pair_sum_factors2_from_u32(r0.x, r0.y, r1.x, r1.y, q01, s01);
+  of::normal_pair_sum_factors2_from_u32(r0.z, r0.w, r1.z, r1.w, q23, s23);
+  return of::add2(w, of::fma2(q23, s23, of::mul2(q01, s01)));
+}
+
+__device__ __forceinline__ float gbm_add_last(float w, const uint4 r, int32_t rem) {
+  if (rem == 1) return __fadd_rn(w, of::normal_pair_from_u32(r.x, r.y).x);
+  w = __fadd_rn(w, of::normal_pair_sum_from_u32(r.x, r.y));
+  return rem == 3 ? __fadd_rn(w, of::normal_pair_from_u32(r.z, r.w).x) : w;
+}
+
 // Simulates the terminal log-returns of ILP samples (and of their antithetic
 // twins) in one loop: the Philox rounds of the samples are separate dependency
 // chains, so their instructions interleave and fill the gaps of one chain, and
@@ -81,38 +106,25 @@ __device__ __forceinline__ void simulate_terminal(const StepConsts& c, int32_t s
   if constexpr (MODEL == OF_MODEL_GBM) {
     // y_T = steps drift + diff sum z; each Box-Muller pair enters as its sum
     // (normal_pair_sum_from_u32), four steps a counter block
-    float2 w = make_float2(0.0f, 0.0f);  // ILP 1: the sums of the block's two pairs; ILP 2: of the two samples
-    const int32_t full = steps >> 2;
-    for (int32_t q = 0; q < full; ++q) {
-      const uint4 t = of::philox_terms<FULL>(T, (uint32_t)q, K);
-      const uint4 r = of::philox_block(t, L[0], K);
-      if constexpr (ILP == 1) {
-        w = of::add2(w, of::normal_pair_sums2_from_u32(r.x, r.y, r.z, r.w));
-      } else {
-        const uint4 r1 = of::philox_block(t, L[1], K);
-        w = of::add2(w, of::add2(of::normal_pair_sums2_from_u32(r.x, r.y, r1.x, r1.y),
-                                 of::normal_pair_sums2_from_u32(r.z, r.w, r1.z, r1.w)));
-      }
-    }
     float sum[ILP];
+    const int32_t full = steps >> 2;
     if constexpr (ILP == 1) {
-      sum[0] = w.x + w.y;
+      sum[0] = 0.0f;
+      for (int32_t q = 0; q < full; ++q)
+        sum[0] = gbm_add_block(sum[0], of::philox_block(of::philox_terms<FULL>(T, (uint32_t)q, K), L[0], K));
     } else {
+      float2 w = make_float2(0.0f, 0.0f);
+      for (int32_t q = 0; q < full; ++q) {
+        const uint4 t = of::philox_terms<FULL>(T, (uint32_t)q, K);
+        w = gbm_add_block2(w, of::philox_block(t, L[0], K), of::philox_block(t, L[1], K));
+      }
       sum[0] = w.x;
       sum[1] = w.y;
     }
     if (const int32_t rem = steps & 3) {
       const uint4 t = of::philox_terms<FULL>(T, (uint32_t)full, K);
 #pragma unroll
-      for (int l = 0; l < ILP; ++l) {
-        const uint4 r = of::philox_block(t, L[l], K);
-        if (rem == 1) {
-          sum[l] += of::normal_pair_from_u32(r.x, r.y).x;
-        } else {
-          sum[l] += of::normal_pair_sum_from_u32(r.x, r.y);
-          if (rem == 3) sum[l] += of::normal_pair_from_u32(r.z, r.w).x;
-        }
-      }
+      for (int l = 0; l < ILP; ++l) sum[l] = gbm_add_last(sum[l], of::philox_block(t, L[l], K), rem);
     }
     const float base = (float)steps * c.drift;
 #pragma unroll
@@ -300,9 +312,9 @@ __global__ void __launch_bounds__(kStripThreads, 4) strip_kernel(const __grid_co
       else simulate_terminal<MODEL, ANTI, ILP, false>(P.c, P.steps, L, T, P.keys, ya, yb);
     }
 #pragma unroll
-    for (int l = 0; l < ILP; ++l) {
-      sa[l] = P.s0 * __expf(ya[l]);
-      sb[l] = P.s0 * __expf(yb[l]);
+    for (int l = 0; l < ILP; ++l) {  // rounded before a strike is taken off, with one strike as with several
+      sa[l] = __fmul_rn(P.s0, __expf(ya[l]));
+      sb[l] = __fmul_rn(P.s0, __expf(yb[l]));
     }
 #pragma unroll
     for (int l = 0; l < ILP; ++l) {
@@ -390,12 +402,8 @@ template <int MODEL, bool ANTI>
 __device__ __forceinline__ void ws_consume(const StepConsts& c, const uint4 r, int32_t q, int32_t steps,
                                            LegState& a, LegState& b, float& w) {
   if (MODEL == OF_MODEL_GBM) {
-    const int32_t j = q * 4;
-    const float2 p = of::normal_pair_from_u32(r.x, r.y), pq = of::normal_pair_from_u32(r.z, r.w);
-    w += p.x;
-    if (j + 1 < steps) w += p.y;
-    if (j + 2 < steps) w += pq.x;
-    if (j + 3 < steps) w += pq.y;
+    const int32_t rem = steps - 4 * q;
+    w = rem >= 4 ? gbm_add_block(w, r) : gbm_add_last(w, r, rem);
   } else if (MODEL == OF_MODEL_HESTON_EULER) {
     of::Polar z = of::polar_from_u32(r.x, r.y, c.bm_k2);
     of::heston_euler_step(a, c, z.q, z.c, z.s);

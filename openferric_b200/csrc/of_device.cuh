@@ -466,17 +466,25 @@ __device__ __forceinline__ float normal_pair_sum_from_u32(uint32_t a, uint32_t b
   return r * __sinf(ang);
 }
 
-// normal_pair_sum_from_u32 of two samples' draw pairs (a0, b0) and (a1, b1)
-// in packed pairs; each half is the scalar form bit for bit.
-__device__ __forceinline__ float2 normal_pair_sums2_from_u32(uint32_t a0, uint32_t b0, uint32_t a1, uint32_t b1) {
+// normal_pair_sum_from_u32 of two draw pairs (a0, b0) and (a1, b1) in packed
+// pairs, as the factors r and sin of the product ...
+__device__ __forceinline__ void normal_pair_sum_factors2_from_u32(uint32_t a0, uint32_t b0, uint32_t a1, uint32_t b1,
+                                                                  float2& r, float2& sn) {
   const float2 u1 = sub2(make_float2(unit_mantissa(a0), unit_mantissa(a1)),
                          splat2(0.999999940395355224609375f));
   const float2 rr = mul2(splat2(2.0f * kBoxMullerK2), make_float2(__log2f(u1.x), __log2f(u1.y)));
-  const float2 r = make_float2(sqrtf(rr.x), sqrtf(rr.y));
+  r = make_float2(sqrtf(rr.x), sqrtf(rr.y));
   const float2 ang = fma2(splat2(6.28318530717959f),
                           make_float2(unit_mantissa(b0), unit_mantissa(b1)),
                           splat2(kBoxMullerAngSum));
-  return mul2(r, make_float2(__sinf(ang.x), __sinf(ang.y)));
+  sn = make_float2(__sinf(ang.x), __sinf(ang.y));
+}
+
+// ... and as the product; each half is the scalar form bit for bit.
+__device__ __forceinline__ float2 normal_pair_sums2_from_u32(uint32_t a0, uint32_t b0, uint32_t a1, uint32_t b1) {
+  float2 r, sn;
+  normal_pair_sum_factors2_from_u32(a0, b0, a1, b1, r, sn);
+  return mul2(r, sn);
 }
 
 // ---------------------------------------------------------------------------
