@@ -1952,14 +1952,17 @@ static of_status book_plan_create(of_ctx* ctx, const of_book_entry* e, int64_t n
     for (int64_t k = 0; k < r.tiles; ++k)
       *tile++ = {r.opt, r.count, r.first + k * tile_samples, (int32_t)(r.slot + k), 0};
   // (from pageable memory the call returns once the bytes have left it)
+  // A plan created while the context's stream is captured uploads on a stream
+  // of its own and waits: captured, the copy would become a node of the
+  // caller's graph that reads `heap` long after it is gone.  (A call that
+  // borrows the context's buffers is refused under capture, as it waits.)
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   cudaStream_t up = ctx->stream;
-  // A plan of its own is uploaded when it is returned, on a stream that no
-  // caller captures: in a capture of the context's stream the copy would
-  // become a node of the caller's graph that reads `heap` long after it is gone.
-  if (!pl->scratch && cudaStreamCreateWithFlags(&up, cudaStreamNonBlocking) != cudaSuccess)
-    return fail(of_fail(ctx, OF_ERR_CUDA, "upload stream creation failed"));
-  cudaError_t up_err = cudaMemcpyAsync(pl->d_image, image, bytes, cudaMemcpyHostToDevice, up);
-  if (!pl->scratch) {
+  cudaError_t up_err = pl->scratch ? cudaSuccess : cudaStreamIsCapturing(up, &capturing);
+  if (up_err == cudaSuccess && capturing == cudaStreamCaptureStatusNone) {
+    up_err = cudaMemcpyAsync(pl->d_image, image, bytes, cudaMemcpyHostToDevice, up);
+  } else if (up_err == cudaSuccess && (up_err = cudaStreamCreateWithFlags(&up, cudaStreamNonBlocking)) == cudaSuccess) {
+    up_err = cudaMemcpyAsync(pl->d_image, image, bytes, cudaMemcpyHostToDevice, up);
     if (up_err == cudaSuccess) up_err = cudaStreamSynchronize(up);
     cudaStreamDestroy(up);
   }
