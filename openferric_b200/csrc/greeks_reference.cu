@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(kGreekThreads) heston_delta_kernel(const __gri
     rng.seed(P.seed + (uint64_t)i * 7919ULL);
     double y = 0.0, v = P.v0;
     for (int64_t left = P.steps; left > 0; left -= of::kDrawBatch / 2) {
-      of::stream_normals(rng, buf, lane);
       const int n = left < of::kDrawBatch / 2 ? (int)left : of::kDrawBatch / 2;
+      of::stream_normals(rng, buf, lane, 2 * n);
 #pragma unroll 2
       for (int k = 0; k < n; ++k) {
         const double z1 = buf.z[2 * k * 32 + lane], z2 = buf.z[(2 * k + 1) * 32 + lane];

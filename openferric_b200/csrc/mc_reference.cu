@@ -272,8 +272,8 @@ __global__ void __launch_bounds__(kRefThreads) mc_ref_gbm_path(const __grid_cons
     double w = 0.0, aa = P.w0, ab = P.w0, g = 0.0, thr = P.bar_thr;
     bool ha = P.bar_hit0 != 0, hb = ha;
     for (int32_t j0 = 0; j0 < steps; j0 += of::kDrawBatch) {
-      of::stream_normals(rng, buf, lane);
       const int n = steps - j0 < of::kDrawBatch ? steps - j0 : of::kDrawBatch;
+      of::stream_normals(rng, buf, lane, n);
 #pragma unroll 4
       for (int k = 0; k < n; ++k) {
         w += buf.z[k * 32 + lane];
@@ -330,8 +330,8 @@ __global__ void __launch_bounds__(kRefThreads) mc_ref_heston(const __grid_consta
     rng.seed(P.seed + (uint64_t)i * 7919ULL);
     double ya = 0.0, yb = 0.0, va = P.v0, vb = va;
     for (int32_t j0 = 0; j0 < steps; j0 += of::kDrawBatch / 2) {
-      of::stream_normals(rng, buf, lane);
       const int n = steps - j0 < of::kDrawBatch / 2 ? steps - j0 : of::kDrawBatch / 2;
+      of::stream_normals(rng, buf, lane, 2 * n);
 #pragma unroll 2
       for (int k = 0; k < n; ++k) {
         const double z1 = buf.z[2 * k * 32 + lane], z2 = buf.z[(2 * k + 1) * 32 + lane];

@@ -271,11 +271,12 @@ __device__ __forceinline__ double stream_normal_sum(RNG& rng, int64_t steps, dou
 }
 
 // ---------------------------------------------------------------------------
-// The next kDrawBatch normals of each lane's stream, in order, into the
-// warp's z[draw][lane] (shared memory).  The tail draws of all lanes are
-// queued (a mask per lane, a prefix sum over the warp) and evaluated 32 at a
-// time: with 16 draws per lane about 25 of 512, one round.  Called by whole
-// warps.
+// The next `n` normals of each lane's stream, at most kDrawBatch, in order, into
+// the warp's z[draw][lane] (shared memory); n is the warp's, and taken as the next
+// multiple of four or one past it (a path of one step would wait for 15 draws
+// that nothing reads).  The tail draws of all lanes are queued (a mask per lane, a prefix sum
+// over the warp) and evaluated 32 at a time: with 16 draws per lane about 25 of
+// 512, one round.  Called by whole warps.
 // ---------------------------------------------------------------------------
 constexpr int kDrawBatch = 16;
 
@@ -285,20 +286,24 @@ struct DrawBuf {
 };
 
 template <typename RNG>
-__device__ __forceinline__ void stream_normals(RNG& rng, DrawBuf& buf, int lane) {
+__device__ __forceinline__ void stream_normals(RNG& rng, DrawBuf& buf, int lane, int n = kDrawBatch) {
   unsigned tails = 0;
+  auto draw = [&](int k) {
+    const double q = draw_q(rng.next_u64());
+    const bool tail = draw_in_tail(q);
+    double num, den;
+    central_parts(draw_masked(q, tail), num, den);
+    const double z = num * rcp64(den);
+    buf.z[k * 32 + lane] = tail ? q : z;
+    if (tail) tails |= 1u << k;
+  };
 #pragma unroll
   for (int g = 0; g < kDrawBatch; g += 4) {
+    if (g >= n) break;
+    draw(g);
+    if (g + 1 == n) break;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const double q = draw_q(rng.next_u64());
-      const bool tail = draw_in_tail(q);
-      double n, d;
-      central_parts(draw_masked(q, tail), n, d);
-      const double z = n * rcp64(d);
-      buf.z[(g + k) * 32 + lane] = tail ? q : z;
-      if (tail) tails |= 1u << (g + k);
-    }
+    for (int k = 1; k < 4; ++k) draw(g + k);
   }
   int at = __popc(tails);  // inclusive prefix sum of the counts
 #pragma unroll
