@@ -54,14 +54,28 @@ constexpr int kRangePerWarp = 32 * 4;  // paths one warp scans for in-the-money 
 constexpr float kLn2 = 0.69314718055994531f;
 
 constexpr int kPathThreads = 128;
-// The sweep back runs where fewer than kSweepShare of at least kSweepPathsPerSm
-// paths an SM are expected in the money.  1,048,576 paths of 512 steps, Asian:
-// 3.82 ms for the tangent pass whatever the share; forward pass and sweep 4.1
-// at a share of 0.13, 3.4 at 0.07, 3.0 at 0.  One round of sweeps takes 0.75 ms
-// however few they are, which the tangent pass undercuts below 2^20 paths:
-// 32,768 paths take 0.22 ms against 2.06 at the money.
-constexpr double kSweepShare = 0.10;
-constexpr int64_t kSweepPathsPerSm = 7000;
+// The sweep back runs where few paths are expected in the money (sweep_pays).
+// Its time over the tangent pass's, by paths an SM and share in the money, at 32
+// to 2,048 steps (they agree to 0.03 from 128 steps on):
+//              Asian                              European
+//    3,540     0.90 (0.1 %)  1.07 (3 %)           0.92  1.11
+//    7,080     0.88 (6 %)  0.99 (10 %)  1.03 (12 %)   0.92  1.03  1.08
+//   14,170     0.89 (10 %)  0.96 (12 %)  1.03 (14 %)  0.92  0.99  1.06
+//   28,340     0.90 (12 %)  0.94 (14 %)  1.03 (17 %)  0.92  1.00  1.09
+//   56,680     0.87 (12 %)  0.93 (14 %)  1.02 (17 %)  0.90  0.97  1.06
+// They meet at a share of 0.16 - 425 / (paths an SM), the second term a round of
+// sweeps, whose time does not fall with their number; below 7,000 paths an SM
+// that round is no longer covered but where there are next to no sweeps.
+// 8,388,608 Asian paths of 128 steps with 12 % in the money: 8.1 ms for the
+// tangents, 7.0 for the sweep; 32,768 paths of 512 steps at the money: 0.22 and
+// 2.06.
+constexpr double kSweepShare = 0.16, kSweepRound = 425.0, kSweepShareFew = 0.01;
+constexpr double kSweepPathsPerSm = 7000.0, kSweepPathsPerSmFew = 3500.0;
+
+bool sweep_pays(double share, double paths_per_sm) {
+  if (paths_per_sm >= kSweepPathsPerSm) return share < kSweepShare - kSweepRound / paths_per_sm;
+  return paths_per_sm >= kSweepPathsPerSmFew && share < kSweepShareFew;
+}
 
 __device__ __forceinline__ float rsqrt_approx(float x) {
   float r;
@@ -692,16 +706,20 @@ extern "C" of_status of_heston_price_adjoint(of_ctx* ctx, const of_heston_adjoin
     }
     c.rho_w = -r / (1.0 - r * r);
     const bool greeks = p->forward_only == 0;
-    const bool tangent = greeks && !(p->num_paths >= kSweepPathsPerSm * ctx->sm_count && itm_share(p) < kSweepShare);
+    bool tangent = greeks && !sweep_pays(itm_share(p), (double)p->num_paths / ctx->sm_count);
     void* d_ck = nullptr;
     if (greeks && !tangent) {
       // checkpoints (v, y) + per-path gradient and underlying
       const size_t ck_bytes = (size_t)n_seg * p->num_paths * 2 * sizeof(float) + (size_t)p->num_paths * 2 * sizeof(float);
-      OF_TRY(of_scratch(ctx, SLOT_ADJ_CKPT, ck_bytes, &d_ck));
-      c.ck_v = (float*)d_ck;
-      c.ck_y = c.ck_v + (size_t)n_seg * p->num_paths;
-      c.grad = c.ck_y + (size_t)n_seg * p->num_paths;
-      c.und = c.grad + p->num_paths;
+      if (of_scratch(ctx, SLOT_ADJ_CKPT, ck_bytes, &d_ck) == OF_OK) {
+        c.ck_v = (float*)d_ck;
+        c.ck_y = c.ck_v + (size_t)n_seg * p->num_paths;
+        c.grad = c.ck_y + (size_t)n_seg * p->num_paths;
+        c.und = c.grad + p->num_paths;
+      } else {  // no room for them: the tangent pass needs none
+        cudaGetLastError();
+        tangent = true;
+      }
     }
     // every pass runs on the tangent pass's grid, so that a price is the same
     // sum whichever pass computed it
