@@ -560,6 +560,17 @@ of_status of_xoshiro_jump(of_ctx* ctx, uint64_t seed, const uint64_t* draws, int
 of_status of_test_bounded_wait(of_ctx* ctx, int32_t arrive, uint32_t limit_us, int32_t* waited_ok,
                                double* elapsed_us);
 
+/* Test of the bounded wait of the FP64 Longstaff-Schwartz backward induction,
+ * whose blocks wait for one another's rows (no reference counterpart): a small
+ * American put is priced with that wait limited to `limit_us` microseconds.
+ *   withhold == 0: every row arrives;
+ *   withhold != 0: one block's rows are never written, so the wait runs out.
+ * *waited_ok receives 1 if the call priced the put and 0 if it ended in
+ * OF_ERR_TIMEOUT, *elapsed_us the host time it took.  The kernel returns either
+ * way and the context stays usable. */
+of_status of_test_lsm_wait(of_ctx* ctx, int32_t withhold, uint32_t limit_us, int32_t* waited_ok,
+                           double* elapsed_us);
+
 /* ---- Heston pathwise Greeks (FP32) ---------------------------------------- */
 typedef struct of_heston_adjoint_params {
   double spot, strike, rate, dividend_yield, expiry;

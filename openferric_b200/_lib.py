@@ -25,7 +25,7 @@ EXPORTED = [
     "of_lsm_price", "of_xoshiro_jump", "of_heston_price_adjoint", "of_mc_european_gpu", "of_mc_strip_noalloc",
     "of_measure_device_peaks", "of_lsm_bermudan", "of_mc_european_qmc", "of_autotune_strip", "of_autotune_book",
     "of_test_bounded_wait", "of_book_price_to_stderr", "of_book_plan_greeks", "of_mc_price_book_greeks",
-    "of_book_price_to_stderr_greeks", "of_lsm_barrier", "of_min_sum_in_order",
+    "of_book_price_to_stderr_greeks", "of_lsm_barrier", "of_min_sum_in_order", "of_test_lsm_wait",
 ]
 
 
@@ -109,6 +109,8 @@ def _declare(L):
     L.of_autotune_book.restype = C.c_int
     L.of_test_bounded_wait.argtypes = [vp, C.c_int32, C.c_uint32, P(C.c_int32), P(C.c_double)]
     L.of_test_bounded_wait.restype = C.c_int
+    L.of_test_lsm_wait.argtypes = [vp, C.c_int32, C.c_uint32, P(C.c_int32), P(C.c_double)]
+    L.of_test_lsm_wait.restype = C.c_int
     L.of_book_price_to_stderr.argtypes = [vp, P(A.OfBookEntry), C.c_int64, P(A.OfBookConfig), P(A.OfStderrTarget),
                                           P(A.OfMcResult), P(C.c_int64), P(A.OfStderrRound), P(C.c_int32)]
     L.of_book_price_to_stderr.restype = C.c_int

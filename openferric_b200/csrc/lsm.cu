@@ -32,6 +32,7 @@
 // single-precision-only flags -ftz=true -prec-sqrt=false -prec-div=false,
 // which leave the FP64 reference mode untouched.
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -213,6 +214,8 @@ struct LsmBatch {
   int32_t lane_paths;        // paths per lane in lsm_gen_stream
   const uint64_t* states;    // lsm_stream_setup's output
   void* rows;                // [2][nc][gridDim.x][kRowWords] 16-byte words of lsm_backward_ref
+  uint64_t wait_ns;          // its waits' limit
+  int32_t withheld;          // the block whose rows are never written, or -1 (of_test_lsm_wait)
 };
 
 template <typename T>
@@ -1443,7 +1446,6 @@ namespace {
 // B.status and leaves, and so do the others at their next wait.
 // ---------------------------------------------------------------------------
 constexpr int kBackThreads = 256;
-constexpr uint64_t kBackWaitNs = 1000000000ull;
 
 __device__ __forceinline__ uint64_t lsm_timer_ns() {
   uint64_t t;
@@ -1530,7 +1532,7 @@ __device__ __forceinline__ bool back_moments(const LsmBatch& B, int c, int k, co
   ulonglong2* rows = (ulonglong2*)B.rows + ((size_t)(k & 1) * B.nc + c) * gridDim.x * kRowWords;
   if (warp == 0) {
     const double t = back_cross_warp(sh, lane);
-    if (lane < NM) row_store(rows + (size_t)blockIdx.x * kRowWords + lane, t, tag);
+    if (lane < NM && (int)blockIdx.x != B.withheld) row_store(rows + (size_t)blockIdx.x * kRowWords + lane, t, tag);
   }
   // thread t adds rows t / 16, t / 16 + 16, ... of moment t % 16
   const int m = threadIdx.x & 15;
@@ -1550,7 +1552,7 @@ __device__ __forceinline__ bool back_moments(const LsmBatch& B, int c, int k, co
           v[i] = 0.0;
           if (r < gridDim.x) got &= row_load(rows + (size_t)r * kRowWords + m, tag, v[i]);
         }
-        if (!got && lsm_timer_ns() - start > kBackWaitNs) {
+        if (!got && lsm_timer_ns() - start > B.wait_ns) {
           ok = false;
           break;
         }
@@ -2081,6 +2083,8 @@ of_status lsm_enqueue(of_ctx* ctx, LsmRun& r, const of_lsm_config* cfg, cudaStre
     OF_CUDA_TRY(ctx, cudaMemcpyAsync(r.d_inj, r.inj_host, cnt * sizeof(double), cudaMemcpyHostToDevice, gs));
     B.inj = (const double*)r.d_inj;
   }
+  B.wait_ns = ctx->lsm_wait_ns;
+  B.withheld = ctx->lsm_withheld;
   const int back_ppt = fp64 ? lsm_back_ppt(ctx, B.n, nc) : 0;
   if (fp64 && lsm_log_space(r)) {
     B.lane_paths = lsm_lane_paths(B.n);
@@ -2448,6 +2452,40 @@ extern "C" of_status of_lsm_price(of_ctx* ctx, const of_lsm_contract* ks, int64_
   }
   for (int64_t i = 0; i < n; ++i) res[i].kernel_ms = total_ms;
   return OF_OK;
+}
+
+// The bounded wait of lsm_backward_ref on a small American put (1,024 paths in
+// four blocks, four dates), with or without the rows of one block.
+extern "C" of_status of_test_lsm_wait(of_ctx* ctx, int32_t withhold, uint32_t limit_us, int32_t* waited_ok,
+                                      double* elapsed_us) {
+  if (!ctx || !waited_ok || !elapsed_us) return OF_ERR_INVALID_INPUT;
+  if (limit_us == 0 || limit_us > 1000000u)
+    return of_fail(ctx, OF_ERR_INVALID_INPUT, "limit_us must be in 1..1000000");
+  of_lsm_contract k{};
+  k.option_type = OF_PUT;
+  k.exercise = OF_EXERCISE_AMERICAN;
+  k.spot = 38.0;
+  k.strike = 40.0;
+  k.rate = 0.05;
+  k.vol = 0.3;
+  k.expiry = 1.0;
+  k.num_steps = 4;
+  of_lsm_config cfg{};
+  cfg.num_paths = 1024;
+  cfg.seed = 7;
+  cfg.basis_degree = 2;
+  cfg.precision = OF_PREC_FP64_REFERENCE;
+  of_lsm_result res{};
+  const uint64_t limit = ctx->lsm_wait_ns;
+  ctx->lsm_wait_ns = (uint64_t)limit_us * 1000u;
+  ctx->lsm_withheld = withhold ? 1 : -1;
+  const auto start = std::chrono::steady_clock::now();
+  const of_status st = of_lsm_price(ctx, &k, 1, &cfg, &res);
+  *elapsed_us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - start).count();
+  ctx->lsm_wait_ns = limit;
+  ctx->lsm_withheld = -1;
+  *waited_ok = st == OF_OK ? 1 : 0;
+  return st == OF_ERR_TIMEOUT ? OF_OK : st;
 }
 
 static bool strictly_increasing(const double* g, int64_t n) {

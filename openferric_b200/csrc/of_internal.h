@@ -52,6 +52,10 @@ struct of_ctx {
   // flight into shared memory it no longer owns: from then on the context
   // refuses work, and the caller destroys it and creates a new one.
   bool unusable = false;
+  // Limit of lsm_backward_ref's waits for its other blocks, and the block whose
+  // rows a test withholds (-1: none).
+  uint64_t lsm_wait_ns = 1000000000ull;
+  int32_t lsm_withheld = -1;
 };
 
 // Records a formatted message as the context's last error and returns `st`.
