@@ -2216,6 +2216,27 @@ of_status lsm_collect(of_ctx* ctx, const LsmRun& r, std::vector<double>& results
   return OF_OK;
 }
 
+// Pinned staging of a call: the context's buffer, which stays, up to 8 MB; more
+// (130,000 dates of contracts) is allocated for the call and given back with it.
+struct LsmStaging {
+  void* own = nullptr;
+  LsmStaging() = default;
+  LsmStaging(const LsmStaging&) = delete;
+  LsmStaging& operator=(const LsmStaging&) = delete;
+  ~LsmStaging() {
+    if (own) cudaFreeHost(own);
+  }
+  of_status get(of_ctx* ctx, size_t bytes, void** out) {
+    if (bytes <= ((size_t)8 << 20)) return of_pinned(ctx, bytes, out);
+    if (cudaMallocHost(&own, bytes) != cudaSuccess) {
+      own = nullptr;
+      return of_fail(ctx, OF_ERR_ALLOC, "LSM staging allocation failed");
+    }
+    *out = own;
+    return OF_OK;
+  }
+};
+
 // The context's lowest-priority stream, created on first use.
 of_status lsm_side_stream(of_ctx* ctx, cudaStream_t* out) {
   if (!ctx->side_stream) {
@@ -2248,8 +2269,9 @@ of_status lsm_run_batch(of_ctx* ctx, std::vector<LsmHost>& hs, int64_t steps, co
   OF_TRY(of_scratch(ctx, SLOT_LSM_AUX, r.aux_bytes, &dAux));
   if (inj_host)
     OF_TRY(of_scratch(ctx, SLOT_INJECT, (size_t)cfg->num_paths * steps * draws * sizeof(double), &r.d_inj));
+  LsmStaging stage;  // outlives the drain below
   void* pin = nullptr;
-  OF_TRY(of_pinned(ctx, r.dev.image, &pin));
+  OF_TRY(stage.get(ctx, r.dev.image, &pin));
   OF_TRY(lsm_bind(ctx, r, cfg, dS, dVal, dAux, jump, pin, false));
   OF_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
   const of_status st = lsm_enqueue(ctx, r, cfg, ctx->stream, ctx->stream);
@@ -2407,8 +2429,9 @@ extern "C" of_status of_lsm_price(of_ctx* ctx, const of_lsm_contract* ks, int64_
   if (inj_need) OF_TRY(of_scratch(ctx, SLOT_INJECT, inj_need, &d_inj));  // fed by the side stream, in order
   size_t staging = 0;
   for (const std::unique_ptr<LsmRun>& run : runs) staging += run->dev.image;
+  LsmStaging stage;  // outlives the drain below
   void* pin = nullptr;
-  OF_TRY(of_pinned(ctx, staging, &pin));
+  OF_TRY(stage.get(ctx, staging, &pin));
   for (size_t i = 0; i < runs.size(); ++i) {
     runs[i]->d_inj = d_inj;
     const int s = (int)(i % 2);
