@@ -21,7 +21,6 @@ namespace of {
 // 1/d for a normal d, by the cubically convergent iteration
 // y' = y (1 + e + e^2), e = 1 - d y (Householder's method for 1/x), from the
 // 20-bit rcp.approx: the error left is of the order of the last rounding.
-// Three FP64 operations against the divide's eight and its slow-path test.
 __device__ __forceinline__ double rcp64(double d) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
