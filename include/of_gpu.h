@@ -627,7 +627,7 @@ of_status of_heston_price_adjoint(of_ctx* ctx, const of_heston_adjoint_params* p
  * It creates no context, stream or event either.
  *
  * Same computation as of_mc_strip (FP32 Philox, one shared path set), with
- * its scratch (strikes, per-block partial sums, final sums) in one static
+ * its scratch (per-block partial sums, final sums, a status word) in one static
  * device array of OF_STRIP_NOALLOC_SCRATCH_BYTES that every GPU loading the
  * library holds until the process exits.  Limits: at most
  * OF_STRIP_NOALLOC_MAX_STRIKES strikes and OF_STRIP_NOALLOC_MAX_BLOCKS blocks
@@ -649,8 +649,8 @@ of_status of_heston_price_adjoint(of_ctx* ctx, const of_heston_adjoint_params* p
  * kernel_ms is not measured (0). */
 #define OF_STRIP_NOALLOC_MAX_STRIKES 64
 #define OF_STRIP_NOALLOC_MAX_BLOCKS 1024
-#define OF_STRIP_NOALLOC_SCRATCH_BYTES                                  \
-  (OF_STRIP_NOALLOC_MAX_STRIKES * 4 + (OF_STRIP_NOALLOC_MAX_STRIKES * 2 + 1) * 8 + \
+#define OF_STRIP_NOALLOC_SCRATCH_BYTES         \
+  ((OF_STRIP_NOALLOC_MAX_STRIKES * 2 + 1) * 8 + \
    OF_STRIP_NOALLOC_MAX_BLOCKS * OF_STRIP_NOALLOC_MAX_STRIKES * 2 * 8)
 of_status of_mc_strip_noalloc(void* cuda_stream, const of_model* model, int32_t option_type,
                               const double* strikes, int64_t n_strikes, const of_mc_config* cfg,

@@ -403,8 +403,8 @@ __device__ __forceinline__ void gk_asian(const GreekConsts<R>& c, uint64_t i, GE
 }
 
 // gk_terminal<float, G, ANTI> of samples i0 and i1: the normals' sums in
-// packed pairs, in the scalar loop's order (each half bit for bit the scalar
-// sum).
+// packed pairs, in the scalar loop's order (each half the scalar sum, up to the
+// compiler's contraction).
 template <bool G, bool ANTI, typename GEN>
 __device__ __forceinline__ void gk_terminal_pair(const GreekConsts<float>& c, uint64_t i0, uint64_t i1,
                                                  GEN K, GreekSample<float>& o0, GreekSample<float>& o1) {

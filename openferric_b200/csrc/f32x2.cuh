@@ -3,8 +3,11 @@
 // 64-bit register pair, so one issued instruction does the work of two.  Each
 // half is rounded exactly as the scalar instruction would round it: code
 // written with these gives the same bits as the scalar form with the same
-// operation order (fma stays fma, a product followed by an add stays two
-// roundings).
+// operation order, fma staying fma.  A product followed by an add stays two
+// roundings in the units compiled with --fmad=false; elsewhere the assembler
+// contracts a packed product with the packed sum that reads it (seen as one
+// rounding less in the results), so code that needs the bits there writes the
+// fma2, or the scalar __fmul_rn and __fadd_rn.
 #pragma once
 
 namespace of {

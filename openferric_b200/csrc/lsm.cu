@@ -1741,7 +1741,7 @@ int lsm_back_ppt(const of_ctx* ctx, int64_t n, int nc) {
 // (31 products a warp, as long as 40 draws of a path), fewer fill the
 // schedulers.  Device time of a European on 50 steps with 1, 2 and 4 paths a
 // lane: 109, 109, 120 us at 50,000 paths; 157, 136, 147 at 100,000; 244, 211,
-// 195 at 200,000.
+// 195 at 200,000 (148 SMs: the lines lie at 400 and 1,000 paths an SM).
 int lsm_lane_paths(int64_t n) { return n < 60000 ? 1 : n < 150000 ? 2 : 4; }
 
 }  // namespace

@@ -1048,8 +1048,8 @@ __device__ __forceinline__ void book_gbm_legs2(const BookOpt& o, uint64_t i0, ui
 // from the plain transform.  The antithetic twin has y_T = steps drift -
 // diff sum z.  The drift is added once instead of every step, so y_T differs
 // from the stepwise sum of the general loop by FP32 rounding only.  The
-// packed-pair form below sums in the same order, so each of its halves is
-// this scalar sum bit for bit.
+// packed-pair form below sums in the same order: each of its halves is this
+// scalar sum, up to where the compiler contracts a product with the sum.
 template <typename GEN>
 __device__ __forceinline__ float book_terminal_sum(const BookOpt& o, uint64_t i, GEN G) {
   const of::PhiloxLane L = G.lane(i);
@@ -1910,8 +1910,8 @@ static of_status book_plan_create(of_ctx* ctx, const of_book_entry* e, int64_t n
   // The tables in one image, uploaded once: [options | tiles | weights |
   // dividends | Greek constants | slot ranges | counters].  A plan that lives
   // inside one call borrows the context's cached buffers (no cudaMalloc,
-  // cudaFree or cudaMallocHost per call) and stages images of up to 8 MB, a
-  // quarter of a million tiles, in its pinned buffer behind the sums; larger
+  // cudaFree or cudaMallocHost per call) and stages images of up to 8 MB,
+  // some 340,000 tiles of 24 bytes, in its pinned buffer behind the sums; larger
   // ones go from pageable memory, so that the buffer stays small.  A call on
   // 384 options (21,000 tiles) spends 0.6 ms beside its kernels, against 2.0
   // and up with nine allocations, six uploads and their frees.
@@ -2152,7 +2152,7 @@ of_status of_mc_run_fp32(of_ctx* ctx, const of_model* m, const of_payoff* p, con
 // For callers that cannot allocate device memory when they price: every
 // byte of scratch the strip kernel needs lives in the static array below,
 // which each GPU that loads this library holds until the process exits.
-// Layout: [MAX_STRIKES floats unused][sums: 2*MAX_STRIKES doubles]
+// Layout: [sums: 2*MAX_STRIKES doubles][status: one double]
 //         [per-block partials: MAX_BLOCKS * 2*MAX_STRIKES doubles].
 // In host code `g_strip_noalloc_scratch` names a host-side stand-in, not the
 // device array: its device address is looked up with cudaGetSymbolAddress
@@ -2281,7 +2281,7 @@ extern "C" of_status of_mc_strip_noalloc(void* cuda_stream, const of_model* m, i
     noalloc_msg(err, err_len, "device address of the static scratch: %s", cudaGetErrorString(e));
     return OF_ERR_CUDA;
   }
-  double* d_sums = (double*)((char*)base + OF_STRIP_NOALLOC_MAX_STRIKES * 4);
+  double* d_sums = (double*)base;
   double* d_status = d_sums + OF_STRIP_NOALLOC_MAX_STRIKES * 2;  // the warp-specialised kernel's status word
   double* d_partials = d_status + 1;
 
