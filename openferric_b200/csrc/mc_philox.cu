@@ -111,13 +111,14 @@ __device__ __forceinline__ void simulate_terminal(const StepConsts& c, int32_t s
     const int32_t full = steps >> 2;
     if constexpr (ILP == 1) {
       sum[0] = 0.0f;
-      of::philox_for_blocks<FULL>(T, full, K,
-                                  [&](const uint4 t) { sum[0] = gbm_add_block(sum[0], of::philox_block(t, L[0], K)); });
+      for (int32_t q = 0; q < full; ++q)
+        sum[0] = gbm_add_block(sum[0], of::philox_block(of::philox_terms<FULL>(T, (uint32_t)q, K), L[0], K));
     } else {
       float2 w = make_float2(0.0f, 0.0f);
-      of::philox_for_blocks<FULL>(T, full, K, [&](const uint4 t) {
+      for (int32_t q = 0; q < full; ++q) {
+        const uint4 t = of::philox_terms<FULL>(T, (uint32_t)q, K);
         w = gbm_add_block2(w, of::philox_block(t, L[0], K), of::philox_block(t, L[1], K));
-      });
+      }
       sum[0] = w.x;
       sum[1] = w.y;
     }
@@ -135,11 +136,12 @@ __device__ __forceinline__ void simulate_terminal(const StepConsts& c, int32_t s
   } else if constexpr (MODEL == OF_MODEL_HESTON_EULER && ILP == 2 && !ANTI) {
     of::LegState2 a{make_float2(0.0f, 0.0f), make_float2(c.v0, c.v0)};
     const int32_t pairs = steps >> 1;  // full Philox calls; an odd last step below
-    of::philox_for_blocks<FULL>(T, pairs, K, [&](const uint4 t) {
+    for (int32_t q = 0; q < pairs; ++q) {
+      const uint4 t = of::philox_terms<FULL>(T, (uint32_t)q, K);
       const uint4 r0 = of::philox_block(t, L[0], K), r1 = of::philox_block(t, L[1], K);
       of::heston_euler_step2(a, c, of::polars2_from_u32(r0.x, r0.y, r1.x, r1.y, c.bm_k2));
       of::heston_euler_step2(a, c, of::polars2_from_u32(r0.z, r0.w, r1.z, r1.w, c.bm_k2));
-    });
+    }
     if (steps & 1) {
       const uint4 t = of::philox_terms<FULL>(T, (uint32_t)pairs, K);
       const uint4 r0 = of::philox_block(t, L[0], K), r1 = of::philox_block(t, L[1], K);
@@ -171,14 +173,15 @@ __device__ __forceinline__ void simulate_terminal(const StepConsts& c, int32_t s
       }
     };
     const int32_t pairs = steps >> 1;
-    of::philox_for_blocks<FULL>(T, pairs, K, [&](const uint4 t) {
+    for (int32_t q = 0; q < pairs; ++q) {
+      const uint4 t = of::philox_terms<FULL>(T, (uint32_t)q, K);
 #pragma unroll
       for (int l = 0; l < ILP; ++l) {
         const uint4 r = of::philox_block(t, L[l], K);
         step(l, r.x, r.y);
         step(l, r.z, r.w);
       }
-    });
+    }
     if (steps & 1) {
       const uint4 t = of::philox_terms<FULL>(T, (uint32_t)pairs, K);
 #pragma unroll
@@ -255,12 +258,13 @@ __device__ __forceinline__ void strip_finish(const StripParams& P, int cols, con
   if (threadIdx.x == 0) *P.ticket = 0;
 }
 
-// Counter blocks in the q table of the strip (16 KB, four blocks an SM): 4,096
-// GBM or 2,048 Heston steps.  Past it the terms are computed in place behind a
-// range test, which costs more than the table saves where the warps are few:
-// Heston, 65,536 x 1,024 steps x 41 strikes, took 181 us with 256 entries and
-// 158 with 1,024 (172 before there was a table).
-constexpr uint32_t kStripTab = 1024;
+// Counter blocks in the q table of the strip (28 KB, four blocks an SM beside
+// the sums of 128 strikes): 7,168 GBM or 3,584 Heston steps.  Past it the terms
+// are computed in place behind a range test, which costs more than the table
+// saves where the warps are few: Heston, 65,536 x 1,024 steps x 41 strikes, took
+// 181 us with 256 entries and 158 with all of its 512 (172 before there was a
+// table).  A second loop without the test cost the strips that fit 1 %.
+constexpr uint32_t kStripTab = 1792;
 
 // KPL 0: one strike, whose sums each lane keeps for its own samples (no
 // shuffles; for one strike these took longer than 16 steps).

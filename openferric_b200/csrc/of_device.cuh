@@ -239,16 +239,6 @@ __device__ __forceinline__ uint4 philox_terms(const PhiloxTab& T, uint32_t q, co
   return FULL || q < T.n ? T.tab[q] : philox_q(q, T.hi, T.stream, K);
 }
 
-// body(terms) for the counter blocks 0 .. n-1: those in the table, then the
-// others, in two loops without a range test.
-template <bool FULL, typename BODY>
-__device__ __forceinline__ void philox_for_blocks(const PhiloxTab& T, int32_t n, const PhiloxKeys& K, BODY body) {
-  const int32_t split = FULL || n < (int32_t)T.n ? n : (int32_t)T.n;
-  for (int32_t q = 0; q < split; ++q) body(T.tab[q]);
-  if constexpr (!FULL)
-    for (int32_t q = split; q < n; ++q) body(philox_q((uint32_t)q, T.hi, T.stream, K));
-}
-
 // The counter blocks of one stream for a block of threads: the keys and the
 // stream's table.  lane(i) is sample i's part; a copy serves the samples of
 // one high word.  FULL: the table covers every counter block and every

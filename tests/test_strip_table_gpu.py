@@ -1,6 +1,6 @@
-"""The strip's paths across the end of its table of Philox terms (1,024 counter
-blocks: 4,096 GBM or 2,048 Heston steps), past which a second loop computes the
-terms in place: prices on the strip's own draws, paths in numpy and FP64, with
+"""The strip's paths across the end of its table of Philox terms (1,792 counter
+blocks: 7,168 GBM or 3,584 Heston steps), past which the terms are computed in
+place: prices on the strip's own draws, paths in numpy and FP64, with
 the tolerance derived beside them."""
 import numpy as np
 import pytest
@@ -12,9 +12,9 @@ from test_strip_draws_gpu import S0, _gen, _paths
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("model,steps", [("gbm", 4095), ("gbm", 4096), ("gbm", 4100), ("gbm", 4105),
-                                         ("heston", 2047), ("heston", 2048), ("heston", 2049), ("heston", 2053),
-                                         ("qe", 2050)])
+@pytest.mark.parametrize("model,steps", [("gbm", 7167), ("gbm", 7168), ("gbm", 7172), ("gbm", 7177),
+                                         ("heston", 3583), ("heston", 3584), ("heston", 3585), ("heston", 3589),
+                                         ("qe", 3586)])
 @pytest.mark.parametrize("anti", [False, True])
 @pytest.mark.parametrize("tile", [1, 2])
 def test_paths_across_the_end_of_the_table(model, steps, anti, tile):
