@@ -887,6 +887,8 @@ def main():
                 "frac": sfu_frac, "per_step": SFU_PER_STEP,
                 "peak_source": f"{probe_src} (MUFU lg2/sqrt/sin/cos chains); derived nominal "
                                f"{148 * 16 * sm_max * 1e6 / 1e12:.2f} TOP/s at 16/clk/SM"}
+    # the declared budget with the larger fraction; the busiest pipe is the FMA pipe's heavy half (72 %), with
+    # Philox's wide multiplies, which neither budget counts (profiles/strip_kernel_heston_euler_ilp2_2p20.md)
     bound, main_line, other_name, other_line = (
         ("sfu", sfu_line, "fp32", fp32_line) if sfu_frac >= fp32_frac else ("fp32", fp32_line, "sfu", sfu_line))
     # issue slots: Philox, conversions and control flow included
@@ -910,6 +912,7 @@ def main():
                          # times the squared radius
                          frac_at_4_mufu_per_step=per_gpu * 4.0 / sfu_peak),
         "e2e": {"value": world * PATH_STEPS * args.steps / e2e_s, "unit": UNIT,
+                # the strikes travel in the launch's parameters, the sums by the kernel's stores to pinned memory
                 "h2d_bytes_per_step": 41 * 4, "d2h_bytes_per_step": 41 * 2 * 8},
         "gpu_launches": 2 * args.steps,
         "clocks": clk,

@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(128) mc_ref_kernel(RefParams P, double* __rest
 // and after on one B200 (launch included):
 //   European 100,000 x 252              387 -> 90 us
 //   Asian 50,000 pairs x 252, both averages  ~660 -> 95 us
-//   knock-out 25,001 pairs x 126        144 -> 38 us
+//   knock-out 25,001 pairs x 126        144 -> 37 us
 //   Heston European 131,072 x 256       940 -> 250 us
 // ---------------------------------------------------------------------------
 constexpr int kRefThreads = 64;  // small blocks: 100,000 samples fill 148 SMs to 96 %, blocks of 128 to 88 %
