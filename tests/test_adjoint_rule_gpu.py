@@ -27,14 +27,15 @@ def _strike(share, asian, T=1.0):
 
 
 @pytest.mark.parametrize("asian", [False, True])
-@pytest.mark.parametrize("per_sm", [3600, 7100, 30_000])
-def test_both_sides_of_the_rule_agree(asian, per_sm):
+@pytest.mark.parametrize("per_sm,steps", [(3600, 33), (7100, 33), (30_000, 33), (3600, 2048), (7100, 2048)])
+def test_both_sides_of_the_rule_agree(asian, per_sm, steps):
     """Strikes 1e-6 apart on the two sides of the rule: the same paths, 1e-5 of
     whose in-the-money ones change sides.  Either pass is within 1e-3 (2e-4
-    absolute) of the FP64 difference, so within twice that of the other."""
+    absolute) of the FP64 difference, so within twice that of the other; at 2,048
+    steps, the longest path, both share what the FP32 path itself is off."""
     paths = per_sm * context(0).sm_count
     K = _strike(0.16 - 425.0 / per_sm if per_sm >= 7000 else 0.01, asian)
-    a, b = (heston_adjoint(HestonAdjointSpec(strike=K * x, expiry=1.0, num_paths=paths, num_steps=33, seed=3,
+    a, b = (heston_adjoint(HestonAdjointSpec(strike=K * x, expiry=1.0, num_paths=paths, num_steps=steps, seed=3,
                                              asian=asian), **BASE) for x in (1.0 - 5e-7, 1.0 + 5e-7))
     assert a.price == pytest.approx(b.price, rel=1e-4)
     for name in A.OF_ADJ_NAMES:
